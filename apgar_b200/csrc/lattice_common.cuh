@@ -135,6 +135,57 @@ struct FrontierClasses {
   FrontierLaunch c[5];
 };
 
+// The tile form's "no label yet": labels stay below it, and a 16-bit move cost
+// added to it, or to it with the top bit set, does not wrap.
+constexpr uint32_t kTileLabelLimit = 0x7FFE0000u;
+
+// Search state of a net in the tile form: the pending queue (a ring in the
+// net's workspace), the units queued or being relaxed, the level and the goal.
+struct TileNetState {
+  uint32_t phase;         // 0 not started, 1 searching, 2 done
+  uint32_t head, tail;    // the ring's next entry to take / to write
+  uint32_t active;        // units queued or being relaxed
+  uint32_t thr;           // the level's key limit
+  uint32_t far_par;       // the far list in use
+  uint32_t far_count[2];
+  uint32_t goal;          // least goal label so far
+  uint32_t stop;          // 1 cancelled, 2 a broken invariant
+  uint32_t steps, units, levels;
+  uint32_t slot;          // workspace slot (slot mode)
+  uint32_t guests;        // warps that help the owner
+  uint32_t level_width;
+};
+static_assert(sizeof(TileNetState) == 64, "states are carved from the counters, 64 bytes each");
+
+// One size class of the tile form of the frontier (lattice_tiles.cu): net
+// workspaces (lattice_tile_words 32-bit words) at pool + plan.dist_offset
+// (per_net) or in `slots` slots of slot_words each.
+struct TileClass {
+  uint32_t* pool;
+  uint64_t slot_words;
+  uint32_t begin, end;  // its plans
+  uint32_t slots;       // warps (CTAs, in a team class) that take its nets
+  uint32_t team;        // 1: a net is a whole CTA's from the start
+  uint32_t level_width;
+  unsigned int* next_plan;
+};
+
+struct TileLaunch {
+  LatticeDeviceView lat;
+  const apgar_b200_lattice_net* nets;
+  const NetPlan* plans;    // class by class, largest windows first
+  TileNetState* states;    // zeroed, one per plan
+  uint32_t total;
+  uint32_t per_net;
+  apgar_b200_lattice_result* results;
+  uint32_t* path_arena;
+  uint64_t path_arena_capacity;
+  unsigned long long* arena_cursor;
+  const volatile uint32_t* cancel;
+  unsigned int* finished;  // nets that are done
+  TileClass c[5];          // the widest first
+};
+
 __device__ __forceinline__ uint32_t sat(uint32_t v) { return v < kLabelInf ? v : kLabelInf; }
 
 // 32 bits of a bit-packed row starting at signed bit position `pos`; bits

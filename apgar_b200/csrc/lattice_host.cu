@@ -29,6 +29,9 @@ cudaError_t launch_accumulate_cells(const apgar_b200_lattice_result* results, ui
                                     int sm_count, cudaStream_t stream);
 cudaError_t launch_lattice_frontier(const FrontierClasses& classes, int sm_count,
                                     cudaStream_t stream);
+uint64_t lattice_tile_words(int layers, uint32_t win_w, uint32_t win_h);
+cudaError_t lattice_tile_warps(int sm_count, uint32_t* out);
+cudaError_t launch_lattice_tiles(const TileLaunch& launch, int sm_count, cudaStream_t stream);
 cudaError_t launch_lattice_validate(const LatticeDeviceView& lat, const apgar_b200_lattice_net* nets,
                                     const apgar_b200_lattice_result* results, const uint32_t* paths,
                                     uint64_t path_count, uint32_t count,
@@ -68,11 +71,9 @@ namespace {
 // lanes cover its frame row (each lane holds lattice_cells_per_lane(L) cells
 // of every layer, so G warps cover 32 * C * G cells): the widest class is
 // issue-bound, and warps past the row's end would run every instruction on
-// padding.  The frontier uses the power-of-two sizes (kFrontierClasses).
+// padding.  The frontier's classes are 1, 2, 4, 8 and 16 warps.
 constexpr int kGroupSizes[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16};
 constexpr int kClassCount = 16;
-// Frontier width classes 0..4 (1, 2, 4, 8 and 16 warps) as kGroupSizes indices.
-constexpr int kFrontierClasses[] = {0, 1, 3, 7, 15};
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;
 
 struct LatticeObject;
@@ -101,8 +102,16 @@ uint32_t default_chain(int) { return 0u; }
 // and 8-warp classes), the autotuner's choice on the medium batch.
 constexpr uint32_t kDefaultClassBounds = 12u | (15u << 8) | (17u << 16) | (19u << 24);
 
+// The tile form takes the same limits: above the last, a net is a whole CTA's
+// from the start; the lower classes only size the slots of the slot workspace
+// (a net's warps there are its owner and whoever has none).  On the medium
+// batch (4096 nets, 4 x 2048^2) limits of 2^17 to 2^21 measured 11.3 to 12.8
+// ms, 2^19 best; all nets on whole CTAs 13.1.
+
 // Queue entries per list per frontier slot (a net needing more is rejected).
 constexpr uint64_t kMaxListEntries = 1ull << 25;
+// A frontier budget of this many rounds is no bound.
+constexpr uint32_t kUnboundedRounds = 1u << 30;
 // Frontier workspace above which nets share persistent slot slabs instead of
 // owning one slab each.
 constexpr uint64_t kPerNetFrontierBytes = 24ull << 30;
@@ -132,6 +141,15 @@ struct PlanObject {
   uint32_t wide_chain = 0;  // FRONTIER: apgar_b200_lattice_options::wide_chain
   uint32_t class_bounds = kDefaultClassBounds;  // FRONTIER: log2 class limits, byte per class
   bool per_net = false;  // FRONTIER: one slab per net (else persistent slots)
+  // FRONTIER, tile form: its own width classes, plan records and workspace
+  bool tiles = false;
+  bool tiles_per_net = false;
+  std::vector<ClassRange> tile_classes;
+  DeviceBuffer<NetPlan> tile_plans;
+  DeviceBuffer<uint32_t> tile_pool;
+  uint32_t tile_warps = 0;  // warps of a launch
+  std::vector<apgar_b200_lattice_net> host_nets;  // FRONTIER: the batch, as planned
+  std::vector<uint32_t> admitted;                 // FRONTIER: its admitted nets
   const uint32_t* cell_cost = nullptr;  // caller-owned device prices (frontier only)
   // partial rip-up (set by a negotiation): kept nets and their previous routes
   const uint8_t* skip = nullptr;
@@ -156,7 +174,9 @@ struct PlanObject {
   DeviceBuffer<uint32_t> paths;
   DeviceBuffer<unsigned long long> words;  // FRONTIER: label | ~round stamp per cell
   DeviceBuffer<uint32_t> lists;            // FRONTIER: three queue lists per net
-  // [0] arena cursor, [1] packed total, [2 + class] work-stealing cursors
+  // [0] arena cursor, [1] packed total, [2 + class] work-stealing cursors,
+  // [2 + kClassCount] finished nets, then (64-byte aligned) the tile form's net
+  // states
   DeviceBuffer<unsigned long long> counters;
   uint64_t label_cells = 0;
   uint64_t arena_capacity = 0;
@@ -175,9 +195,16 @@ struct PlanObject {
     if (cancel_host != nullptr) cudaFreeHost(cancel_host);
   }
 
+  // Counters and, for the tile form, a state per net.
+  size_t counter_words() const {
+    const size_t head = 2 + kClassCount + 6;
+    return tiles ? head + admitted.size() * (sizeof(TileNetState) / 8) : head;
+  }
+
   uint64_t workspace_bytes() const {
     return nets.bytes() + plans.bytes() + dist_pool.bytes() + results.bytes() + arena.bytes() +
-           paths.bytes() + counters.bytes() + words.bytes() + lists.bytes();
+           paths.bytes() + counters.bytes() + words.bytes() + lists.bytes() + tile_plans.bytes() +
+           tile_pool.bytes();
   }
 };
 
@@ -290,6 +317,173 @@ std::vector<uint32_t> sweep_planes(const uint32_t* in, int planes, int height, i
   return out;
 }
 
+// The admitted nets of a frontier batch by width class, largest windows first
+// (longest-processing-time order).
+std::vector<std::vector<uint32_t>> frontier_members(const PlanObject* plan, uint32_t bounds) {
+  std::vector<std::vector<uint32_t>> members(5);
+  const auto& nets = plan->host_nets;
+  const auto cells = [&](uint32_t i) { return static_cast<uint64_t>(nets[i].win_w) * nets[i].win_h; };
+  for (uint32_t i : plan->admitted) {
+    members[frontier_class(cells(i) * plan->lattice->view.layers, bounds)].push_back(i);
+  }
+  for (auto& m : members) {
+    std::stable_sort(m.begin(), m.end(), [&](uint32_t a, uint32_t b) { return cells(a) > cells(b); });
+  }
+  return members;
+}
+
+// Slot workspace within its budget: the class with the largest slot gives up
+// an eighth of its slots until the total fits (every class keeps at least
+// one; fewer slots only means fewer of its nets in flight).
+template <typename SlotBytes>
+void fit_slots(std::vector<ClassRange>& classes, uint64_t budget, SlotBytes slot_bytes) {
+  const auto total = [&]() {
+    uint64_t t = 0;
+    for (const ClassRange& c : classes) t += c.slots * slot_bytes(c);
+    return t;
+  };
+  while (total() > budget) {
+    ClassRange* widest = nullptr;
+    for (ClassRange& c : classes) {
+      if (c.slots > 1 && (widest == nullptr || slot_bytes(c) > slot_bytes(*widest))) widest = &c;
+    }
+    if (widest == nullptr) break;
+    widest->slots -= std::max<uint32_t>(1u, widest->slots / 8u);
+  }
+}
+
+uint64_t per_net_budget() { return budget_from_env("APGAR_B200_FRONTIER_PER_NET_BYTES", kPerNetFrontierBytes); }
+uint64_t slot_budget() { return budget_from_env("APGAR_B200_FRONTIER_SLOT_BYTES", kSlotFrontierBytes); }
+
+int upload_plans(DeviceBuffer<NetPlan>& dst, const std::vector<NetPlan>& plans) {
+  APGAR_B200_CUDA("cudaMalloc(plans)", dst.ensure(std::max<size_t>(plans.size(), 1)));
+  if (!plans.empty()) {
+    APGAR_B200_CUDA("cudaMemcpy(plans)", cudaMemcpy(dst.get(), plans.data(), plans.size() * sizeof(NetPlan),
+                                                    cudaMemcpyHostToDevice));
+  }
+  return APGAR_B200_OK;
+}
+
+// Classes, plan records and workspace of the cell form of the frontier
+// (lattice_frontier.cu).  Every net gets its own slab (8 B words + 3 x 4 B
+// list entries per cell) when that fits the per-net budget; otherwise the
+// persistent groups reuse their slot slabs net after net.
+int plan_cells(PlanObject* plan) {
+  const LatticeDeviceView& v = plan->lattice->view;
+  const auto members = frontier_members(plan, plan->class_bounds);
+  std::vector<NetPlan> plans;
+  plans.reserve(plan->admitted.size());
+  plan->classes.clear();
+  uint64_t net_cells = 0;  // padded window cells over all nets
+  for (int k = 0; k < 5; ++k) {
+    if (members[k].empty()) continue;
+    ClassRange range;
+    range.warps_per_net = 1 << k;
+    range.begin = static_cast<uint32_t>(plans.size());
+    range.count = static_cast<uint32_t>(members[k].size());
+    for (uint32_t i : members[k]) {
+      const apgar_b200_lattice_net& n = plan->host_nets[i];
+      NetPlan np{};
+      // window layout [layer][y][x] in the slot's slab, padded to 128 cells
+      np.net = i;
+      np.rows = n.win_h;
+      np.width = np.pitch = n.win_w;
+      const uint64_t padded = (static_cast<uint64_t>(v.layers) * n.win_w * n.win_h + 127ull) & ~127ull;
+      np.dist_offset = net_cells;  // used when every net gets its own slab
+      net_cells += padded;
+      range.slab_cells = std::max<uint64_t>(range.slab_cells, padded);
+      plans.push_back(np);
+    }
+    uint32_t resident = 0;
+    APGAR_B200_CUDA("cudaOccupancyMaxActiveBlocksPerMultiprocessor",
+                    lattice_frontier_resident_groups(range.warps_per_net, plan->sm_count, &resident));
+    range.slots = std::min<uint32_t>(resident, range.count);
+    range.list_cap = static_cast<uint32_t>(std::min<uint64_t>(range.slab_cells, kMaxListEntries));
+    // slot slabs are spaced by the largest window plus a 4 KB skew, so that
+    // equal offsets of different slots do not alias in the L2
+    range.slab_cells += 512;
+    plan->classes.push_back(range);
+  }
+  plan->per_net = net_cells * 20ull <= per_net_budget();
+  if (!plan->per_net) {
+    fit_slots(plan->classes, slot_budget(),
+              [](const ClassRange& c) { return c.slab_cells * 8ull + 12ull * c.list_cap; });
+  }
+  uint64_t words = 0, lists = 0;
+  for (ClassRange& range : plan->classes) {
+    range.words_offset = words;
+    words += static_cast<uint64_t>(range.slots) * range.slab_cells;
+    range.lists_offset = lists;
+    lists += static_cast<uint64_t>(range.slots) * 3ull * range.list_cap;
+  }
+  plan->label_cells = words;
+  if (plan->per_net) {
+    words = net_cells;
+    lists = 3ull * net_cells;
+  }
+  APGAR_B200_CUDA("cudaMalloc(label words)", plan->words.ensure(std::max<uint64_t>(words, 128)));
+  APGAR_B200_CUDA("cudaMalloc(queue lists)", plan->lists.ensure(std::max<uint64_t>(lists, 3)));
+  if (int rc = upload_plans(plan->plans, plans); rc != APGAR_B200_OK) return rc;
+  return APGAR_B200_OK;
+}
+
+// The same for the tile form (lattice_tiles.cu): about 4.1 B per window cell,
+// per net when that fits the per-net budget, else in slots.
+int plan_tiles(PlanObject* plan) {
+  const LatticeDeviceView& v = plan->lattice->view;
+  const auto members = frontier_members(plan, plan->class_bounds);
+  std::vector<NetPlan> plans;
+  plans.reserve(plan->admitted.size());
+  plan->tile_classes.clear();
+  APGAR_B200_CUDA("cudaOccupancyMaxActiveBlocksPerMultiprocessor",
+                  lattice_tile_warps(plan->sm_count, &plan->tile_warps));
+  uint64_t net_words = 0;
+  for (int k = 4; k >= 0; --k) {
+    if (members[k].empty()) continue;
+    ClassRange range;
+    range.warps_per_net = 1;
+    range.begin = static_cast<uint32_t>(plans.size());
+    range.count = static_cast<uint32_t>(members[k].size());
+    for (uint32_t i : members[k]) {
+      const apgar_b200_lattice_net& n = plan->host_nets[i];
+      NetPlan np{};
+      np.net = i;
+      np.dist_offset = net_words;  // used when every net gets its own workspace
+      const uint64_t words = lattice_tile_words(v.layers, n.win_w, n.win_h);
+      net_words += words;
+      range.slab_cells = std::max<uint64_t>(range.slab_cells, words);
+      plans.push_back(np);
+    }
+    range.warps_per_net = k == 4 ? 8 : 1;
+    range.slots = plan->tile_warps / static_cast<uint32_t>(range.warps_per_net);
+    plan->tile_classes.push_back(range);
+  }
+  plan->tiles_per_net = net_words * 4ull <= per_net_budget();
+  uint64_t words = net_words;
+  if (!plan->tiles_per_net) {
+    fit_slots(plan->tile_classes, slot_budget(), [](const ClassRange& c) { return c.slab_cells * 4ull; });
+    words = 0;
+    for (ClassRange& range : plan->tile_classes) {
+      range.words_offset = words;
+      words += static_cast<uint64_t>(range.slots) * range.slab_cells;
+    }
+  }
+  plan->label_cells = words;
+  APGAR_B200_CUDA("cudaMalloc(tile workspace)", plan->tile_pool.ensure(std::max<uint64_t>(words, 32)));
+  return upload_plans(plan->tile_plans, plans);
+}
+
+// Prices and corridors are the cell form's: a plan that gets either moves
+// over to it for good (and gives the tile form's workspace back first).
+int use_cells(PlanObject* plan) {
+  if (!plan->tiles) return APGAR_B200_OK;
+  APGAR_B200_CUDA("cudaDeviceSynchronize(tile form)", cudaDeviceSynchronize());
+  plan->tile_pool.reset();
+  plan->tile_plans.reset();
+  plan->tiles = false;
+  return plan_cells(plan);
+}
+
 // Builds (or rebuilds into existing buffers) a plan for `nets`.
 int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint32_t count,
                uint32_t max_sweeps, PlanObject* plan,
@@ -319,7 +513,12 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
                                          lat->device));
   const uint64_t max_move = std::max(v.orth, std::max(v.diag, v.via));
 
-  std::vector<std::vector<uint32_t>> members(kClassCount);
+  std::vector<std::vector<uint32_t>> members(kClassCount);  // SWEEP
+  uint64_t arena_cells = 0;
+  uint64_t largest = 0;  // FRONTIER: cells of the largest window
+  plan->admitted.clear();
+  plan->tiles = false;
+  plan->classes.clear();
   std::vector<apgar_b200_lattice_result> init(count);
   std::memset(init.data(), 0, init.size() * sizeof(apgar_b200_lattice_result));
   for (uint32_t i = 0; i < count; ++i) {
@@ -341,7 +540,9 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
     if (frontier) {
       // packed queue entries hold x and y in 14 bits each
       if (n.win_w > 16384u || n.win_h > 16384u) continue;
-      members[kFrontierClasses[frontier_class(cells, plan->class_bounds)]].push_back(i);
+      plan->admitted.push_back(i);
+      arena_cells += 8ull * (n.win_w + n.win_h) + 64ull * v.layers;
+      largest = std::max(largest, cells);
       continue;
     }
     const uint32_t frame_width = std::max(n.win_w, n.win_h);
@@ -354,11 +555,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
 
   std::vector<NetPlan> plans;
   plans.reserve(count);
-  plan->classes.clear();
   uint64_t dist_cells = 0;
-  uint64_t arena_cells = 0;
-  uint64_t arena_lists = 0;    // frontier queue entries over all slots
-  uint64_t per_net_cells = 0;  // frontier: padded window cells over all nets
   for (int ci = 0; ci < kClassCount; ++ci) {
     std::vector<uint32_t>& m = members[ci];
     if (m.empty()) continue;
@@ -376,96 +573,42 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
       const apgar_b200_lattice_net& n = host_nets[i];
       NetPlan np{};
       np.net = i;
-      if (frontier) {
-        // window layout [layer][y][x] in the slot's slab, padded to 128 cells
-        np.transposed = 0;
-        np.rows = n.win_h;
-        np.width = n.win_w;
-        np.pitch = n.win_w;
-        const uint64_t padded = (static_cast<uint64_t>(v.layers) * n.win_w * n.win_h + 127ull) & ~127ull;
-        np.dist_offset = per_net_cells;  // used when every net gets its own slab
-        per_net_cells += padded;
-        range.slab_cells = std::max<uint64_t>(range.slab_cells, padded);
-      } else {
-        np.transposed = n.win_h > n.win_w ? 1u : 0u;
-        np.rows = np.transposed ? n.win_w : n.win_h;
-        np.width = np.transposed ? n.win_h : n.win_w;
-        np.pitch = (np.width + 3u) & ~3u;
-        np.dist_offset = dist_cells;
-        dist_cells += static_cast<uint64_t>(v.layers) * np.rows * np.pitch;
-      }
+      np.transposed = n.win_h > n.win_w ? 1u : 0u;
+      np.rows = np.transposed ? n.win_w : n.win_h;
+      np.width = np.transposed ? n.win_h : n.win_w;
+      np.pitch = (np.width + 3u) & ~3u;
+      np.dist_offset = dist_cells;
+      dist_cells += static_cast<uint64_t>(v.layers) * np.rows * np.pitch;
       arena_cells += 8ull * (n.win_w + n.win_h) + 64ull * v.layers;
       range.max_rows = std::max(range.max_rows, static_cast<int>(np.rows));
       plans.push_back(np);
     }
-    if (!frontier && lattice_sweep_smem_bytes(v.layers, range.warps_per_net, range.max_rows) >
-                         kMaxSmemPerBlock) {
+    if (lattice_sweep_smem_bytes(v.layers, range.warps_per_net, range.max_rows) > kMaxSmemPerBlock) {
       return set_error(APGAR_B200_UNSUPPORTED, "window too tall for the shared-memory row map");
-    }
-    if (frontier) {
-      uint32_t resident = 0;
-      APGAR_B200_CUDA("cudaOccupancyMaxActiveBlocksPerMultiprocessor",
-                      lattice_frontier_resident_groups(range.warps_per_net, plan->sm_count, &resident));
-      range.slots = std::min<uint32_t>(resident, range.count);
-      range.list_cap = static_cast<uint32_t>(std::min<uint64_t>(range.slab_cells, kMaxListEntries));
-      // slot slabs are spaced by the largest window plus a 4 KB skew, so that
-      // equal offsets of different slots do not alias in the L2
-      range.slab_cells += 512;
     }
     plan->classes.push_back(range);
   }
-  const uint64_t per_net_budget = budget_from_env("APGAR_B200_FRONTIER_PER_NET_BYTES", kPerNetFrontierBytes);
-  const uint64_t slot_budget = budget_from_env("APGAR_B200_FRONTIER_SLOT_BYTES", kSlotFrontierBytes);
-  if (frontier && per_net_cells * 20ull > per_net_budget) {
-    // Slot workspace within its budget: the class with the largest slot
-    // gives up an eighth of its slots until the total fits (every class keeps
-    // at least one; fewer slots only means fewer of its nets in flight).
-    const auto slot_bytes = [](const ClassRange& c) { return c.slab_cells * 8ull + 12ull * c.list_cap; };
-    const auto total = [&]() {
-      uint64_t t = 0;
-      for (const ClassRange& c : plan->classes) t += c.slots * slot_bytes(c);
-      return t;
-    };
-    while (total() > slot_budget) {
-      ClassRange* widest = nullptr;
-      for (ClassRange& c : plan->classes) {
-        if (c.slots > 1 && (widest == nullptr || slot_bytes(c) > slot_bytes(*widest))) widest = &c;
-      }
-      if (widest == nullptr) break;
-      widest->slots -= std::max<uint32_t>(1u, widest->slots / 8u);
-    }
-  }
-  if (frontier) {
-    for (ClassRange& range : plan->classes) {
-      range.words_offset = dist_cells;
-      dist_cells += static_cast<uint64_t>(range.slots) * range.slab_cells;
-      range.lists_offset = arena_lists;
-      arena_lists += static_cast<uint64_t>(range.slots) * 3ull * range.list_cap;
-    }
-  }
-  plan->label_cells = dist_cells;
+  if (!frontier) plan->label_cells = dist_cells;
   plan->arena_capacity = std::max<uint64_t>(arena_cells, 64);
 
   APGAR_B200_CUDA("cudaMalloc(nets)", plan->nets.ensure(std::max<uint32_t>(count, 1)));
-  APGAR_B200_CUDA("cudaMalloc(plans)", plan->plans.ensure(std::max<size_t>(plans.size(), 1)));
   if (frontier) {
-    // Every net gets its own slab (8 B words + 3 x 4 B list entries per
-    // cell) when that fits the per-net budget; otherwise the persistent
-    // groups reuse their slot slabs net after net.
-    plan->per_net = per_net_cells * 20ull <= per_net_budget;
-    if (plan->per_net) {
-      dist_cells = per_net_cells;
-      arena_lists = 3ull * per_net_cells;
-    }
-    APGAR_B200_CUDA("cudaMalloc(label words)", plan->words.ensure(std::max<uint64_t>(dist_cells, 128)));
-    APGAR_B200_CUDA("cudaMalloc(queue lists)", plan->lists.ensure(std::max<uint64_t>(arena_lists, 3)));
+    plan->host_nets.assign(host_nets, host_nets + count);
+    // The tile form serves a plan whose schedule it can keep: no bound on the
+    // rounds (its rounds are not the cell form's), no chained expansions, and
+    // no window whose queue lists the cell form may cut (a net that outgrows
+    // them is rejected) or whose labels could reach the tile form's limit.
+    plan->tiles = max_sweeps == kUnboundedRounds && plan->chain <= 1u && plan->wide_chain <= 1u &&
+                  largest <= kMaxListEntries && largest * max_move < kTileLabelLimit;
+    if (int rc = plan->tiles ? plan_tiles(plan) : plan_cells(plan); rc != APGAR_B200_OK) return rc;
   } else {
     APGAR_B200_CUDA("cudaMalloc(label slabs)", plan->dist_pool.ensure(std::max<uint64_t>(dist_cells, 4)));
+    if (int rc = upload_plans(plan->plans, plans); rc != APGAR_B200_OK) return rc;
   }
   APGAR_B200_CUDA("cudaMalloc(results)", plan->results.ensure(std::max<uint32_t>(count, 1)));
   APGAR_B200_CUDA("cudaMalloc(path arena)", plan->arena.ensure(plan->arena_capacity));
   APGAR_B200_CUDA("cudaMalloc(paths)", plan->paths.ensure(plan->arena_capacity));
-  APGAR_B200_CUDA("cudaMalloc(counters)", plan->counters.ensure(2 + kClassCount));
+  APGAR_B200_CUDA("cudaMalloc(counters)", plan->counters.ensure(plan->counter_words()));
   if (count > 0) {
     APGAR_B200_CUDA("cudaMemcpy(nets)",
                     cudaMemcpy(plan->nets.get(), host_nets, count * sizeof(apgar_b200_lattice_net),
@@ -473,11 +616,6 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
     APGAR_B200_CUDA("cudaMemcpy(results init)",
                     cudaMemcpy(plan->results.get(), init.data(),
                                count * sizeof(apgar_b200_lattice_result), cudaMemcpyHostToDevice));
-  }
-  if (!plans.empty()) {
-    APGAR_B200_CUDA("cudaMemcpy(plans)",
-                    cudaMemcpy(plan->plans.get(), plans.data(), plans.size() * sizeof(NetPlan),
-                               cudaMemcpyHostToDevice));
   }
   int least_priority = 0, greatest_priority = 0;
   APGAR_B200_CUDA("cudaDeviceGetStreamPriorityRange",
@@ -516,7 +654,7 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
   if (int rc = check_device(plan->device); rc != APGAR_B200_OK) return rc;
   APGAR_B200_CUDA("cudaMemsetAsync(counters)",
                   cudaMemsetAsync(plan->counters.get(), 0,
-                                  (2 + kClassCount) * sizeof(unsigned long long), stream));
+                                  plan->counter_words() * sizeof(unsigned long long), stream));
   const LatticeDeviceView& v = plan->lattice->view;
   FrontierLaunch fbase{};
   fbase.lat = v;
@@ -538,6 +676,38 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
   if (plan->corridor != nullptr) {
     fbase.corridor = plan->corridor;
     fbase.corridor_status = plan->corridor_status.get();
+  }
+  if (plan->tiles) {
+    TileLaunch t{};
+    t.lat = v;
+    t.nets = plan->nets.get();
+    t.per_net = plan->tiles_per_net ? 1u : 0u;
+    t.results = plan->results.get();
+    t.path_arena = plan->arena.get();
+    t.path_arena_capacity = plan->arena_capacity;
+    t.arena_cursor = plan->counters.get();
+    t.cancel = plan->cancel_dev;
+    t.finished = reinterpret_cast<unsigned int*>(plan->counters.get() + 2 + kClassCount);
+    t.plans = plan->tile_plans.get();
+    t.states = reinterpret_cast<TileNetState*>(plan->counters.get() + 2 + kClassCount + 6);
+    t.total = static_cast<uint32_t>(plan->admitted.size());
+    for (TileClass& c : t.c) c.pool = plan->tile_pool.get();
+    for (size_t k = 0; k < plan->tile_classes.size(); ++k) {
+      const ClassRange& c = plan->tile_classes[k];
+      t.c[k].pool = plan->tile_pool.get() + c.words_offset;
+      t.c[k].slot_words = c.slab_cells;
+      t.c[k].begin = c.begin;
+      t.c[k].end = c.begin + c.count;
+      t.c[k].slots = c.slots;
+      t.c[k].team = c.warps_per_net > 1 ? 1u : 0u;
+      t.c[k].level_width = c.warps_per_net > 1 ? plan->wide_bucket_width : plan->bucket_width;
+      t.c[k].next_plan = reinterpret_cast<unsigned int*>(plan->counters.get() + 2 + k);
+    }
+    APGAR_B200_CUDA("lattice tiles launch", launch_lattice_tiles(t, plan->sm_count, stream));
+    APGAR_B200_CUDA("lattice pack launch",
+                    launch_lattice_pack(plan->results.get(), plan->count, plan->counters.get() + 1,
+                                        plan->arena.get(), plan->paths.get(), plan->sm_count, stream));
+    return APGAR_B200_OK;
   }
   SweepLaunch base{};
   base.lat = v;
@@ -793,6 +963,10 @@ extern "C" int apgar_b200_lattice_plan_set_cell_costs(void* plan, const uint32_t
   if (cell_costs != nullptr && p->generator != APGAR_B200_LATTICE_FRONTIER) {
     return set_error(APGAR_B200_UNSUPPORTED, "per-cell prices need the frontier generator");
   }
+  if (cell_costs != nullptr) {
+    if (int rc = check_device(p->device); rc != APGAR_B200_OK) return rc;
+    if (int rc = use_cells(p); rc != APGAR_B200_OK) return rc;
+  }
   p->cell_cost = cell_costs;
   clear_error();
   return APGAR_B200_OK;
@@ -806,6 +980,7 @@ extern "C" int apgar_b200_lattice_plan_set_corridors(void* plan, const uint32_t*
       return set_error(APGAR_B200_UNSUPPORTED, "corridors need the frontier generator");
     }
     if (int rc = check_device(p->device); rc != APGAR_B200_OK) return rc;
+    if (int rc = use_cells(p); rc != APGAR_B200_OK) return rc;
     APGAR_B200_CUDA("cudaMalloc(corridor status)",
                     p->corridor_status.ensure(std::max<uint32_t>(p->count, 1)));
   }
@@ -902,7 +1077,7 @@ extern "C" int apgar_b200_lattice_plan_info(void* plan, apgar_b200_plan_info* ou
   auto* p = static_cast<PlanObject*>(plan);
   std::memset(out, 0, sizeof(*out));
   out->net_count = p->count;
-  out->class_count = static_cast<uint32_t>(p->classes.size());
+  out->class_count = static_cast<uint32_t>(p->tiles ? p->tile_classes.size() : p->classes.size());
   // the frontier runs all its classes in one launch; the sweep one per class
   const uint32_t search_launches =
       p->generator == APGAR_B200_LATTICE_FRONTIER ? (out->class_count > 0 ? 1u : 0u) : out->class_count;
@@ -1527,6 +1702,7 @@ extern "C" int apgar_b200_negotiation_create(void* plan, const apgar_b200_price_
     return set_error(APGAR_B200_UNSUPPORTED, "lattice has more cells than a price pass indexes");
   }
   try {
+    if (int rc = use_cells(p); rc != APGAR_B200_OK) return rc;
     auto n = std::make_unique<NegotiationObject>();
     n->plan = p;
     n->policy = *policy;

@@ -517,13 +517,16 @@ APGAR_B200_API int apgar_b200_lattice_plan_info(void* plan, apgar_b200_plan_info
  *  SWEEP:    alternating row sweeps to the full-window fixed point.  Result
  *            counters: sweeps, row_steps, row_stores, row_loads.
  *  FRONTIER: bucketed, label-correcting A* (key = label + octile-plus-via
- *            bound) in key levels of `bucket_width`.  One warp group per net,
- *            persistent and work-stealing, largest windows first.  It stops
- *            once every cell with key <= the goal label is final.  Result
- *            counters: sweeps = rounds, row_steps = cell expansions,
- *            row_stores = key levels opened, row_loads = 0.  Rounds and
- *            expansions depend on the order of concurrent relaxations;
- *            costs and paths do not. */
+ *            bound) in key levels of `bucket_width`, persistent and
+ *            work-stealing, largest windows first.  It stops once every cell
+ *            with key <= the goal label is final.  Two forms: over 32 x 32
+ *            tiles (plans without a bound on the rounds, chains, prices or
+ *            corridors, and without windows above 2^25 cells), and over
+ *            single cells (the rest), one warp group per net.  Result
+ *            counters, tiles / cells: sweeps = units relaxed / rounds,
+ *            row_steps = line steps of 32 cells / cell expansions,
+ *            row_stores = key levels opened, row_loads = 0.  They depend on
+ *            the order of concurrent relaxations; costs and paths do not. */
 #define APGAR_B200_LATTICE_SWEEP 0u
 #define APGAR_B200_LATTICE_FRONTIER 1u
 typedef struct apgar_b200_lattice_options {
@@ -538,7 +541,9 @@ typedef struct apgar_b200_lattice_options {
   uint32_t class_bounds;   /* FRONTIER: width classes of 1, 2, 4, 8 and 16 warps per net;
                               byte k (k = 0..3) is log2 of the largest window (cells over
                               all layers) of the 2^k-warp class, strictly increasing in
-                              1..31; larger windows take 16 warps.  0 = the default
+                              1..31; larger windows take 16 warps.  (Over tiles, larger
+                              windows take a whole CTA from the start, all others one
+                              warp and whoever is idle.)  0 = the default
                               0x13110F0C (2^12, 2^15, 2^17, 2^19).  Results do not
                               depend on it. */
   uint32_t wide_bucket_width; /* FRONTIER: key width of the 16-warp class's levels (its
