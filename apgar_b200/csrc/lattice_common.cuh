@@ -154,8 +154,11 @@ struct TileNetState {
   uint32_t slot;          // workspace slot (slot mode)
   uint32_t guests;        // warps that help the owner
   uint32_t level_width;
+  uint32_t limit;         // keys above it no longer matter
+  uint32_t start_key;     // the start's key
+  uint32_t reserved[14];
 };
-static_assert(sizeof(TileNetState) == 64, "states are carved from the counters, 64 bytes each");
+static_assert(sizeof(TileNetState) == 128, "a line of its own per net: its warps' atomics and looks meet there");
 
 // One size class of the tile form of the frontier (lattice_tiles.cu): net
 // workspaces (lattice_tile_words 32-bit words) at pool + plan.dist_offset
@@ -183,6 +186,17 @@ struct TileLaunch {
   unsigned long long* arena_cursor;
   const volatile uint32_t* cancel;
   unsigned int* finished;  // nets that are done
+  // prices, kept routes and rip-up pricing, as in FrontierLaunch; own_bits is
+  // one bit per label word of the pool.  A net whose prices or labels come
+  // near the 32-bit limit goes to `redo` (the cell form then decides it).
+  const uint32_t* cell_cost;
+  const uint32_t* cell_cost_own;
+  uint32_t* own_bits;
+  const uint8_t* skip;
+  const apgar_b200_lattice_result* prev_results;
+  const uint32_t* prev_paths;
+  NetPlan* redo;
+  uint32_t* redo_count;
   TileClass c[5];          // the widest first
 };
 

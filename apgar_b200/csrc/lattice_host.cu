@@ -75,6 +75,7 @@ namespace {
 constexpr int kGroupSizes[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16};
 constexpr int kClassCount = 16;
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;
+constexpr size_t kStatesAt = 32;  // of PlanObject::counters (256 bytes on: the states are 128 bytes each)
 
 struct LatticeObject;
 
@@ -148,6 +149,12 @@ struct PlanObject {
   DeviceBuffer<NetPlan> tile_plans;
   DeviceBuffer<uint32_t> tile_pool;
   uint32_t tile_warps = 0;  // warps of a launch
+  // FRONTIER, tile form with prices: nets whose prices or labels come near the
+  // 32-bit limit, and the slots (in words and lists) of their cell-form search
+  DeviceBuffer<NetPlan> redo;
+  DeviceBuffer<uint32_t> redo_own;
+  uint32_t redo_slots = 0;
+  uint64_t redo_cells = 0;
   std::vector<apgar_b200_lattice_net> host_nets;  // FRONTIER: the batch, as planned
   std::vector<uint32_t> admitted;                 // FRONTIER: its admitted nets
   const uint32_t* cell_cost = nullptr;  // caller-owned device prices (frontier only)
@@ -175,8 +182,8 @@ struct PlanObject {
   DeviceBuffer<unsigned long long> words;  // FRONTIER: label | ~round stamp per cell
   DeviceBuffer<uint32_t> lists;            // FRONTIER: three queue lists per net
   // [0] arena cursor, [1] packed total, [2 + class] work-stealing cursors,
-  // [2 + kClassCount] finished nets, then (64-byte aligned) the tile form's net
-  // states
+  // [2 + kClassCount] the tile form's finished nets, nets handed over and their
+  // cursor, then its net states
   DeviceBuffer<unsigned long long> counters;
   uint64_t label_cells = 0;
   uint64_t arena_capacity = 0;
@@ -197,14 +204,14 @@ struct PlanObject {
 
   // Counters and, for the tile form, a state per net.
   size_t counter_words() const {
-    const size_t head = 2 + kClassCount + 6;
+    const size_t head = kStatesAt;
     return tiles ? head + admitted.size() * (sizeof(TileNetState) / 8) : head;
   }
 
   uint64_t workspace_bytes() const {
     return nets.bytes() + plans.bytes() + dist_pool.bytes() + results.bytes() + arena.bytes() +
            paths.bytes() + counters.bytes() + words.bytes() + lists.bytes() + tile_plans.bytes() +
-           tile_pool.bytes();
+           tile_pool.bytes() + redo.bytes() + redo_own.bytes();
   }
 };
 
@@ -473,13 +480,44 @@ int plan_tiles(PlanObject* plan) {
   return upload_plans(plan->tile_plans, plans);
 }
 
-// Prices and corridors are the cell form's: a plan that gets either moves
-// over to it for good (and gives the tile form's workspace back first).
+// Workspace budget of the nets that a priced tile search hands over.
+constexpr uint64_t kRedoBytes = 256ull << 20;
+
+int use_cells(PlanObject* plan);
+
+// Prices on a tile plan: a place for the nets whose prices or labels come
+// near the 32-bit limit, which the cell form then decides.  (Its rejections
+// depend on the level width, so one width for all nets is needed.)
+int use_prices(PlanObject* plan) {
+  if (!plan->tiles || plan->redo_slots != 0) return APGAR_B200_OK;
+  if (plan->wide_bucket_width != plan->bucket_width) return use_cells(plan);
+  uint64_t cells = 0;
+  for (uint32_t i : plan->admitted) {
+    const apgar_b200_lattice_net& n = plan->host_nets[i];
+    cells = std::max(cells, static_cast<uint64_t>(plan->lattice->view.layers) * n.win_w * n.win_h);
+  }
+  cells = ((cells + 127ull) & ~127ull) + 512ull;
+  const uint64_t slots = std::min<uint64_t>(std::max<uint64_t>(kRedoBytes / (cells * 20ull), 1),
+                                            std::max<size_t>(plan->admitted.size(), 1));
+  plan->redo_cells = cells;
+  APGAR_B200_CUDA("cudaMalloc(handed over nets)", plan->redo.ensure(std::max<size_t>(plan->admitted.size(), 1)));
+  plan->redo_slots = static_cast<uint32_t>(std::min<uint64_t>(slots, static_cast<uint64_t>(plan->sm_count)));
+  APGAR_B200_CUDA("cudaMalloc(label words)", plan->words.ensure(plan->redo_slots * cells));
+  APGAR_B200_CUDA("cudaMalloc(queue lists)", plan->lists.ensure(plan->redo_slots * 3ull * cells));
+  APGAR_B200_CUDA("cudaMalloc(own-route bits)", plan->redo_own.ensure(plan->redo_slots * cells / 32 + 1));
+  return APGAR_B200_OK;
+}
+
+// Corridors are the cell form's: a plan that gets them moves over to it for
+// good (and gives the tile form's workspace back first).
 int use_cells(PlanObject* plan) {
   if (!plan->tiles) return APGAR_B200_OK;
   APGAR_B200_CUDA("cudaDeviceSynchronize(tile form)", cudaDeviceSynchronize());
   plan->tile_pool.reset();
   plan->tile_plans.reset();
+  plan->redo.reset();
+  plan->redo_own.reset();
+  plan->redo_slots = 0;
   plan->tiles = false;
   return plan_cells(plan);
 }
@@ -518,6 +556,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
   uint64_t largest = 0;  // FRONTIER: cells of the largest window
   plan->admitted.clear();
   plan->tiles = false;
+  plan->redo_slots = 0;
   plan->classes.clear();
   std::vector<apgar_b200_lattice_result> init(count);
   std::memset(init.data(), 0, init.size() * sizeof(apgar_b200_lattice_result));
@@ -689,7 +728,7 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
     t.cancel = plan->cancel_dev;
     t.finished = reinterpret_cast<unsigned int*>(plan->counters.get() + 2 + kClassCount);
     t.plans = plan->tile_plans.get();
-    t.states = reinterpret_cast<TileNetState*>(plan->counters.get() + 2 + kClassCount + 6);
+    t.states = reinterpret_cast<TileNetState*>(plan->counters.get() + kStatesAt);
     t.total = static_cast<uint32_t>(plan->admitted.size());
     for (TileClass& c : t.c) c.pool = plan->tile_pool.get();
     for (size_t k = 0; k < plan->tile_classes.size(); ++k) {
@@ -703,7 +742,29 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
       t.c[k].level_width = c.warps_per_net > 1 ? plan->wide_bucket_width : plan->bucket_width;
       t.c[k].next_plan = reinterpret_cast<unsigned int*>(plan->counters.get() + 2 + k);
     }
+    t.cell_cost = plan->cell_cost;
+    t.cell_cost_own = plan->cell_cost_own;
+    t.own_bits = plan->own_bits;
+    t.skip = plan->skip;
+    t.prev_results = plan->prev_results;
+    t.prev_paths = plan->prev_paths;
+    t.redo = plan->redo.get();
+    t.redo_count = reinterpret_cast<uint32_t*>(plan->counters.get() + 2 + kClassCount + 1);
     APGAR_B200_CUDA("lattice tiles launch", launch_lattice_tiles(t, plan->sm_count, stream));
+    if (plan->cell_cost != nullptr) {
+      FrontierClasses fc{};
+      FrontierLaunch& fl = fc.c[4];
+      fl = fbase;
+      fl.plans = plan->redo.get();
+      fl.plan_count_dev = t.redo_count;
+      fl.skip = nullptr;
+      fl.slab_cells = plan->redo_cells;
+      fl.list_cap = static_cast<uint32_t>(plan->redo_cells);
+      fl.slots = plan->redo_slots;
+      fl.own_bits = plan->cell_cost_own != nullptr ? plan->redo_own.get() : nullptr;
+      fl.next_plan = reinterpret_cast<unsigned int*>(plan->counters.get() + 2 + kClassCount + 2);
+      APGAR_B200_CUDA("lattice frontier launch", launch_lattice_frontier(fc, plan->sm_count, stream));
+    }
     APGAR_B200_CUDA("lattice pack launch",
                     launch_lattice_pack(plan->results.get(), plan->count, plan->counters.get() + 1,
                                         plan->arena.get(), plan->paths.get(), plan->sm_count, stream));
@@ -965,7 +1026,7 @@ extern "C" int apgar_b200_lattice_plan_set_cell_costs(void* plan, const uint32_t
   }
   if (cell_costs != nullptr) {
     if (int rc = check_device(p->device); rc != APGAR_B200_OK) return rc;
-    if (int rc = use_cells(p); rc != APGAR_B200_OK) return rc;
+    if (int rc = use_prices(p); rc != APGAR_B200_OK) return rc;
   }
   p->cell_cost = cell_costs;
   clear_error();
@@ -1568,6 +1629,7 @@ struct NegotiationObject {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   uint32_t graph_rounds = 0;
+  bool form_tiles = false;  // the plan's form when own_bits was sized
   // split-round steps: the next (round, phase) a step may run
   uint32_t step_round = 0, step_phase = 0;
 
@@ -1589,6 +1651,25 @@ struct NegotiationObject {
     }
   }
 };
+
+// One own-route bit per label word of the plan's form (which set_corridors
+// may have changed since; a captured run is then captured again).
+int ensure_own_bits(NegotiationObject* n) {
+  const PlanObject* p = n->plan;
+  const size_t words = (p->tiles ? p->tile_pool.count() : p->words.count()) / 32 + 1;
+  if (words > n->own_bits.count()) {
+    APGAR_B200_CUDA("cudaDeviceSynchronize(own-route bits)", cudaDeviceSynchronize());
+    APGAR_B200_CUDA("cudaMalloc(own-route bits)", n->own_bits.ensure(words));
+  }
+  if (n->form_tiles != p->tiles && n->exec != nullptr) {
+    cudaGraphExecDestroy(n->exec);
+    cudaGraphDestroy(n->graph);
+    n->exec = nullptr;
+    n->graph = nullptr;
+  }
+  n->form_tiles = p->tiles;
+  return APGAR_B200_OK;
+}
 
 bool checked_factor(const apgar_b200_price_policy& p, uint64_t epoch, uint64_t* out) {
   const unsigned __int128 f =
@@ -1702,7 +1783,7 @@ extern "C" int apgar_b200_negotiation_create(void* plan, const apgar_b200_price_
     return set_error(APGAR_B200_UNSUPPORTED, "lattice has more cells than a price pass indexes");
   }
   try {
-    if (int rc = use_cells(p); rc != APGAR_B200_OK) return rc;
+    if (int rc = use_prices(p); rc != APGAR_B200_OK) return rc;
     auto n = std::make_unique<NegotiationObject>();
     n->plan = p;
     n->policy = *policy;
@@ -1710,7 +1791,7 @@ extern "C" int apgar_b200_negotiation_create(void* plan, const apgar_b200_price_
     APGAR_B200_CUDA("cudaMalloc(usage)", n->usage.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(cell costs)", n->cell_cost.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(own-route cell costs)", n->cell_cost_own.ensure(cells));
-    APGAR_B200_CUDA("cudaMalloc(own-route bits)", n->own_bits.ensure(p->words.count() / 32 + 1));
+    if (int rc = ensure_own_bits(n.get()); rc != APGAR_B200_OK) return rc;
     APGAR_B200_CUDA("cudaMalloc(history)", n->history.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(previous results)", n->prev_results.ensure(std::max<uint32_t>(p->count, 1)));
     APGAR_B200_CUDA("cudaMalloc(previous paths)", n->prev_paths.ensure(std::max<uint64_t>(p->arena_capacity, 1)));
@@ -1742,6 +1823,7 @@ extern "C" int apgar_b200_negotiation_run_ex(void* negotiation, uint32_t rounds,
     APGAR_B200_CUDA("cudaMalloc(round stats)", n->stats.ensure(2ull * rounds));
     n->rounds_capacity = rounds;
   }
+  if (int rc = ensure_own_bits(n); rc != APGAR_B200_OK) return rc;
   // work runs on the negotiation's own stream, ordered after the caller's
   APGAR_B200_CUDA("cudaEventRecord(entry)", cudaEventRecord(n->entry, caller));
   APGAR_B200_CUDA("cudaStreamWaitEvent", cudaStreamWaitEvent(n->work, n->entry, 0));
@@ -1825,6 +1907,7 @@ extern "C" int apgar_b200_negotiation_step(void* negotiation, uint32_t round, ui
     APGAR_B200_CUDA("cudaMalloc(round stats)", n->stats.ensure(2ull * kMaxStepRounds));
     n->rounds_capacity = kMaxStepRounds;
   }
+  if (int rc = ensure_own_bits(n); rc != APGAR_B200_OK) return rc;
   const auto caller = static_cast<cudaStream_t>(stream);
   APGAR_B200_CUDA("cudaEventRecord(entry)", cudaEventRecord(n->entry, caller));
   APGAR_B200_CUDA("cudaStreamWaitEvent", cudaStreamWaitEvent(n->work, n->entry, 0));

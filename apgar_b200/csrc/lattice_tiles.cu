@@ -55,6 +55,12 @@ constexpr int kPitch = 35;                  // odd: rows and columns are both co
 constexpr int kTileWords = 34 * kPitch + 2;  // 32 x 32 labels with their rim
 constexpr int kQuadWords = 66;              // 33 rows of 64-bit 2 x 2 freedom bits (path walk)
 constexpr int kWarpWords = kTileWords + kQuadWords;
+constexpr int kPricePitch = 33;
+constexpr int kPriceWords = 32 * kPricePitch;  // prices of the unit's cells
+// Prices and labels below this cannot reach the 32-bit limit in a move; a net
+// that meets one above it is searched by the cell form instead.
+constexpr uint32_t kPriceLimit = 1u << 29;
+constexpr uint32_t kNoLimit = 0xFFFFFFFDu;
 constexpr uint32_t kTileInf = kTileLabelLimit;  // no label yet
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;     // pending key of an idle unit
 constexpr uint32_t kBusyKey = 0xFFFFFFFEu;   // of a unit being relaxed
@@ -328,9 +334,10 @@ struct Swept {
 // source's lane's cell of this line, which that lane checks before it hands
 // its label over.  The outermost lanes get their own label back from a
 // shuffle; p + diag is then no better than the straight p + orth, unless a
-// diagonal is cheaper than a straight move (kCheapDiagonal).
-template <int kStride, bool kCheapDiagonal>
-__device__ __forceinline__ Swept sweep_lines(uint32_t* cell, uint32_t blocked, uint32_t need, uint32_t orth,
+// diagonal is cheaper than a straight move (kCheapDiagonal).  Priced, every
+// move into a cell also costs price + i * kPriceStride.
+template <int kStride, int kPriceStride, bool kCheapDiagonal, bool kPriced>
+__device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* price, uint32_t blocked, uint32_t need, uint32_t orth,
                                              uint32_t diag, int lane, uint32_t& steps) {
   Swept out{0u, 0u, 0u};
   uint32_t pair = blocked | (blocked << 1);
@@ -350,8 +357,14 @@ __device__ __forceinline__ Swept sweep_lines(uint32_t* cell, uint32_t blocked, u
           if (lane == 0) before = kTileInf;
           if (lane == 31) after = kTileInf;
         }
-        uint32_t t = __viaddmin_u32(given, orth, v[k]);
-        t = __viaddmin_u32(unless(pair, k, min(before, after)), diag, t);
+        uint32_t t;
+        if constexpr (kPriced) {
+          t = __viaddmin_u32(unless(pair, k, min(before, after)), diag, given + orth);
+          t = __viaddmin_u32(min(t, kTileInf), price[k * kPriceStride], v[k]);
+        } else {
+          t = __viaddmin_u32(given, orth, v[k]);
+          t = __viaddmin_u32(unless(pair, k, min(before, after)), diag, t);
+        }
         cell[k * kStride] = t;
         diff |= t ^ v[k];
         if (k == 0) first = diff;
@@ -368,6 +381,7 @@ __device__ __forceinline__ Swept sweep_lines(uint32_t* cell, uint32_t blocked, u
       steps += 8;
     }
     cell += 8 * kStride;
+    price += 8 * kPriceStride;
     blocked >>= 8;
     pair >>= 8;
   }
@@ -375,13 +389,16 @@ __device__ __forceinline__ Swept sweep_lines(uint32_t* cell, uint32_t blocked, u
 }
 
 // The moves from one side's rim into its line of cells: line and rim are this
-// lane's cells, lane_step the distance to the next lane's.
+// lane's cells, lane_step the distance to the next lane's; price is that of
+// entering the lane's cell.
+template <bool kPriced>
 __device__ __forceinline__ bool enter_side(uint32_t* line, const uint32_t* rim, int lane_step, uint32_t legal,
-                                           bool is_free, uint32_t orth, uint32_t diag) {
+                                           bool is_free, uint32_t price, uint32_t orth, uint32_t diag) {
   const uint32_t v = *line;
-  uint32_t t = __viaddmin_u32(unless(~legal, 0, rim[-lane_step]), diag, v);
+  uint32_t t = __viaddmin_u32(unless(~legal, 0, rim[-lane_step]), diag, rim[0] + orth);
   t = __viaddmin_u32(unless(~legal, 1, rim[lane_step]), diag, t);
-  t = __viaddmin_u32(rim[0], orth, t);
+  if constexpr (kPriced) t = min(t, kTileInf) + price;
+  t = min(t, v);
   if (is_free) *line = t;
   return is_free && t != v;
 }
@@ -403,6 +420,7 @@ struct Space {
   uint32_t* ring;
   uint32_t ring_mask;
   uint32_t far_cap;
+  uint32_t* own;  // own-route bits, a word per unit row; nullptr without rip-up pricing
 };
 
 // Slots of a net's ring: a power of two that holds every unit once.
@@ -422,6 +440,7 @@ __device__ __forceinline__ Space space_at(uint32_t* base, uint32_t units) {
   ws.ring = ws.far[1] + units;
   ws.ring_mask = ring_slots(units) - 1u;
   ws.far_cap = units;
+  ws.own = nullptr;
   return ws;
 }
 
@@ -508,13 +527,13 @@ __device__ __forceinline__ uint32_t touched_neighbours(const Space& ws, const La
 __device__ __noinline__ void open_level(int tx, int ty, Space ws, TileNetState* st, int lane) {
   for (;;) {
     __threadfence();
-    const uint32_t par = peek(&st->far_par), waiting = min(peek(&st->far_count[par]), ws.far_cap), limit = peek(&st->goal);
+    const uint32_t par = peek(&st->far_par), waiting = min(peek(&st->far_count[par]), ws.far_cap), limit = peek(&st->limit);
     uint32_t least = kNoKey;
     for (uint32_t i = lane; i < waiting; i += 32) {
       least = min(least, __ldcg(ws.pend + unit_id(tx, ty, __ldcg(ws.far[par] + i))));
     }
     least = __reduce_min_sync(kFull, least);
-    if (least > limit || peek(&st->stop) != 0u) {  // every cell with key <= the goal label is final
+    if (least > limit || peek(&st->stop) != 0u) {  // every cell whose key still matters is final
       __syncwarp();
       if (lane == 0) {
         __threadfence();
@@ -579,14 +598,55 @@ __device__ __noinline__ void open_level(int tx, int ty, Space ws, TileNetState* 
   }
 }
 
+// Price of entering window cell (l, x, y): without the net's own use on a cell
+// of its previous route.
+__device__ __forceinline__ uint32_t price_of(const TileLaunch& p, const Win& win, int l, int x, int y, bool mine) {
+  const size_t i = (static_cast<size_t>(l) * p.lat.height + (win.y0 + y)) * p.lat.width + (win.x0 + x);
+  return __ldg((mine ? p.cell_cost_own : p.cell_cost) + i);
+}
+
+__device__ __forceinline__ uint32_t price_of(const TileLaunch& p, const Win& win, const Space& ws, int l, int x, int y) {
+  bool mine = false;
+  if (ws.own != nullptr) {
+    const int id = (l * win.ty + (y >> 5)) * win.tx + (x >> 5);
+    mine = ((__ldcg(ws.own + static_cast<size_t>(id) * 32u + (y & 31)) >> (x & 31)) & 1u) != 0u;
+  }
+  return price_of(p, win, l, x, y, mine);
+}
+
+// Prices of a unit's cells into shared memory (at most kPriceLimit each);
+// returns whether a free cell's reaches the limit.
+__device__ __forceinline__ bool load_prices(const TileLaunch& p, const Win& win, const Space& ws, const Unit& u,
+                                            uint32_t col_free, uint32_t* prices, int lane) {
+  uint32_t own = 0;  // lane = row
+  if (ws.own != nullptr) own = __ldcg(ws.own + static_cast<size_t>(u.id) * 32u + lane);
+  bool high = false;
+#pragma unroll 1
+  for (int c = 0; c < 32; c += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t word = __shfl_sync(kFull, own, c + i);
+      const bool in = u.bx + lane < win.w && u.by + c + i < win.h;
+      v[i] = in ? price_of(p, win, u.l, u.bx + lane, u.by + c + i, ((word >> lane) & 1u) != 0u) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      high = high || (v[i] >= kPriceLimit && ((col_free >> (c + i)) & 1u) != 0u);
+      prices[(c + i) * kPricePitch + lane] = min(v[i], kPriceLimit);
+    }
+  }
+  return high;
+}
+
 // Relaxes one pending unit to its fixed point and makes the neighbours it
 // lowers pending.  Ends by handing its place in `active` to the units it
 // queued.
-template <bool kCheapDiagonal>
+template <bool kCheapDiagonal, bool kPriced>
 __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, const Space& ws, uint32_t packed,
                                            const LanePart& part, uint32_t start_unit, int start_cell,
                                            uint32_t goal_unit, int goal_cell, TileNetState* st, uint32_t* tile,
-                                           int lane) {
+                                           uint32_t* prices, int lane) {
   const LatticeDeviceView& lat = p.lat;
   const Unit u = unpack_unit(win, packed);
   uint32_t key = 0, flags = 0, steps = 0;
@@ -635,9 +695,9 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
   };
   if (lane == 0) {
     key = atomicExch(ws.pend + u.id, kBusyKey);
-    // a key above the goal label can no longer matter; its side bits stay
-    // set, because a source sets its bit before it lowers the key
-    if (key <= peek(&st->goal) && peek(&st->stop) == 0u) {
+    // a key above the limit can no longer matter; its side bits stay set,
+    // because a source sets its bit before it lowers the key
+    if (key <= peek(&st->limit) && peek(&st->stop) == 0u) {
       flags = atomicAnd(ws.flags + u.id, ~kSourceBits);
       __threadfence();  // the sources' labels are read after their bits
     } else {
@@ -657,7 +717,10 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
   const uint32_t exist = neighbours(win, u, lat.layers);
   const uint32_t touched = touched_neighbours(ws, part, u.id, exist, lane);
   load_unit(ws.labels, win, u, touched, own, tile, lane);
+  bool high = false;  // a price or label near the 32-bit limit
+  if constexpr (kPriced) high = load_prices(p, win, ws, u, m.col_free, prices, lane);
   __syncwarp();
+  const auto price_at = [&](int r, int c) { return kPriced ? prices[r * kPricePitch + c] : 0u; };
 
   uint32_t down = 0, up = 0, right = 0, left = 0;  // lines whose source line changed
   uint32_t rows = 0, cols = 0;                     // changed rows and columns
@@ -690,7 +753,9 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const uint32_t v = cell[i * kPitch];
-        const uint32_t t = __viaddmin_u32(unless(closed, i, o[i]), via, v);
+        uint32_t t = unless(closed, i, o[i]) + via;
+        if constexpr (kPriced) t = min(t, kTileInf) + price_at(c + i, lane);
+        t = min(t, v);
         cell[i * kPitch] = t;
         diff |= t ^ v;
       }
@@ -706,24 +771,24 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
   // moves from the rim: the top and bottom rows (lane = column), then the
   // left and right columns (lane = row)
   if ((flags & 0x31u) != 0u) {
-    const unsigned hit = __ballot_sync(kFull, enter_side(tile + kPitch + 1 + lane, tile + 1 + lane, 1, m.rim,
-                                                         (m.col_free & 1u) != 0u, orth, diag));
+    const unsigned hit = __ballot_sync(kFull, enter_side<kPriced>(tile + kPitch + 1 + lane, tile + 1 + lane, 1, m.rim,
+                                                                  (m.col_free & 1u) != 0u, price_at(0, lane), orth, diag));
     if (hit != 0u) rows |= 1u, cols |= hit;
   }
   if ((flags & 0xC2u) != 0u) {
-    const unsigned hit = __ballot_sync(kFull, enter_side(tile + 32 * kPitch + 1 + lane, tile + 33 * kPitch + 1 + lane, 1,
-                                                         m.rim >> 2, (m.col_free >> 31) != 0u, orth, diag));
+    const unsigned hit = __ballot_sync(kFull, enter_side<kPriced>(tile + 32 * kPitch + 1 + lane, tile + 33 * kPitch + 1 + lane, 1,
+                                                                  m.rim >> 2, (m.col_free >> 31) != 0u, price_at(31, lane), orth, diag));
     if (hit != 0u) rows |= 0x80000000u, cols |= hit;
   }
   __syncwarp();
   if ((flags & 0x4u) != 0u) {
-    const unsigned hit = __ballot_sync(kFull, enter_side(tile + (lane + 1) * kPitch + 1, tile + (lane + 1) * kPitch,
-                                                         kPitch, m.rim >> 4, (m.row_free & 1u) != 0u, orth, diag));
+    const unsigned hit = __ballot_sync(kFull, enter_side<kPriced>(tile + (lane + 1) * kPitch + 1, tile + (lane + 1) * kPitch,
+                                                                  kPitch, m.rim >> 4, (m.row_free & 1u) != 0u, price_at(lane, 0), orth, diag));
     if (hit != 0u) cols |= 1u, rows |= hit;
   }
   if ((flags & 0x8u) != 0u) {
-    const unsigned hit = __ballot_sync(kFull, enter_side(tile + (lane + 1) * kPitch + 32, tile + (lane + 1) * kPitch + 33,
-                                                         kPitch, m.rim >> 6, (m.row_free >> 31) != 0u, orth, diag));
+    const unsigned hit = __ballot_sync(kFull, enter_side<kPriced>(tile + (lane + 1) * kPitch + 32, tile + (lane + 1) * kPitch + 33,
+                                                                  kPitch, m.rim >> 6, (m.row_free >> 31) != 0u, price_at(lane, 31), orth, diag));
     if (hit != 0u) cols |= 0x80000000u, rows |= hit;
   }
   down = rows << 1;
@@ -741,7 +806,7 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     }
     __syncwarp();
     if (down != 0u) {
-      const Swept w = sweep_lines<kPitch, kCheapDiagonal>(first_row, ~m.col_free, down, orth, diag, lane, steps);
+      const Swept w = sweep_lines<kPitch, kPricePitch, kCheapDiagonal, kPriced>(first_row, prices + lane, ~m.col_free, down, orth, diag, lane, steps);
       down = 0u;
       up |= w.back;
       right |= w.lanes << 1;
@@ -750,8 +815,8 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
       cols |= w.lanes;
     }
     if (up != 0u) {
-      const Swept w = sweep_lines<-kPitch, kCheapDiagonal>(first_row + 31 * kPitch, __brev(~m.col_free),
-                                                           __brev(up), orth, diag, lane, steps);
+      const Swept w = sweep_lines<-kPitch, -kPricePitch, kCheapDiagonal, kPriced>(
+          first_row + 31 * kPitch, prices + 31 * kPricePitch + lane, __brev(~m.col_free), __brev(up), orth, diag, lane, steps);
       up = 0u;
       down |= __brev(w.back);
       right |= w.lanes << 1;
@@ -761,7 +826,8 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     }
     __syncwarp();
     if (right != 0u) {
-      const Swept w = sweep_lines<1, kCheapDiagonal>(first_col, ~m.row_free, right, orth, diag, lane, steps);
+      const Swept w = sweep_lines<1, 1, kCheapDiagonal, kPriced>(first_col, prices + lane * kPricePitch, ~m.row_free, right,
+                                                                orth, diag, lane, steps);
       right = 0u;
       left |= w.back;
       down |= w.lanes << 1;
@@ -770,8 +836,8 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
       rows |= w.lanes;
     }
     if (left != 0u) {
-      const Swept w = sweep_lines<-1, kCheapDiagonal>(first_col + 31, __brev(~m.row_free), __brev(left), orth,
-                                                      diag, lane, steps);
+      const Swept w = sweep_lines<-1, -1, kCheapDiagonal, kPriced>(
+          first_col + 31, prices + lane * kPricePitch + 31, __brev(~m.row_free), __brev(left), orth, diag, lane, steps);
       left = 0u;
       right |= __brev(w.back);
       down |= w.lanes << 1;
@@ -792,10 +858,27 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     if (own && ((rows >> c) & 0xFFu) == 0u) continue;
     const uint32_t* row = tile + (c + 1) * kPitch + 1 + lane;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) mine[(c + k) * 32] = row[k * kPitch];
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t v = row[k * kPitch];
+      mine[(c + k) * 32] = v;
+      if constexpr (kPriced) high = high || (v >= kPriceLimit && v < kTileInf);
+    }
   }
   if (packed == goal_unit && lane == 0) {
-    atomicMin(&st->goal, tile[((goal_cell >> 5) + 1) * kPitch + 1 + (goal_cell & 31)]);
+    const uint32_t goal = tile[((goal_cell >> 5) + 1) * kPitch + 1 + (goal_cell & 31)];
+    if (goal < kTileInf) {
+      atomicMin(&st->goal, goal);
+      // Priced, the search goes on to the end of the key level that holds the
+      // goal, as the cell form does: a price that overflows there rejects
+      // the net.
+      uint32_t limit = goal;
+      if constexpr (kPriced) {
+        const unsigned long long width = peek(&st->level_width), first = peek(&st->start_key);
+        limit = static_cast<uint32_t>(min(first + width * ((goal - first) / width + 1ull) - 1ull,
+                                          static_cast<unsigned long long>(kNoLimit)));
+      }
+      atomicMin(&st->limit, limit);
+    }
   }
   // the least key this unit lowers in each neighbour
   uint32_t out_key = kNoKey;
@@ -803,6 +886,18 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     if (!__any_sync(kFull, lowers)) return kNoKey;
     const uint32_t f = lowers ? cost + bound_to_goal(lat, win, l, x, y) : kNoKey;
     return __reduce_min_sync(kFull, f);
+  };
+  // a move's cost into a cell of a neighbour, with its price
+  const auto priced = [&](uint32_t t, int l, int x, int y) {
+    if constexpr (kPriced) {
+      if (t < kTileInf) {
+        const uint32_t price = price_of(p, win, ws, l, x, y);
+        high = high || price >= kPriceLimit;
+        t = min(t + min(price, kPriceLimit), kTileInf);
+      }
+      __syncwarp();
+    }
+    return t;
   };
   // rows above and below the unit, and its corners
 #pragma unroll 1
@@ -815,10 +910,12 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     if (lane > 0) t = __viaddmin_u32(unless(closed, 0, line[-1]), diag, t);
     if (lane < 31) t = __viaddmin_u32(unless(closed, 1, line[1]), diag, t);
     const int y = k == 0 ? u.by - 1 : u.by + 32;
+    t = priced(t, u.l, u.bx + lane, y);
     const uint32_t f = key_min(t < rim[0], t, u.l, u.bx + lane, y);
     if (lane == k) out_key = f;
     // corners: from the first and the last cell of the line
-    const uint32_t corner = unless(closed, lane == 0 ? 0 : 1, line[0]) + diag;
+    uint32_t corner = lane == 0 || lane == 31 ? unless(closed, lane == 0 ? 0 : 1, line[0]) + diag : kTileInf;
+    corner = priced(corner, u.l, u.bx + (lane == 0 ? -1 : 32), y);
     const bool low = (lane == 0 && corner < rim[-1]) || (lane == 31 && corner < rim[1]);
     if (__any_sync(kFull, low)) {
       const uint32_t cf = low ? corner + bound_to_goal(lat, win, u.l, u.bx + (lane == 0 ? -1 : 32), y) : kNoKey;
@@ -837,6 +934,7 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     uint32_t t = unless(~(m.rim >> (10 + k)), 0, line[0]) + orth;
     if (lane > 0) t = __viaddmin_u32(unless(closed, 0, line[-kPitch]), diag, t);
     if (lane < 31) t = __viaddmin_u32(unless(closed, 1, line[kPitch]), diag, t);
+    t = priced(t, u.l, u.bx + (k == 0 ? -1 : 32), u.by + lane);
     const uint32_t f = key_min(t < rim[0], t, u.l, u.bx + (k == 0 ? -1 : 32), u.by + lane);
     if (lane == 2 + k) out_key = f;
   }
@@ -863,7 +961,9 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
       bool lowers = false;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const uint32_t t = unless(closed, i, row[i * kPitch]) + via;
+        uint32_t t = unless(closed, i, row[i * kPitch]) + via;
+        // (an unchanged row of the block lowers nothing: no need of its prices)
+        t = !kPriced || (rows & (1u << (c + i))) != 0u ? priced(t, l, u.bx + lane, u.by + c + i) : kTileInf;
         lowers = lowers || t < o[i];
         o[i] = t < o[i] ? t : kNoKey;
       }
@@ -881,10 +981,13 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     f = __reduce_min_sync(kFull, f);
     if (lane == k && f != kNoKey) out_key = f + static_cast<uint32_t>(abs(l - win.gl)) * via;
   }
+  if constexpr (kPriced) {
+    if (__any_sync(kFull, high) && lane == 0) atomicMax(&st->stop, 3u);
+  }
   __threadfence();  // labels before the flags and keys that announce them
   __syncwarp();
   if (!own && lane == 0) atomicOr(ws.flags + u.id, kTouched);
-  const uint32_t limit = peek(&st->goal), thr = peek(&st->thr);
+  const uint32_t limit = peek(&st->limit), thr = peek(&st->thr);
   bool near = false, far = false;
   if (out_key <= limit) {  // lanes 0..9 only: the others hold kNoKey
     const int nb = u.id + part.offset;
@@ -907,10 +1010,11 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
 // memory, so a step costs a few shared-memory reads; a step onto another unit
 // loads that one.  Vias are tried only when no planar predecessor matches
 // (headings 0-7 come first).  Returns the path length, 0 when broken.
+template <bool kPriced>
 __device__ __forceinline__ uint32_t walk_path(const TileLaunch& p, const Win& win, const Space& ws,
                                               const LanePart& part, int sl, int sx, int sy, uint32_t goal, unsigned long long base,
                                               unsigned long long bound, uint32_t* tile, uint64_t* quads,
-                                              int lane) {
+                                              uint32_t* prices, int lane) {
   const LatticeDeviceView& lat = p.lat;
   int l = win.gl, x = win.gx, y = win.gy;
   uint32_t here = goal, len = 0;
@@ -941,17 +1045,20 @@ __device__ __forceinline__ uint32_t walk_path(const TileLaunch& p, const Win& wi
       quads[lane] = quads34(line, above);
       if (lane == 31) quads[32] = quads34(line, rims.bottom);
       load_unit(ws.labels, win, u, touched_neighbours(ws, part, u.id, neighbours(win, u, lat.layers), lane), true, tile, lane);
+      if constexpr (kPriced) load_prices(p, win, ws, u, m.col_free, prices, lane);
       __syncwarp();
       loaded = unit;
     }
     const int r = y - u.by, c = x - u.bx;
+    // the move into this cell paid its price
+    const uint32_t paid = kPriced ? prices[r * kPricePitch + c] : 0u;
     bool ok = false;
     uint32_t label = kTileInf;
     if (lane < 8) {
       const int pr = r - dy, pc = c - dx;
       label = tile[(pr + 1) * kPitch + 1 + pc];
       const bool legal = (lane & 1) == 0 || ((quads[max(r, pr)] >> max(c, pc)) & 1ull) != 0ull;
-      ok = legal && label < kTileInf && label + ((lane & 1) ? lat.diag : lat.orth) == here;
+      ok = legal && label < kTileInf && label + ((lane & 1) ? lat.diag : lat.orth) + paid == here;
     }
     unsigned hit = __ballot_sync(kFull, ok);
     int nl = l;
@@ -968,7 +1075,7 @@ __device__ __forceinline__ uint32_t walk_path(const TileLaunch& p, const Win& wi
           }
           if (allowed) {
             label = __ldcg(ws.labels + static_cast<size_t>(other) * 1024u + r * 32 + c);
-            ok = label < kTileInf && label + lat.via == here;
+            ok = label < kTileInf && label + lat.via + paid == here;
           }
         }
       }
@@ -1022,6 +1129,7 @@ __device__ __forceinline__ TileNet net_at(const TileLaunch& p, uint32_t index, u
   n.sy = static_cast<int>(net.start_y) - n.win.y0;
   n.units = static_cast<uint32_t>(p.lat.layers) * n.win.tx * n.win.ty;
   n.ws = space_at(base, n.units);
+  if (p.cell_cost_own != nullptr) n.ws.own = p.own_bits + (base - p.c[0].pool) / 32;
   n.start_unit = pack_unit(n.sl, n.sy >> 5, n.sx >> 5);
   n.goal_unit = pack_unit(n.win.gl, n.win.gy >> 5, n.win.gx >> 5);
   n.start_cell = ((n.sy & 31) << 5) | (n.sx & 31);
@@ -1097,11 +1205,30 @@ __device__ __forceinline__ uint32_t find_net(const TileLaunch& p, uint32_t& low,
 
 // Clears the net's workspace and queues its start.
 __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n, TileNetState* st, uint32_t level_width,
-                                          uint32_t slot, int lane) {
+                                          uint32_t slot, uint32_t net, int lane) {
   const bool free_ends = free_at(p.lat, n.win, n.sl, n.sx, n.sy) &&
                          free_at(p.lat, n.win, n.win.gl, n.win.gx, n.win.gy);
   for (uint32_t i = lane; i < 2u * n.units; i += 32) __stcg(n.ws.pend + i, i < n.units ? kNoKey : 0u);
   for (uint32_t i = lane; i <= n.ws.ring_mask; i += 32) __stcg(n.ws.ring + i, kEmptySlot);
+  if (n.ws.own != nullptr) {
+    // the cells of the net's previous route (a packed reverse path of global
+    // cells; a cell outside the window cannot be entered anyway)
+    for (uint32_t i = lane; i < 32u * n.units; i += 32) __stcg(n.ws.own + i, 0u);
+    __syncwarp();
+    const apgar_b200_lattice_result prev = p.prev_results[net];
+    if (prev.completion == APGAR_B200_COMPLETION_REACHED) {
+      const uint32_t lw = static_cast<uint32_t>(p.lat.width), lh = static_cast<uint32_t>(p.lat.height);
+      for (uint32_t j = lane; j < prev.path_len; j += 32) {
+        const uint32_t c = p.prev_paths[prev.path_offset + j];
+        const int x = static_cast<int>(c % lw) - n.win.x0, y = static_cast<int>((c / lw) % lh) - n.win.y0;
+        const uint32_t l = c / lw / lh;
+        if (l < static_cast<uint32_t>(p.lat.layers) && x >= 0 && x < n.win.w && y >= 0 && y < n.win.h) {
+          const int id = (static_cast<int>(l) * n.win.ty + (y >> 5)) * n.win.tx + (x >> 5);
+          atomicOr(n.ws.own + static_cast<size_t>(id) * 32u + (y & 31), 1u << (x & 31));
+        }
+      }
+    }
+  }
   __syncwarp();
   if (lane == 0) {
     const uint32_t h0 = bound_to_goal(p.lat, n.win, n.sl, n.sx, n.sy);
@@ -1111,6 +1238,8 @@ __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n,
     st->thr = h0 + min(level_width, kNoKey - h0);
     st->far_par = st->far_count[0] = st->far_count[1] = 0u;
     st->goal = kTileInf;
+    st->limit = kNoLimit;
+    st->start_key = h0;
     st->stop = p.cancel != nullptr && *p.cancel != 0u ? 1u : 0u;
     st->steps = st->units = st->levels = 0u;
     st->slot = slot;
@@ -1126,11 +1255,20 @@ __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n,
 }
 
 // The net's result, and its path by the canonical walk.
+template <bool kPriced>
 __device__ __forceinline__ void finish_net(const TileLaunch& p, const TileNet& n, const TileNetState* st, bool free_ends,
-                                           uint32_t net, uint32_t* tile, uint64_t* quads, int lane) {
+                                           uint32_t net, uint32_t* tile, uint64_t* quads, uint32_t* prices, int lane) {
   const LatticeDeviceView& lat = p.lat;
   __threadfence();
   const uint32_t goal = peek(&st->goal), stop = peek(&st->stop);
+  if (kPriced && stop == 3u) {  // for the cell form
+    if (lane == 0) {
+      NetPlan plan{};
+      plan.net = net;
+      p.redo[atomicAdd(p.redo_count, 1u)] = plan;
+    }
+    return;
+  }
   apgar_b200_lattice_result res{};
   res.cost = APGAR_B200_UNREACHABLE;
   res.completion = APGAR_B200_COMPLETION_DISCONNECTED;
@@ -1148,7 +1286,8 @@ __device__ __forceinline__ void finish_net(const TileLaunch& p, const TileNet& n
     base = __shfl_sync(kFull, base, 0);
     uint32_t len = 0;
     if (base + bound <= p.path_arena_capacity) {
-      len = walk_path(p, n.win, n.ws, lane_part(n.win, lane), n.sl, n.sx, n.sy, goal, base, bound, tile, quads, lane);
+      len = walk_path<kPriced>(p, n.win, n.ws, lane_part(n.win, lane), n.sl, n.sx, n.sy, goal, base, bound, tile, quads,
+                               prices, lane);
     }
     res.completion = len != 0u ? APGAR_B200_COMPLETION_REACHED : APGAR_B200_COMPLETION_REJECTED;
     if (len != 0u) {
@@ -1160,18 +1299,40 @@ __device__ __forceinline__ void finish_net(const TileLaunch& p, const TileNet& n
   if (lane == 0) p.results[net] = res;
 }
 
+// A kept route (partial rip-up): the net's previous result and path go into
+// this execution.
+__device__ __forceinline__ void keep_net(const TileLaunch& p, uint32_t net, int lane) {
+  apgar_b200_lattice_result res = p.prev_results[net];
+  res.arena_offset = 0;
+  if (res.completion == APGAR_B200_COMPLETION_REACHED && res.path_len > 0) {
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(p.arena_cursor, static_cast<unsigned long long>(res.path_len));
+    base = __shfl_sync(kFull, base, 0);
+    if (base + res.path_len > p.path_arena_capacity) {
+      res.completion = APGAR_B200_COMPLETION_REJECTED;
+      res.cost = APGAR_B200_UNREACHABLE;
+      res.path_len = 0;
+    } else {
+      for (uint32_t j = lane; j < res.path_len; j += 32) p.path_arena[base + j] = p.prev_paths[res.path_offset + j];
+      res.arena_offset = base;
+    }
+  }
+  if (lane == 0) p.results[net] = res;
+}
+
 // Every warp takes nets, largest first, and relaxes their units.  A warp that
 // finds no net left is a guest of other warps' nets: it relaxes their units
 // until they have none to spare.  A guest may leave at any time: a net's
 // owner finishes it alone.
-template <bool kCheapDiagonal>
+template <bool kCheapDiagonal, bool kPriced>
 __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kernel(const __grid_constant__ TileLaunch p) {
   extern __shared__ __align__(16) uint32_t tile_smem[];
   __shared__ Lookout look;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = blockIdx.x * (kTileThreads / 32) + (threadIdx.x >> 5);
-  uint32_t* const tile = tile_smem + (threadIdx.x >> 5) * kWarpWords;
+  uint32_t* const tile = tile_smem + (threadIdx.x >> 5) * (kWarpWords + (kPriced ? kPriceWords : 0));
   uint64_t* const quads = reinterpret_cast<uint64_t*>(tile + kTileWords);
+  uint32_t* const prices = tile + kWarpWords;
   if (threadIdx.x == 0) {
     look.probed = static_cast<uint32_t>(clock64());
     look.net = kNoKey;
@@ -1181,7 +1342,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
   __syncthreads();
   int k = 0;
   uint32_t index = 0, low = 0, skip = 0;
-  bool busy = false, owner = false, member = false, free_ends = false;
+  bool busy = false, owner = false, member = false, free_ends = false, kept = false;
   TileNetState* st = nullptr;
   TileNet n;
   LanePart part{};
@@ -1227,7 +1388,14 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
       const uint32_t place = k < 5 && p.c[k].team != 0u ? blockIdx.x : warp;
       n = net_at(p, index, k < 5 ? place : peek(&st->slot));
       part = lane_part(n.win, lane);
-      if (owner) free_ends = start_net(p, n, st, p.c[k].level_width, place, lane);
+      kept = p.skip != nullptr && k < 5 && p.skip[p.plans[index].net] != 0u;
+      if (owner && kept) {
+        keep_net(p, p.plans[index].net, lane);
+        if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&st->phase) = 2u;
+        __syncwarp();
+      } else if (owner) {
+        free_ends = start_net(p, n, st, p.c[k].level_width, place, p.plans[index].net, lane);
+      }
       if (k < 5 && p.c[k].team != 0u) __syncthreads();  // the team waits for the net's set-up
       if (k == 5) {
         if (lane == 0) atomicAdd(&st->guests, 1u);
@@ -1243,8 +1411,8 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
     }
     const uint32_t unit = pop_unit(st, n.ws, lane);
     if (unit != kEmptySlot) {
-      relax_unit<kCheapDiagonal>(p, n.win, n.ws, unit, part, n.start_unit, n.start_cell, n.goal_unit, n.goal_cell, st,
-                                 tile, lane);
+      relax_unit<kCheapDiagonal, kPriced>(p, n.win, n.ws, unit, part, n.start_unit, n.start_cell, n.goal_unit,
+                                          n.goal_cell, st, tile, prices, lane);
       __syncwarp();
       idle = misses = 0;
       continue;
@@ -1265,7 +1433,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
     } else if (done || idle > kIdleLimit) {
       if (!done && lane == 0) atomicMax(&st->stop, 2u);
       __syncwarp();
-      finish_net(p, n, st, free_ends, p.plans[index].net, tile, quads, lane);
+      if (!kept) finish_net<kPriced>(p, n, st, free_ends, p.plans[index].net, tile, quads, prices, lane);
       __syncwarp();
       if (lane == 0) atomicAdd(p.finished, 1u);
       busy = false;
@@ -1279,8 +1447,18 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
   }
 }
 
-constexpr int kTileSmem = kTileThreads / 32 * kWarpWords * 4;
+constexpr int tile_smem_bytes(bool priced) {
+  return kTileThreads / 32 * (kWarpWords + (priced ? kPriceWords : 0)) * 4;
+}
 
+using TileKernel = void (*)(TileLaunch);
+
+TileKernel tile_kernel(bool cheap_diagonal, bool priced) {
+  if (cheap_diagonal) return priced ? lattice_tiles_kernel<true, true> : lattice_tiles_kernel<true, false>;
+  return priced ? lattice_tiles_kernel<false, true> : lattice_tiles_kernel<false, false>;
+}
+
+// CTAs per SM that every form of the kernel can keep resident.
 std::atomic<int> g_tile_blocks[64];
 
 cudaError_t tile_blocks_per_sm(int* out) {
@@ -1294,16 +1472,19 @@ cudaError_t tile_blocks_per_sm(int* out) {
       return cudaSuccess;
     }
   }
-  cudaError_t e = cudaFuncSetAttribute(lattice_tiles_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem);
-  if (e == cudaSuccess) {
-    e = cudaFuncSetAttribute(lattice_tiles_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem);
+  int least = kTileBlocks;
+  for (int form = 0; form < 4; ++form) {
+    const bool priced = (form & 2) != 0;
+    const void* kernel = reinterpret_cast<const void*>(tile_kernel((form & 1) != 0, priced));
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_bytes(priced));
+    int blocks = 0;
+    if (e == cudaSuccess) {
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kTileThreads, tile_smem_bytes(priced));
+    }
+    if (e != cudaSuccess) return e;
+    least = std::min(least, blocks);
   }
-  int blocks = 0;
-  if (e == cudaSuccess) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, lattice_tiles_kernel<false>, kTileThreads, kTileSmem);
-  }
-  if (e != cudaSuccess) return e;
-  *out = std::max(1, blocks);
+  *out = std::max(1, least);
   if (cacheable) g_tile_blocks[device].store(*out, std::memory_order_release);
   return cudaSuccess;
 }
@@ -1329,11 +1510,8 @@ cudaError_t launch_lattice_tiles(const TileLaunch& launch, int sm_count, cudaStr
   uint32_t warps = 0;
   if (cudaError_t e = lattice_tile_warps(sm_count, &warps); e != cudaSuccess) return e;
   const unsigned grid = warps / (kTileThreads / 32);
-  if (launch.lat.diag < launch.lat.orth) {
-    lattice_tiles_kernel<true><<<grid, kTileThreads, kTileSmem, stream>>>(launch);
-  } else {
-    lattice_tiles_kernel<false><<<grid, kTileThreads, kTileSmem, stream>>>(launch);
-  }
+  const bool priced = launch.cell_cost != nullptr;
+  tile_kernel(launch.lat.diag < launch.lat.orth, priced)<<<grid, kTileThreads, tile_smem_bytes(priced), stream>>>(launch);
   return cudaGetLastError();
 }
 

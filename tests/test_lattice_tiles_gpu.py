@@ -94,3 +94,42 @@ def test_few_slots_and_many_guests(monkeypatch):
     monkeypatch.setenv("APGAR_B200_FRONTIER_PER_NET_BYTES", "1")
     monkeypatch.setenv("APGAR_B200_FRONTIER_SLOT_BYTES", str(24 << 20))
     _check(lat, nets)
+
+
+CELL_FORM = (1 << 30) - 1  # a bound on the rounds: the search over single cells
+
+
+@pytest.mark.parametrize("high", [0, (1 << 29) - 1, 1 << 29, (1 << 31) - 1])
+@pytest.mark.parametrize("layers,width,height", [(1, 96, 65), (3, 160, 130)])
+def test_priced_results_equal_the_cell_forms(layers, width, height, high):
+    # sparse congestion prices, and a few cells priced around the limit at
+    # which the tile form hands a net over to the cell form
+    import torch
+
+    base = synth.make_lattice(300 + layers, layers, 160, 0.2, via_mask=layers > 1)
+    lat = synth.Lattice(layers, height, width, np.ascontiguousarray(base.blocked[:, :height, :width // 32]),
+                        None if layers == 1 else np.ascontiguousarray(base.via_ok[:, :height, :width // 32]))
+    nets = synth.make_nets(lat, 301, 48, hpwl_median=50.0, hpwl_sigma=0.6, margin=12)
+    rng = np.random.default_rng(302)
+    cells = layers * height * width
+    price = np.where(rng.random(cells) < 0.2, rng.integers(1, 900, cells), 0).astype(np.uint32)
+    if high:
+        price[rng.integers(0, cells, size=8)] = high
+    prices = torch.from_numpy(price.view(np.int32)).cuda()
+    dev = apgar_b200.DeviceLattice(lat)
+    try:
+        out = []
+        for rounds in (1 << 30, CELL_FORM):
+            plan = dev.plan(nets, generator="frontier", max_rounds=rounds)
+            for costs in (prices, None, prices):  # prices come, go and come back
+                plan.set_cell_costs(costs)
+                plan.execute()
+                res, paths = plan.readback()
+                out.append((res, paths.copy()))
+            plan.close()
+    finally:
+        dev.close()
+    for (a, pa), (b, pb) in zip(out[:3], out[3:]):
+        for field in ("cost", "completion", "path_len", "path_offset"):
+            assert np.array_equal(a[field], b[field]), field
+        assert np.array_equal(pa, pb)
