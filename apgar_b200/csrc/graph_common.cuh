@@ -46,6 +46,7 @@ struct GraphLaunch {
   uint32_t max_policy_edges;  // the largest policy_count of the batch
   uint32_t policy_smem_offset;  // where a query's edges are staged in shared memory, or ~0u
   uint32_t nbr_smem_offset;     // where the neighbour table is staged in shared memory, or ~0u
+  uint64_t max_transition;      // the largest finite move of the batch (bend, surcharges and policy included)
 };
 
 struct PathCheckLaunch {

@@ -299,9 +299,11 @@ bool full_workspace_generator(uint8_t generator) {
 
 int validate_batch(const ViewObject& v, const apgar_b200_batch_request& req,
                    const apgar_b200_batch_query_v1* queries, uint32_t count,
-                   const apgar_b200_policy_edge_v1* edges, uint64_t edge_count) {
+                   const apgar_b200_policy_edge_v1* edges, uint64_t edge_count,
+                   uint64_t* max_transition) {
   const uint64_t n = v.legal.size();
   const uint64_t S = 9ull * n;
+  *max_transition = 0;
   if (req.schema_version != 1u || req.batch_id == 0 || count == 0 ||
       edge_count > kMaximumPolicyEntries || req.maximum_rounds == 0 ||
       req.generator > APGAR_B200_GENERATOR_B200_PERSISTENT_WORKSPACE) {
@@ -350,6 +352,7 @@ int validate_batch(const ViewObject& v, const apgar_b200_batch_request& req,
     if (orth >= inf || diag >= inf || bend >= inf || max_t * n * 8u >= inf) {
       return invariant("candidate batch policy cost bound collides with the unreachable sentinel");
     }
+    *max_transition = std::max(*max_transition, static_cast<uint64_t>(max_t));  // below the sentinel
     expected_policy = pend;
   }
   if (expected_policy != edge_count) return invariant("candidate batch contains unowned policy-edge storage");
@@ -359,7 +362,7 @@ int validate_batch(const ViewObject& v, const apgar_b200_batch_request& req,
 int run_batch(ViewObject* v, const apgar_b200_batch_request& req,
               const apgar_b200_batch_query_v1* queries, uint32_t count,
               const apgar_b200_policy_edge_v1* edges, uint64_t edge_count,
-              const volatile uint8_t* cancel, PendingBatch* pending) {
+              uint64_t max_transition, const volatile uint8_t* cancel, PendingBatch* pending) {
   const uint64_t n = v->legal.size();
   const uint64_t S = 9ull * n;
   const bool workspace_mode = full_workspace_generator(req.generator);
@@ -431,6 +434,7 @@ int run_batch(ViewObject* v, const apgar_b200_batch_request& req,
   L.generator = req.generator;
   L.workspace_mode = workspace_mode ? 1 : 0;
   L.cancel = v->cancel_dev;
+  L.max_transition = max_transition;
   for (uint64_t i = 0; i < Q; ++i) L.max_policy_edges = std::max(L.max_policy_edges, queries[i].policy_count);
 
   cudaEvent_t t0 = nullptr, t1 = nullptr;
@@ -564,11 +568,12 @@ extern "C" int apgar_b200_execute_batch(void* view, const apgar_b200_batch_reque
     v->lease.acquire();
     pending->view = v;
     pending->leased = true;
-    if (int rc = validate_batch(*v, *request, queries, query_count, policy_edges, policy_edge_count);
+    uint64_t max_transition = 0;
+    if (int rc = validate_batch(*v, *request, queries, query_count, policy_edges, policy_edge_count, &max_transition);
         rc != APGAR_B200_OK) {
       return rc;
     }
-    if (int rc = run_batch(v, *request, queries, query_count, policy_edges, policy_edge_count, cancel,
+    if (int rc = run_batch(v, *request, queries, query_count, policy_edges, policy_edge_count, max_transition, cancel,
                            pending.get());
         rc != APGAR_B200_OK) {
       return rc;
@@ -701,7 +706,9 @@ extern "C" int apgar_b200_execute_route(void* view, uint8_t generator, uint32_t 
     q.frontier_state_capacity = 9ull * n;
     q.maximum_rounds = maximum_rounds;
     q.generator = APGAR_B200_GENERATOR_BUCKETED_FRONTIER;
-    if (int rc = run_batch(v, req, &q, 1, nullptr, 0, cancel, route->batch.get()); rc != APGAR_B200_OK) {
+    const uint64_t max_transition =
+        static_cast<uint64_t>(std::max(v->header.orthogonal_step, v->header.diagonal_step)) + v->header.bend;
+    if (int rc = run_batch(v, req, &q, 1, nullptr, 0, max_transition, cancel, route->batch.get()); rc != APGAR_B200_OK) {
       return rc;
     }
     apgar_b200_route_result_header_v1& h = route->header;

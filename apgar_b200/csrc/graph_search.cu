@@ -123,6 +123,35 @@ __device__ __forceinline__ void set_completion(apgar_b200_batch_result_v1& r, ui
   r.completion = static_cast<uint8_t>(c);
 }
 
+// The query's result record (one thread).
+__device__ __forceinline__ void write_result(const GraphLaunch& p, uint32_t qi, const apgar_b200_batch_query_v1& q,
+                                             uint32_t completion, uint32_t goal_state, uint32_t rounds,
+                                             unsigned long long examined, unsigned long long turns) {
+  const GraphDeviceView& g = p.g;
+  apgar_b200_batch_result_v1 r{};
+  r.schema_version = 1;
+  r.compiler_version = g.compiler_version;
+  r.input_ordinal = q.input_ordinal;
+  r.start_node = q.start_node;
+  r.goal_node = q.goal_node;
+  r.goal_state = completion == APGAR_B200_COMPLETION_REACHED ? goal_state : kInvalid32;
+  r.rounds = rounds;
+  r.generator = p.generator;
+  set_completion(r, completion);
+  r.batch_id = q.batch_id;
+  r.query_id = q.query_id;
+  r.workspace_owner = q.workspace_owner;
+  r.policy_identity = q.policy_identity;
+  r.routing_profile_fingerprint = q.routing_profile_fingerprint;
+  r.source_board_content_hash = g.source_board_content_hash;
+  r.compiler_profile_fingerprint = g.compiler_profile_fingerprint;
+  r.rule_bucket_identity = g.rule_bucket_identity;
+  r.device_view_fingerprint = g.device_view_fingerprint;
+  r.examined_work = examined;
+  r.heading_turn_relaxations = turns;
+  p.results[qi] = r;
+}
+
 // kShared: the query's labels, queues and stamps, and the neighbour table,
 // live in shared memory (a graph small enough for them to fit: the drop-in
 // corpus has 10-697 nodes), so each round's label reads, atomics and
@@ -409,30 +438,313 @@ __global__ void __launch_bounds__(kThreads) graph_search_kernel(GraphLaunch p) {
     if (lane == 0) p.compact[qi] = cp;
   }
 
-  if (tid == 0) {
-    apgar_b200_batch_result_v1 r{};
-    r.schema_version = 1;
-    r.compiler_version = g.compiler_version;
-    r.input_ordinal = q.input_ordinal;
-    r.start_node = q.start_node;
-    r.goal_node = q.goal_node;
-    r.goal_state = completion == APGAR_B200_COMPLETION_REACHED ? goal_state : kInvalid32;
-    r.rounds = rounds;
-    r.generator = p.generator;
-    set_completion(r, completion);
-    r.batch_id = q.batch_id;
-    r.query_id = q.query_id;
-    r.workspace_owner = q.workspace_owner;
-    r.policy_identity = q.policy_identity;
-    r.routing_profile_fingerprint = q.routing_profile_fingerprint;
-    r.source_board_content_hash = g.source_board_content_hash;
-    r.compiler_profile_fingerprint = g.compiler_profile_fingerprint;
-    r.rule_bucket_identity = g.rule_bucket_identity;
-    r.device_view_fingerprint = g.device_view_fingerprint;
-    r.examined_work = sh_examined;
-    r.heading_turn_relaxations = sh_turns;
-    p.results[qi] = r;
+  if (tid == 0) write_result(p, qi, q, completion, goal_state, rounds, sh_examined, sh_turns);
+}
+
+// The same search for graphs whose state fits one SM: 32-bit labels, 16-bit
+// neighbours and queues in shared memory (65.5 B per node: about 3,400 nodes).
+//
+// Every label is the cost of a walk without a repeated state, so at most
+// states * (the batch's largest finite move); the host takes this form only
+// when that stays below 2^31, so no 32-bit sum wraps and no 64-bit check could
+// have failed.  Shared 32-bit atomicMin is one instruction where the 64-bit
+// one is a compare-and-swap loop.
+//
+// A round has two barriers instead of five.  Each node keeps the least label
+// lowered since it was last expanded (pend); the next round's least label is
+// the minimum over the lowerings and the carried nodes of this round, and the
+// goal's best label is tracked where it is lowered, so neither takes a pass of
+// its own.  The bucket starts at the least pending label: counting labels that
+// were already expanded (as the form above does) restarts it at old labels
+// and took 2 to 5 times the rounds.  With a budget below kFewRounds the old
+// count is kept, so that a bounded search ends where it did.
+// Measured on one B200: 64 queries on 676 nodes 0.53 -> 0.16 ms, 16 full
+// workspaces of 2,304 nodes 2.3 -> 0.22 ms.
+constexpr uint32_t kFewRounds = 65536;
+enum : uint32_t { kNoLabel = 0xFFFFFFFFu };
+
+// Shared-memory layout of the small form, in bytes from the dynamic base.
+struct SmallLayout {
+  uint32_t pend, stamp, neighbours, queues, policied, legal, policy, total;
+};
+
+__host__ __device__ inline SmallLayout small_layout(uint32_t nodes, uint32_t policy_edges) {
+  SmallLayout o{};
+  uint32_t at = nodes * 36u;  // labels [nodes][9]
+  o.pend = at;
+  at += nodes * 4u;
+  o.stamp = at;
+  at += nodes * 4u;
+  o.neighbours = at;  // [8][nodes]
+  at += nodes * 16u;
+  o.queues = at;  // [2][nodes]
+  at += (nodes * 4u + 3u) & ~3u;
+  o.policied = at;  // a bit per canonical edge (node * 4 + direction) with a policy
+  at += (nodes * 4u + 31u) / 32u * 4u;
+  o.legal = at;
+  at += (nodes + 15u) & ~15u;
+  at = (at + 15u) & ~15u;
+  o.policy = at;
+  at += policy_edges * static_cast<uint32_t>(sizeof(apgar_b200_policy_edge_v1));
+  o.total = at;
+  return o;
+}
+
+template <int kBlock>
+__global__ void __launch_bounds__(kBlock) graph_search_small_kernel(GraphLaunch p) {
+  const uint32_t qi = blockIdx.x;
+  if (qi >= p.query_count) return;
+  const apgar_b200_batch_query_v1 q = p.queries[qi];
+  const uint32_t N = p.g.node_count, S = 9u * N;
+  extern __shared__ __align__(16) uint8_t graph_smem[];
+  const SmallLayout at = small_layout(N, p.max_policy_edges);
+  auto* const lab = reinterpret_cast<uint32_t*>(graph_smem);
+  auto* const pend = reinterpret_cast<uint32_t*>(graph_smem + at.pend);
+  auto* const stamp = reinterpret_cast<uint32_t*>(graph_smem + at.stamp);
+  auto* const next_of = reinterpret_cast<uint16_t*>(graph_smem + at.neighbours);
+  auto* const queues = reinterpret_cast<uint16_t*>(graph_smem + at.queues);
+  auto* const policied = reinterpret_cast<uint32_t*>(graph_smem + at.policied);
+  auto* const legal = graph_smem + at.legal;
+  auto* const pol = reinterpret_cast<apgar_b200_policy_edge_v1*>(graph_smem + at.policy);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ uint32_t sh_count[2], sh_least[2], sh_goal, sh_stop, sh_goal_state;
+  __shared__ unsigned long long sh_examined, sh_turns;
+
+  for (uint32_t s = tid; s < S; s += kBlock) lab[s] = kNoLabel;
+  for (uint32_t n = tid; n < N; n += kBlock) {
+    pend[n] = kNoLabel;
+    stamp[n] = 0u;
+    legal[n] = __ldg(p.g.legal + n);
   }
+  for (uint32_t i = tid; i < 8u * N; i += kBlock) {
+    next_of[i] = static_cast<uint16_t>(min(__ldg(p.g.neighbors + i), 0xFFFFu));
+  }
+  for (uint32_t i = tid; i < (N * 4u + 31u) / 32u; i += kBlock) policied[i] = 0u;
+  for (uint32_t i = tid; i < q.policy_count; i += kBlock) pol[i] = p.policy[q.policy_offset + i];
+  __syncthreads();
+  for (uint32_t i = tid; i < q.policy_count; i += kBlock) {
+    const uint32_t bit = pol[i].physical_edge_index / 8u * 4u + pol[i].physical_edge_index % 8u;
+    atomicOr(policied + (bit >> 5), 1u << (bit & 31u));
+  }
+  if (tid == 0) {
+    lab[q.start_node * 9u + 8u] = 0u;
+    pend[q.start_node] = 0u;
+    stamp[q.start_node] = 1u;
+    queues[0] = static_cast<uint16_t>(q.start_node);
+    sh_count[0] = 1u;
+    sh_count[1] = 0u;
+    sh_least[0] = 0u;
+    sh_least[1] = kNoLabel;
+    sh_goal = kNoLabel;
+    sh_stop = p.cancel != nullptr && *p.cancel != 0u ? 1u : 0u;
+    sh_examined = 0;
+    sh_turns = 0;
+  }
+  __syncthreads();
+
+  const uint32_t cost_orth = p.g.orth + static_cast<uint32_t>(q.orthogonal_step_surcharge);
+  const uint32_t cost_diag = p.g.diag + static_cast<uint32_t>(q.diagonal_step_surcharge);
+  const uint32_t cost_bend = p.g.bend + static_cast<uint32_t>(q.bend_surcharge);
+  const uint32_t delta = min(cost_orth, cost_diag);
+  const bool keep_pend = p.maximum_rounds < kFewRounds;
+  // cost of the move source -> target in direction d without a bend, or
+  // kNoLabel when its edge is banned
+  const auto move_cost = [&](uint32_t source, uint32_t target, uint32_t d) -> uint32_t {
+    const uint32_t canon = d < 4u ? source : target, dir = d & 3u, bit = canon * 4u + dir;
+    uint32_t c = (d & 1u) ? cost_diag : cost_orth;
+    if ((policied[bit >> 5] >> (bit & 31u)) & 1u) {
+      const uint64_t adj = policy_adjustment(pol, q.policy_count, canon * 8u + dir);
+      c = adj == kGraphInf ? kNoLabel : c + static_cast<uint32_t>(adj);
+    }
+    return c;
+  };
+
+  uint32_t completion = APGAR_B200_COMPLETION_BUDGET_EXHAUSTED;
+  uint32_t rounds = 0, examined = 0, turns = 0;
+  for (;;) {
+    const uint32_t cur = rounds & 1u;
+    const uint16_t* const from = queues + cur * N;
+    uint16_t* const to = queues + (cur ^ 1u) * N;
+    const uint32_t count = sh_count[cur], m = sh_least[cur], goal = sh_goal;
+    if (count == 0u) {
+      completion = APGAR_B200_COMPLETION_REACHED;  // converged; refined below
+      break;
+    }
+    if (rounds >= p.maximum_rounds) break;
+    if (sh_stop != 0u) {
+      completion = APGAR_B200_COMPLETION_CANCELLED;
+      break;
+    }
+    if (p.workspace_mode == 0 && m > goal) {
+      // every label not above the best goal label is final
+      completion = APGAR_B200_COMPLETION_REACHED;
+      break;
+    }
+    const uint32_t threshold = m + delta, next_stamp = rounds + 2u;
+    uint32_t least = kNoLabel;
+    const uint32_t pairs = count * 8u;
+    for (uint32_t base = 0; base < pairs; base += kBlock) {
+      const uint32_t pr = base + tid;
+      bool enqueue = false;
+      uint32_t target = 0;
+      // the eight lanes of a node, one direction each
+      const bool valid = pr < pairs;
+      const uint32_t n = valid ? from[pr >> 3] : 0u, d = static_cast<uint32_t>(lane) & 7u;
+      uint32_t waiting = kNoLabel;
+      if (valid && d == 0u) {
+        waiting = *reinterpret_cast<volatile uint32_t*>(pend + n);
+        if (waiting < threshold && !keep_pend) waiting = atomicExch(pend + n, kNoLabel);
+      }
+      __syncwarp();
+      waiting = __shfl_sync(0xFFFFFFFFu, waiting, lane & ~7);
+      const bool open = valid && waiting < threshold;
+      const uint32_t mine = open ? *reinterpret_cast<volatile uint32_t*>(lab + n * 9u + d) : kNoLabel;
+      // the least label of the other seven headings
+      uint32_t others = kNoLabel, all = mine;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        const uint32_t v = __shfl_xor_sync(0xFFFFFFFFu, all, o);
+        others = min(others, v);
+        all = min(all, v);
+      }
+      if (valid && !open) {
+        if (d == 0u && waiting != kNoLabel) {  // carried to the next round
+          enqueue = atomicExch(stamp + n, next_stamp) != next_stamp;
+          target = n;
+          least = min(least, waiting);
+        }
+      } else if (open && ((legal[n] >> d) & 1u) != 0u) {
+        ++examined;
+        const uint32_t start = *reinterpret_cast<volatile uint32_t*>(lab + n * 9u + 8u);  // no bend from the start
+        const uint32_t turned = others == kNoLabel ? kNoLabel : others + cost_bend;
+        const uint32_t dep = min(min(mine, turned), start);
+        if (turned < mine && turned <= start) ++turns;
+        const uint32_t nb = next_of[d * N + n];
+        if (dep != kNoLabel && nb != 0xFFFFu) {
+          const uint32_t c = move_cost(n, nb, d);
+          if (c != kNoLabel) {
+            const uint32_t cand = dep + c;
+            if (cand < atomicMin(lab + nb * 9u + d, cand)) {
+              __threadfence_block();  // the label before the pend that announces it
+              // keep_pend: the bucket counts the node's best label ever
+              least = min(least, keep_pend ? min(cand, atomicMin(pend + nb, cand)) : cand);
+              if (!keep_pend) atomicMin(pend + nb, cand);
+              if (nb == q.goal_node) atomicMin(&sh_goal, cand);
+              enqueue = atomicExch(stamp + nb, next_stamp) != next_stamp;
+              target = nb;
+            }
+          }
+        }
+      }
+      __syncwarp();
+      const unsigned mask = __ballot_sync(0xFFFFFFFFu, enqueue);
+      if (mask != 0u) {
+        uint32_t first = 0;
+        if (lane == 0) first = atomicAdd(&sh_count[cur ^ 1u], __popc(mask));
+        first = __shfl_sync(0xFFFFFFFFu, first, 0);
+        if (enqueue) to[first + __popc(mask & ((1u << lane) - 1u))] = static_cast<uint16_t>(target);
+      }
+    }
+    least = __reduce_min_sync(0xFFFFFFFFu, least);
+    if (lane == 0 && least != kNoLabel) atomicMin(&sh_least[cur ^ 1u], least);
+    __syncthreads();
+    // this round's slots are the round after next's; its own are read after
+    // the barrier below
+    ++rounds;
+    if (tid == 0) {
+      sh_count[cur] = 0u;
+      sh_least[cur] = kNoLabel;
+      // the cancel flag is host-mapped memory (every read crosses the bus):
+      // read every 64 rounds
+      if (p.cancel != nullptr && (rounds % 64u) == 0u && *p.cancel != 0u) sh_stop = 1u;
+    }
+    __syncthreads();
+  }
+  if (examined != 0u) atomicAdd(&sh_examined, static_cast<unsigned long long>(examined));
+  if (turns != 0u) atomicAdd(&sh_turns, static_cast<unsigned long long>(turns));
+  // ---- goal state (smallest label, then smallest state) ----
+  if (warp == 0) {
+    const uint32_t label = lane < 8 ? lab[q.goal_node * 9u + lane] : kNoLabel;
+    const uint32_t best = __reduce_min_sync(0xFFFFFFFFu, label);
+    const unsigned who = __ballot_sync(0xFFFFFFFFu, label == best && lane < 8);
+    if (lane == 0) sh_goal_state = best == kNoLabel ? kInvalid32 : q.goal_node * 9u + static_cast<uint32_t>(__ffs(who) - 1);
+  }
+  __syncthreads();
+  const uint32_t goal_state = sh_goal_state;
+  if (completion == APGAR_B200_COMPLETION_REACHED && goal_state == kInvalid32) {
+    completion = APGAR_B200_COMPLETION_DISCONNECTED;
+  }
+
+  if (p.workspace_mode) {
+    uint64_t* out = p.labels + static_cast<uint64_t>(qi) * S;
+    uint32_t* pred_out = p.predecessors + static_cast<uint64_t>(qi) * S;
+    uint64_t* own = p.state_owners + static_cast<uint64_t>(qi) * S;
+    uint64_t* pown = p.predecessor_owners + static_cast<uint64_t>(qi) * S;
+    for (uint32_t s = tid; s < S; s += kBlock) {
+      const uint32_t here = lab[s], node = s / 9u, h = s - node * 9u;
+      out[s] = here == kNoLabel ? kGraphInf : here;
+      own[s] = q.workspace_owner;
+      pown[s] = q.workspace_owner;
+      // canonical predecessor: the smallest state whose label plus the move
+      // equals this one's (heading 8 only at the start)
+      uint32_t found = kInvalid32;
+      if (h != 8u && here != kNoLabel) {
+        const uint32_t pred = next_of[((h + 4u) & 7u) * N + node];
+        if (pred != 0xFFFFu) {
+          const uint32_t c = move_cost(pred, node, h);
+          if (c != kNoLabel) {
+#pragma unroll
+            for (uint32_t ph = 9; ph-- > 0u;) {
+              const uint32_t l = lab[pred * 9u + ph];
+              const uint32_t t = c + (ph != 8u && ph != h ? cost_bend : 0u);
+              if (l != kNoLabel && l + t == here && (ph != 8u || pred == q.start_node)) found = pred * 9u + ph;
+            }
+          }
+        }
+      }
+      pred_out[s] = found;
+    }
+  } else if (warp == 0) {
+    // canonical reverse walk: lanes 0..8 test the predecessor headings
+    apgar_b200_compact_path_v1 cp{};
+    cp.schema_version = 1;
+    cp.query_id = q.query_id;
+    cp.workspace_owner = q.workspace_owner;
+    uint32_t* stage = p.path_stage + static_cast<uint64_t>(qi) * S;
+    uint32_t n = 0;
+    bool complete = false;
+    if (completion == APGAR_B200_COMPLETION_REACHED) {
+      const uint32_t start_state = q.start_node * 9u + 8u;
+      uint32_t cursor = goal_state;
+      while (n < S) {
+        if (lane == 0) stage[n] = cursor;
+        ++n;
+        if (cursor == start_state) {
+          complete = true;
+          break;
+        }
+        const uint32_t node = cursor / 9u, h = cursor % 9u;
+        if (h == 8u) break;
+        const uint32_t pred = next_of[((h + 4u) & 7u) * N + node];
+        if (pred == 0xFFFFu) break;
+        const uint32_t c = move_cost(pred, node, h), here = lab[cursor];
+        bool ok = false;
+        if (lane < 9 && c != kNoLabel && (lane != 8 || pred == q.start_node)) {
+          const uint32_t l = lab[pred * 9u + lane];
+          ok = l != kNoLabel && l + c + (lane != 8 && static_cast<uint32_t>(lane) != h ? cost_bend : 0u) == here;
+        }
+        const unsigned ballot = __ballot_sync(0xFFFFFFFFu, ok);
+        if (ballot == 0u) break;
+        cursor = pred * 9u + static_cast<uint32_t>(__ffs(ballot) - 1);
+      }
+    }
+    cp.state_count = complete ? n : 0u;
+    if (completion == APGAR_B200_COMPLETION_REACHED && !complete) {
+      completion = APGAR_B200_COMPLETION_DISCONNECTED;  // unreachable with exact labels
+    }
+    if (lane == 0) p.compact[qi] = cp;
+  }
+  if (tid == 0) write_result(p, qi, q, completion, goal_state, rounds, sh_examined, sh_turns);
 }
 
 // Deterministic packing of the compact paths in query order.
@@ -487,12 +799,33 @@ __global__ void graph_pack_copy(const apgar_b200_compact_path_v1* compact, uint3
 // Shared-memory search for graphs whose labels, queues and stamps fit in
 // this many bytes (two CTAs per SM).
 constexpr size_t kSharedSearchBytes = 100 * 1024;
+// Shared memory of the small form per CTA (with the kernel's own 40 bytes, one
+// CTA per SM at the largest).
+constexpr uint32_t kSmallSearchBytes = 226 * 1024;
+constexpr uint32_t kSmallPolicyEdges = 2048;
 // Policy edges staged in shared memory up to this many bytes (2048 edges).
 constexpr size_t kStagedPolicyBytes = 32 * 1024;
 
 cudaError_t launch_graph_search(const GraphLaunch& launch, cudaStream_t stream) {
   if (launch.query_count == 0) return cudaSuccess;
   const size_t n = launch.g.node_count;
+  // the small form: its state in one SM's shared memory, labels in 32 bits
+  const bool fits = n < 0xFFFFu && launch.max_policy_edges <= kSmallPolicyEdges &&
+                    small_layout(static_cast<uint32_t>(n), launch.max_policy_edges).total <= kSmallSearchBytes;
+  if (fits && launch.max_transition < (1ull << 31) / (9ull * n + 1ull)) {
+    const uint32_t bytes = small_layout(static_cast<uint32_t>(n), launch.max_policy_edges).total;
+    const auto run = [&](auto kernel, int block) -> cudaError_t {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(kSmallSearchBytes));
+      if (e != cudaSuccess) return e;
+      kernel<<<launch.query_count, block, bytes, stream>>>(launch);
+      return cudaGetLastError();
+    };
+    // a round's frontier grows with the graph: eight lanes per queued node
+    if (n <= 256) return run(graph_search_small_kernel<256>, 256);
+    if (n <= 1024) return run(graph_search_small_kernel<512>, 512);
+    return run(graph_search_small_kernel<1024>, 1024);
+  }
   // shared layout: labels, queues and stamps; the neighbour table; the policy edges
   const size_t state_bytes = (n * 9u * 8u + n * 12u + 15u) & ~static_cast<size_t>(15);
   const size_t nbr_bytes = n * 8u * 4u;
