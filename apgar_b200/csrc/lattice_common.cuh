@@ -156,7 +156,10 @@ struct TileNetState {
   uint32_t level_width;
   uint32_t limit;         // keys above it no longer matter
   uint32_t start_key;     // the start's key
-  uint32_t reserved[14];
+  uint32_t confined;      // 1 while the search stays in the net's corridor
+  uint32_t exit_key;      // least key of a move out of the corridor
+  uint32_t corridor;      // APGAR_B200_CORRIDOR_* outcome
+  uint32_t reserved[11];
 };
 static_assert(sizeof(TileNetState) == 128, "a line of its own per net: its warps' atomics and looks meet there");
 
@@ -197,6 +200,9 @@ struct TileLaunch {
   const uint32_t* prev_paths;
   NetPlan* redo;
   uint32_t* redo_count;
+  // corridor mode, as in FrontierLaunch
+  const uint32_t* corridor;
+  uint8_t* corridor_status;
   TileClass c[5];          // the widest first
 };
 

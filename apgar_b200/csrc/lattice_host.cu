@@ -508,8 +508,8 @@ int use_prices(PlanObject* plan) {
   return APGAR_B200_OK;
 }
 
-// Corridors are the cell form's: a plan that gets them moves over to it for
-// good (and gives the tile form's workspace back first).
+// Moves a tile plan over to the cell form for good (and gives the tile form's
+// workspace back first).
 int use_cells(PlanObject* plan) {
   if (!plan->tiles) return APGAR_B200_OK;
   APGAR_B200_CUDA("cudaDeviceSynchronize(tile form)", cudaDeviceSynchronize());
@@ -748,6 +748,8 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
     t.skip = plan->skip;
     t.prev_results = plan->prev_results;
     t.prev_paths = plan->prev_paths;
+    t.corridor = fbase.corridor;
+    t.corridor_status = fbase.corridor_status;
     t.redo = plan->redo.get();
     t.redo_count = reinterpret_cast<uint32_t*>(plan->counters.get() + 2 + kClassCount + 1);
     APGAR_B200_CUDA("lattice tiles launch", launch_lattice_tiles(t, plan->sm_count, stream));
@@ -1041,7 +1043,6 @@ extern "C" int apgar_b200_lattice_plan_set_corridors(void* plan, const uint32_t*
       return set_error(APGAR_B200_UNSUPPORTED, "corridors need the frontier generator");
     }
     if (int rc = check_device(p->device); rc != APGAR_B200_OK) return rc;
-    if (int rc = use_cells(p); rc != APGAR_B200_OK) return rc;
     APGAR_B200_CUDA("cudaMalloc(corridor status)",
                     p->corridor_status.ensure(std::max<uint32_t>(p->count, 1)));
   }

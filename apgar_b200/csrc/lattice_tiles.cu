@@ -31,6 +31,15 @@
 // on label + move == label, returns the full-window canonical path
 // (reference tie-break, gpu/cuda/planar_router.cu:977-1009, :1084-1165).
 //
+// Corridor mode first keeps to the net's corridor (only its cells are
+// entered; a diagonal's side cells need not lie in it).  Every legal move from
+// a labelled corridor cell to a free cell outside is an exit with key g + cost
+// + h; the result is certified when the goal's label is strictly below the
+// least exit key (the proof is lattice_frontier.cu's: every exit whose exact
+// key is at most the goal label starts at a cell that is exact here).  If not,
+// the corridor's labels stay, as they are costs of real paths, and the search
+// goes on from every labelled unit without the corridor.
+//
 // What bounds it, and why this split.  One expansion per queued cell
 // (lattice_frontier.cu) costs some 22 scattered 8-byte requests, and its
 // wavefront advances one cell per round of about 10,000 cycles.  Here a
@@ -67,6 +76,7 @@ constexpr uint32_t kBusyKey = 0xFFFFFFFEu;   // of a unit being relaxed
 constexpr uint32_t kSourceBits = 0x3FFu;    // unit flags: sides that lowered something
 constexpr uint32_t kInFar = 1u << 16;       // the unit stands in the far list
 constexpr uint32_t kTouched = 1u << 17;     // the unit's labels have been written
+constexpr uint32_t kWhole = 1u << 18;       // every cell of the unit may lower others (the corridor was lifted)
 // The cancel flag is read across the bus: by one lane, when a net starts and
 // after every so many turns of one warp.
 constexpr uint32_t kCancelPollTurns = 256;
@@ -335,12 +345,14 @@ struct Swept {
 // its label over.  The outermost lanes get their own label back from a
 // shuffle; p + diag is then no better than the straight p + orth, unless a
 // diagonal is cheaper than a straight move (kCheapDiagonal).  Priced, every
-// move into a cell also costs price + i * kPriceStride.
-template <int kStride, int kPriceStride, bool kCheapDiagonal, bool kPriced>
-__device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* price, uint32_t blocked, uint32_t need, uint32_t orth,
+// move into a cell also costs price + i * kPriceStride.  In a corridor
+// (kCorr), `blocked` has the cells outside it too and `sides`, for the
+// diagonals' side cells, only the blocked ones; else both are the same.
+template <int kStride, int kPriceStride, bool kCheapDiagonal, bool kPriced, bool kCorr>
+__device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* price, uint32_t blocked, uint32_t sides, uint32_t need, uint32_t orth,
                                              uint32_t diag, int lane, uint32_t& steps) {
   Swept out{0u, 0u, 0u};
-  uint32_t pair = blocked | (blocked << 1);
+  uint32_t pair = blocked | (sides << 1);
 #pragma unroll 1
   for (int c = 0; c < 32; c += 8) {
     if (((need >> c) & 0xFFu) != 0u) {
@@ -351,7 +363,8 @@ __device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* pri
       uint32_t diff = 0, first = 0, last = 0;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const uint32_t given = unless(blocked, k, p);
+        const uint32_t given = unless(kCorr ? sides : blocked, k, p);
+        const uint32_t straight = kCorr ? unless(blocked, k, p) : given;
         uint32_t before = __shfl_up_sync(kFull, given, 1), after = __shfl_down_sync(kFull, given, 1);
         if constexpr (kCheapDiagonal) {
           if (lane == 0) before = kTileInf;
@@ -359,10 +372,10 @@ __device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* pri
         }
         uint32_t t;
         if constexpr (kPriced) {
-          t = __viaddmin_u32(unless(pair, k, min(before, after)), diag, given + orth);
+          t = __viaddmin_u32(unless(pair, k, min(before, after)), diag, straight + orth);
           t = __viaddmin_u32(min(t, kTileInf), price[k * kPriceStride], v[k]);
         } else {
-          t = __viaddmin_u32(given, orth, v[k]);
+          t = __viaddmin_u32(straight, orth, v[k]);
           t = __viaddmin_u32(unless(pair, k, min(before, after)), diag, t);
         }
         cell[k * kStride] = t;
@@ -383,6 +396,7 @@ __device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* pri
     cell += 8 * kStride;
     price += 8 * kPriceStride;
     blocked >>= 8;
+    sides >>= 8;
     pair >>= 8;
   }
   return out;
@@ -522,8 +536,47 @@ __device__ __forceinline__ uint32_t touched_neighbours(const Space& ws, const La
   return __ballot_sync(kFull, t);
 }
 
+// Not certified: the net goes on without its corridor, from every labelled
+// unit (one warp; nothing is queued or being relaxed).  True when nothing is
+// left active.
+__device__ __noinline__ bool lift_corridor(int tx, int ty, Space ws, TileNetState* st, int lane) {
+  const uint32_t units = ws.far_cap;
+  if (lane == 0) {
+    st->corridor = peek(&st->goal) < kTileInf ? APGAR_B200_CORRIDOR_FALLBACK_EXIT : APGAR_B200_CORRIDOR_FALLBACK_UNREACHED;
+    st->confined = 0u;
+    st->far_count[0] = st->far_count[1] = 0u;
+    atomicAdd(&st->active, 1u);  // this warp, until every unit is queued
+  }
+  for (uint32_t i = lane; i < units; i += 32) {
+    const bool touched = (__ldcg(ws.flags + i) & kTouched) != 0u;
+    __stcg(ws.flags + i, touched ? kTouched | kSourceBits | kWhole : 0u);
+    __stcg(ws.pend + i, touched ? 0u : kNoKey);
+  }
+  __threadfence();
+  __syncwarp();
+  for (uint32_t base = 0; base < units; base += 32) {
+    const uint32_t i = base + lane;
+    // a unit that others have queued since has no kWhole: it was not labelled
+    const bool take = i < units && (__ldcg(ws.flags + i) & kWhole) != 0u;
+    const unsigned lanes = __ballot_sync(kFull, take);
+    if (lane == 0 && lanes != 0u) atomicAdd(&st->active, __popc(lanes));
+    __threadfence();
+    __syncwarp();
+    const int plane = tx * ty, l = static_cast<int>(i) / plane, rest = static_cast<int>(i) - l * plane, y = rest / tx;
+    push_units(st, ws, take, pack_unit(l, y, rest - y * tx), lane);
+  }
+  uint32_t left = 1;
+  if (lane == 0) {
+    __threadfence();
+    left = atomicSub(&st->active, 1u) - 1u;
+  }
+  __syncwarp();
+  return __shfl_sync(kFull, left, 0) == 0u;
+}
+
 // Nothing is queued or being relaxed: opens the next level from the far list,
 // or ends the search (one warp, the one that finished the last unit).
+template <bool kCorr>
 __device__ __noinline__ void open_level(int tx, int ty, Space ws, TileNetState* st, int lane) {
   for (;;) {
     __threadfence();
@@ -534,6 +587,14 @@ __device__ __noinline__ void open_level(int tx, int ty, Space ws, TileNetState* 
     }
     least = __reduce_min_sync(kFull, least);
     if (least > limit || peek(&st->stop) != 0u) {  // every cell whose key still matters is final
+      __syncwarp();
+      if constexpr (kCorr) {
+        const uint32_t goal = peek(&st->goal);
+        if (peek(&st->stop) == 0u && peek(&st->confined) != 0u && (goal >= kTileInf || goal >= peek(&st->exit_key))) {
+          if (!lift_corridor(tx, ty, ws, st, lane)) return;
+          continue;  // its units are already done
+        }
+      }
       __syncwarp();
       if (lane == 0) {
         __threadfence();
@@ -639,14 +700,102 @@ __device__ __forceinline__ bool load_prices(const TileLaunch& p, const Win& win,
   return high;
 }
 
+// A net's corridor: the 64 x 64 coarse bitmap over its window.
+struct Corridor {
+  const uint32_t* bits;
+  int shift;
+};
+
+__device__ __forceinline__ bool in_corridor(const Corridor& corr, const Win& win, int x, int y) {
+  const uint32_t cx = static_cast<uint32_t>(min(max(x, 0), win.w - 1)) >> corr.shift;
+  const uint32_t cy = static_cast<uint32_t>(min(max(y, 0), win.h - 1)) >> corr.shift;
+  return ((__ldg(corr.bits + cy * 2u + (cx >> 5)) >> (cx & 31u)) & 1u) != 0u;
+}
+
+// The corridor cells (bit i) of column x over rows by .. by + 31, or of row y
+// over columns bx .. bx + 31: coarse cells are 4 or more cells a side, and a
+// unit's corner is a corner of one or lies inside it.
+__device__ __forceinline__ uint32_t corridor_column(const Corridor& corr, const Win& win, int x, int by) {
+  const int side = min(32, 1 << corr.shift);
+  uint32_t m = 0;
+  for (int r = 0; r < 32; r += side) m |= in_corridor(corr, win, x, by + r) ? low_bits(side) << r : 0u;
+  return m;
+}
+
+__device__ __forceinline__ uint32_t corridor_row(const Corridor& corr, const Win& win, int y, int bx) {
+  const int side = min(32, 1 << corr.shift);
+  uint32_t m = 0;
+  for (int c = 0; c < 32; c += side) m |= in_corridor(corr, win, bx + c, y) ? low_bits(side) << c : 0u;
+  return m;
+}
+
+// The least key of the moves that leave the corridor from the labelled cells
+// of the given rows of a unit (its labels in the tile).
+__device__ __noinline__ uint32_t exit_key(const LatticeDeviceView& lat, Win win, Corridor corr, Unit u,
+                                          const uint32_t* tile, uint32_t rows, int lane) {
+  Masks m;
+  Rims rims;
+  unit_free(lat, win, u, lane, m, rims);
+  // free cells, and those of them outside the corridor, of this lane's column
+  // and the columns beside it: bit r + 1 is row r, from -1 to 32
+  const auto outside = [&](int x, uint64_t open) {
+    uint64_t in = static_cast<uint64_t>(corridor_column(corr, win, x, u.by)) << 1;
+    if (in_corridor(corr, win, x, u.by - 1)) in |= 1ull;
+    if (in_corridor(corr, win, x, u.by + 32)) in |= 1ull << 33;
+    return open & ~in;
+  };
+  const auto column = [&](int at, uint32_t cells) {  // at: the column's place in the rim lines
+    return line34(static_cast<uint32_t>(rims.top >> at), cells, static_cast<uint32_t>(rims.bottom >> at));
+  };
+  uint64_t open[3], out[3];
+  open[1] = column(lane + 1, m.col_free);
+  out[1] = outside(u.bx + lane, open[1]);
+  open[0] = __shfl_up_sync(kFull, open[1], 1);
+  out[0] = __shfl_up_sync(kFull, out[1], 1);
+  open[2] = __shfl_down_sync(kFull, open[1], 1);
+  out[2] = __shfl_down_sync(kFull, out[1], 1);
+  if (lane == 0) {
+    open[0] = column(0, static_cast<uint32_t>(rims.left >> 1));
+    out[0] = outside(u.bx - 1, open[0]);
+  }
+  if (lane == 31) {
+    open[2] = column(33, static_cast<uint32_t>(rims.right >> 1));
+    out[2] = outside(u.bx + 32, open[2]);
+  }
+  __syncwarp();
+  uint32_t least = kNoKey;
+  if (!__any_sync(kFull, (out[0] | out[1] | out[2]) != 0ull)) return least;
+  for (uint32_t rest = rows; rest != 0u; rest &= rest - 1u) {
+    const int r = __ffs(rest) - 1;
+    const uint32_t label = tile[(r + 1) * kPitch + 1 + lane];
+    if (label < kTileInf && (((out[0] | out[1] | out[2]) >> r) & 7ull) != 0ull) {
+      const int x = u.bx + lane, y = u.by + r;
+#pragma unroll
+      for (int d = 0; d < 9; ++d) {
+        const int dx = d % 3 - 1, dy = d / 3 - 1;
+        if (dx == 0 && dy == 0) continue;
+        bool leaves = ((out[dx + 1] >> (r + 1 + dy)) & 1ull) != 0ull;
+        if (dx != 0 && dy != 0) {
+          leaves = leaves && ((open[dx + 1] >> (r + 1)) & 1ull) != 0ull && ((open[1] >> (r + 1 + dy)) & 1ull) != 0ull;
+        }
+        if (leaves) {
+          least = min(least, label + (dx != 0 && dy != 0 ? lat.diag : lat.orth) + bound_to_goal(lat, win, u.l, x + dx, y + dy));
+        }
+      }
+    }
+  }
+  __syncwarp();
+  return __reduce_min_sync(kFull, least);
+}
+
 // Relaxes one pending unit to its fixed point and makes the neighbours it
 // lowers pending.  Ends by handing its place in `active` to the units it
 // queued.
-template <bool kCheapDiagonal, bool kPriced>
+template <bool kCheapDiagonal, bool kPriced, bool kCorr>
 __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, const Space& ws, uint32_t packed,
                                            const LanePart& part, uint32_t start_unit, int start_cell,
-                                           uint32_t goal_unit, int goal_cell, TileNetState* st, uint32_t* tile,
-                                           uint32_t* prices, int lane) {
+                                           uint32_t goal_unit, int goal_cell, TileNetState* st, const Corridor& corr,
+                                           uint32_t* tile, uint32_t* prices, int lane) {
   const LatticeDeviceView& lat = p.lat;
   const Unit u = unpack_unit(win, packed);
   uint32_t key = 0, flags = 0, steps = 0;
@@ -690,7 +839,7 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     __syncwarp();
     left = __shfl_sync(kFull, left, 0);
     push_units(st, ws, near, unit, lane);
-    if (left == 0u) open_level(win.tx, win.ty, ws, st, lane);
+    if (left == 0u) open_level<kCorr>(win.tx, win.ty, ws, st, lane);
     __syncwarp();
   };
   if (lane == 0) {
@@ -698,7 +847,7 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     // a key above the limit can no longer matter; its side bits stay set,
     // because a source sets its bit before it lowers the key
     if (key <= peek(&st->limit) && peek(&st->stop) == 0u) {
-      flags = atomicAnd(ws.flags + u.id, ~kSourceBits);
+      flags = atomicAnd(ws.flags + u.id, kCorr ? ~(kSourceBits | kWhole) : ~kSourceBits);
       __threadfence();  // the sources' labels are read after their bits
     } else {
       key = kNoKey;
@@ -714,6 +863,15 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     return;
   }
   const bool own = (flags & kTouched) != 0u;
+  const uint32_t col_open = m.col_free, row_open = m.row_free;
+  bool confined = false;
+  if constexpr (kCorr) {
+    confined = __shfl_sync(kFull, peek(&st->confined), 0) != 0u;
+    if (confined) {
+      m.col_free &= corridor_column(corr, win, u.bx + lane, u.by);
+      m.row_free &= corridor_row(corr, win, u.by + lane, u.bx);
+    }
+  }
   const uint32_t exist = neighbours(win, u, lat.layers);
   const uint32_t touched = touched_neighbours(ws, part, u.id, exist, lane);
   load_unit(ws.labels, win, u, touched, own, tile, lane);
@@ -791,6 +949,7 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
                                                                   kPitch, m.rim >> 6, (m.row_free >> 31) != 0u, price_at(lane, 31), orth, diag));
     if (hit != 0u) cols |= 0x80000000u, rows |= hit;
   }
+  if (kCorr && (flags & kWhole) != 0u) rows = cols = kFull;
   down = rows << 1;
   up = rows >> 1;
   right = cols << 1;
@@ -806,7 +965,7 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     }
     __syncwarp();
     if (down != 0u) {
-      const Swept w = sweep_lines<kPitch, kPricePitch, kCheapDiagonal, kPriced>(first_row, prices + lane, ~m.col_free, down, orth, diag, lane, steps);
+      const Swept w = sweep_lines<kPitch, kPricePitch, kCheapDiagonal, kPriced, kCorr>(first_row, prices + lane, ~m.col_free, ~col_open, down, orth, diag, lane, steps);
       down = 0u;
       up |= w.back;
       right |= w.lanes << 1;
@@ -815,8 +974,8 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
       cols |= w.lanes;
     }
     if (up != 0u) {
-      const Swept w = sweep_lines<-kPitch, -kPricePitch, kCheapDiagonal, kPriced>(
-          first_row + 31 * kPitch, prices + 31 * kPricePitch + lane, __brev(~m.col_free), __brev(up), orth, diag, lane, steps);
+      const Swept w = sweep_lines<-kPitch, -kPricePitch, kCheapDiagonal, kPriced, kCorr>(
+          first_row + 31 * kPitch, prices + 31 * kPricePitch + lane, __brev(~m.col_free), __brev(~col_open), __brev(up), orth, diag, lane, steps);
       up = 0u;
       down |= __brev(w.back);
       right |= w.lanes << 1;
@@ -826,7 +985,7 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     }
     __syncwarp();
     if (right != 0u) {
-      const Swept w = sweep_lines<1, 1, kCheapDiagonal, kPriced>(first_col, prices + lane * kPricePitch, ~m.row_free, right,
+      const Swept w = sweep_lines<1, 1, kCheapDiagonal, kPriced, kCorr>(first_col, prices + lane * kPricePitch, ~m.row_free, ~row_open, right,
                                                                 orth, diag, lane, steps);
       right = 0u;
       left |= w.back;
@@ -836,8 +995,8 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
       rows |= w.lanes;
     }
     if (left != 0u) {
-      const Swept w = sweep_lines<-1, -1, kCheapDiagonal, kPriced>(
-          first_col + 31, prices + lane * kPricePitch + 31, __brev(~m.row_free), __brev(left), orth, diag, lane, steps);
+      const Swept w = sweep_lines<-1, -1, kCheapDiagonal, kPriced, kCorr>(
+          first_col + 31, prices + lane * kPricePitch + 31, __brev(~m.row_free), __brev(~row_open), __brev(left), orth, diag, lane, steps);
       left = 0u;
       right |= __brev(w.back);
       down |= w.lanes << 1;
@@ -910,11 +1069,13 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     if (lane > 0) t = __viaddmin_u32(unless(closed, 0, line[-1]), diag, t);
     if (lane < 31) t = __viaddmin_u32(unless(closed, 1, line[1]), diag, t);
     const int y = k == 0 ? u.by - 1 : u.by + 32;
+    if (kCorr && confined && !in_corridor(corr, win, u.bx + lane, y)) t = kTileInf;
     t = priced(t, u.l, u.bx + lane, y);
     const uint32_t f = key_min(t < rim[0], t, u.l, u.bx + lane, y);
     if (lane == k) out_key = f;
     // corners: from the first and the last cell of the line
     uint32_t corner = lane == 0 || lane == 31 ? unless(closed, lane == 0 ? 0 : 1, line[0]) + diag : kTileInf;
+    if (kCorr && confined && !in_corridor(corr, win, u.bx + (lane == 0 ? -1 : 32), y)) corner = kTileInf;
     corner = priced(corner, u.l, u.bx + (lane == 0 ? -1 : 32), y);
     const bool low = (lane == 0 && corner < rim[-1]) || (lane == 31 && corner < rim[1]);
     if (__any_sync(kFull, low)) {
@@ -934,6 +1095,7 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     uint32_t t = unless(~(m.rim >> (10 + k)), 0, line[0]) + orth;
     if (lane > 0) t = __viaddmin_u32(unless(closed, 0, line[-kPitch]), diag, t);
     if (lane < 31) t = __viaddmin_u32(unless(closed, 1, line[kPitch]), diag, t);
+    if (kCorr && confined && !in_corridor(corr, win, u.bx + (k == 0 ? -1 : 32), u.by + lane)) t = kTileInf;
     t = priced(t, u.l, u.bx + (k == 0 ? -1 : 32), u.by + lane);
     const uint32_t f = key_min(t < rim[0], t, u.l, u.bx + (k == 0 ? -1 : 32), u.by + lane);
     if (lane == 2 + k) out_key = f;
@@ -980,6 +1142,13 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     }
     f = __reduce_min_sync(kFull, f);
     if (lane == k && f != kNoKey) out_key = f + static_cast<uint32_t>(abs(l - win.gl)) * via;
+  }
+  if constexpr (kCorr) {
+    if (confined) {
+      const uint32_t leaving = exit_key(lat, win, corr, u, tile, rows, lane);
+      if (lane == 0 && leaving != kNoKey) atomicMin(&st->exit_key, leaving);
+      __syncwarp();
+    }
   }
   if constexpr (kPriced) {
     if (__any_sync(kFull, high) && lane == 0) atomicMax(&st->stop, 3u);
@@ -1101,6 +1270,7 @@ struct TileNet {
   uint32_t units, start_unit, goal_unit;
   int start_cell, goal_cell;
   int sl, sx, sy;
+  Corridor corr;
 };
 
 __device__ __forceinline__ TileNet net_at(const TileLaunch& p, uint32_t index, uint32_t slot) {
@@ -1129,6 +1299,9 @@ __device__ __forceinline__ TileNet net_at(const TileLaunch& p, uint32_t index, u
   n.sy = static_cast<int>(net.start_y) - n.win.y0;
   n.units = static_cast<uint32_t>(p.lat.layers) * n.win.tx * n.win.ty;
   n.ws = space_at(base, n.units);
+  n.corr.bits = p.corridor == nullptr ? nullptr : p.corridor + static_cast<size_t>(plan.net) * 128u;
+  n.corr.shift = 2;  // at most 63 coarse cells a side
+  while (((max(n.win.w, n.win.h) - 1) >> n.corr.shift) >= 63) ++n.corr.shift;
   if (p.cell_cost_own != nullptr) n.ws.own = p.own_bits + (base - p.c[0].pool) / 32;
   n.start_unit = pack_unit(n.sl, n.sy >> 5, n.sx >> 5);
   n.goal_unit = pack_unit(n.win.gl, n.win.gy >> 5, n.win.gx >> 5);
@@ -1229,6 +1402,16 @@ __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n,
       }
     }
   }
+  uint32_t confined = 0, outcome = APGAR_B200_CORRIDOR_NONE;
+  if (n.corr.bits != nullptr) {
+    uint32_t any = 0;
+    for (int i = lane; i < 128; i += 32) any |= __ldg(n.corr.bits + i);
+    confined = in_corridor(n.corr, n.win, n.sx, n.sy) && in_corridor(n.corr, n.win, n.win.gx, n.win.gy) ? 1u : 0u;
+    // an empty bitmap proposes no corridor
+    const bool proposed = __any_sync(kFull, any != 0u);
+    outcome = confined != 0u ? APGAR_B200_CORRIDOR_CERTIFIED
+                             : (proposed ? APGAR_B200_CORRIDOR_FALLBACK_UNREACHED : APGAR_B200_CORRIDOR_NONE);
+  }
   __syncwarp();
   if (lane == 0) {
     const uint32_t h0 = bound_to_goal(p.lat, n.win, n.sl, n.sx, n.sy);
@@ -1240,6 +1423,9 @@ __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n,
     st->goal = kTileInf;
     st->limit = kNoLimit;
     st->start_key = h0;
+    st->confined = confined;
+    st->exit_key = kNoKey;
+    st->corridor = outcome;
     st->stop = p.cancel != nullptr && *p.cancel != 0u ? 1u : 0u;
     st->steps = st->units = st->levels = 0u;
     st->slot = slot;
@@ -1296,7 +1482,10 @@ __device__ __forceinline__ void finish_net(const TileLaunch& p, const TileNet& n
       res.arena_offset = base;
     }
   }
-  if (lane == 0) p.results[net] = res;
+  if (lane == 0) {
+    p.results[net] = res;
+    if (p.corridor_status != nullptr) p.corridor_status[net] = static_cast<uint8_t>(peek(&st->corridor));
+  }
 }
 
 // A kept route (partial rip-up): the net's previous result and path go into
@@ -1324,7 +1513,7 @@ __device__ __forceinline__ void keep_net(const TileLaunch& p, uint32_t net, int 
 // finds no net left is a guest of other warps' nets: it relaxes their units
 // until they have none to spare.  A guest may leave at any time: a net's
 // owner finishes it alone.
-template <bool kCheapDiagonal, bool kPriced>
+template <bool kCheapDiagonal, bool kPriced, bool kCorr>
 __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kernel(const __grid_constant__ TileLaunch p) {
   extern __shared__ __align__(16) uint32_t tile_smem[];
   __shared__ Lookout look;
@@ -1411,8 +1600,8 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
     }
     const uint32_t unit = pop_unit(st, n.ws, lane);
     if (unit != kEmptySlot) {
-      relax_unit<kCheapDiagonal, kPriced>(p, n.win, n.ws, unit, part, n.start_unit, n.start_cell, n.goal_unit,
-                                          n.goal_cell, st, tile, prices, lane);
+      relax_unit<kCheapDiagonal, kPriced, kCorr>(p, n.win, n.ws, unit, part, n.start_unit, n.start_cell, n.goal_unit,
+                                                 n.goal_cell, st, n.corr, tile, prices, lane);
       __syncwarp();
       idle = misses = 0;
       continue;
@@ -1453,9 +1642,14 @@ constexpr int tile_smem_bytes(bool priced) {
 
 using TileKernel = void (*)(TileLaunch);
 
-TileKernel tile_kernel(bool cheap_diagonal, bool priced) {
-  if (cheap_diagonal) return priced ? lattice_tiles_kernel<true, true> : lattice_tiles_kernel<true, false>;
-  return priced ? lattice_tiles_kernel<false, true> : lattice_tiles_kernel<false, false>;
+template <bool kCheapDiagonal>
+TileKernel tile_kernel(bool priced, bool corridor) {
+  if (corridor) return priced ? lattice_tiles_kernel<kCheapDiagonal, true, true> : lattice_tiles_kernel<kCheapDiagonal, false, true>;
+  return priced ? lattice_tiles_kernel<kCheapDiagonal, true, false> : lattice_tiles_kernel<kCheapDiagonal, false, false>;
+}
+
+TileKernel tile_kernel(bool cheap_diagonal, bool priced, bool corridor) {
+  return cheap_diagonal ? tile_kernel<true>(priced, corridor) : tile_kernel<false>(priced, corridor);
 }
 
 // CTAs per SM that every form of the kernel can keep resident.
@@ -1473,9 +1667,9 @@ cudaError_t tile_blocks_per_sm(int* out) {
     }
   }
   int least = kTileBlocks;
-  for (int form = 0; form < 4; ++form) {
+  for (int form = 0; form < 8; ++form) {
     const bool priced = (form & 2) != 0;
-    const void* kernel = reinterpret_cast<const void*>(tile_kernel((form & 1) != 0, priced));
+    const void* kernel = reinterpret_cast<const void*>(tile_kernel((form & 1) != 0, priced, (form & 4) != 0));
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_bytes(priced));
     int blocks = 0;
     if (e == cudaSuccess) {
@@ -1511,7 +1705,8 @@ cudaError_t launch_lattice_tiles(const TileLaunch& launch, int sm_count, cudaStr
   if (cudaError_t e = lattice_tile_warps(sm_count, &warps); e != cudaSuccess) return e;
   const unsigned grid = warps / (kTileThreads / 32);
   const bool priced = launch.cell_cost != nullptr;
-  tile_kernel(launch.lat.diag < launch.lat.orth, priced)<<<grid, kTileThreads, tile_smem_bytes(priced), stream>>>(launch);
+  const TileKernel kernel = tile_kernel(launch.lat.diag < launch.lat.orth, priced, launch.corridor != nullptr);
+  kernel<<<grid, kTileThreads, tile_smem_bytes(priced), stream>>>(launch);
   return cudaGetLastError();
 }
 

@@ -520,9 +520,9 @@ APGAR_B200_API int apgar_b200_lattice_plan_info(void* plan, apgar_b200_plan_info
  *            bound) in key levels of `bucket_width`, persistent and
  *            work-stealing, largest windows first.  It stops once every cell
  *            with key <= the goal label is final.  Two forms: over 32 x 32
- *            tiles (plans without a bound on the rounds, chains or
- *            corridors, and without windows above 2^25 cells), and over
- *            single cells (the rest), one warp group per net.  Result
+ *            tiles (plans without a bound on the rounds and without chains
+ *            or windows above 2^25 cells), and over single cells (the rest,
+ *            and priced nets near the 32-bit limit).  Result
  *            counters, tiles / cells: sweeps = units relaxed / rounds,
  *            row_steps = line steps of 32 cells / cell expansions,
  *            row_stores = key levels opened, row_loads = 0.  They depend on

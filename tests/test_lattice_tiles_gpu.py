@@ -133,3 +133,46 @@ def test_priced_results_equal_the_cell_forms(layers, width, height, high):
         for field in ("cost", "completion", "path_len", "path_offset"):
             assert np.array_equal(a[field], b[field]), field
         assert np.array_equal(pa, pb)
+
+
+@pytest.mark.parametrize("layers,size,hpwl,margin", [(1, 2112, 1500, 400), (2, 640, 300, 90), (3, 160, 40, 9)])
+@pytest.mark.parametrize("priced", [False, True])
+def test_corridor_outcomes_equal_the_cell_forms(layers, size, hpwl, margin, priced):
+    # coarse cells from 4 to 64 lattice cells a side (a unit holds 64 to part of one)
+    import torch
+
+    from apgar_b200 import corridor
+
+    lat = synth.make_lattice(400 + layers, layers, size, 0.2, via_mask=layers > 1)
+    nets = synth.make_nets(lat, 401, 24, hpwl_median=float(hpwl), hpwl_sigma=0.3, margin=margin)
+    if size == 2112:
+        assert max(corridor.coarse_shift(int(n["win_w"]), int(n["win_h"])) for n in nets) >= 5
+    rng = np.random.default_rng(402)
+    masks = np.concatenate([corridor.segment_corridor(nets[:8], 0), corridor.segment_corridor(nets[8:16], 2),
+                            corridor.segment_corridor(nets[16:], 5)])
+    masks &= rng.random(masks.shape) < 0.97
+    bits = torch.from_numpy(corridor.pack(masks).view(np.int32)).cuda().view(torch.uint32)
+    prices = None
+    if priced:
+        cells = layers * size * size
+        price = np.where(rng.random(cells) < 0.1, rng.integers(1, 60, cells), 0).astype(np.uint32)
+        prices = torch.from_numpy(price.view(np.int32)).cuda()
+    dev = apgar_b200.DeviceLattice(lat)
+    try:
+        out = []
+        for rounds in (1 << 30, CELL_FORM):
+            plan = dev.plan(nets, generator="frontier", max_rounds=rounds)
+            plan.set_cell_costs(prices)
+            plan.set_corridors(bits)
+            plan.execute()
+            res, paths = plan.readback()
+            out.append((res, paths.copy(), plan.corridor_status()))
+            plan.close()
+    finally:
+        dev.close()
+    (a, pa, sa), (b, pb, sb) = out
+    assert np.array_equal(sa, sb), (sa, sb)
+    assert len(set(sa.tolist())) > 1
+    for field in ("cost", "completion", "path_len"):
+        assert np.array_equal(a[field], b[field]), field
+    assert np.array_equal(pa, pb)
