@@ -349,50 +349,6 @@ struct ConvArgs {
 
 enum { kEpiRelu = 0, kEpiGate = 1 };
 
-// The input halo of a 128-cell tile (rows y0 - 1 .. y0 + 2, columns -1 .. 64
-// of one net): [4][66][cin] bf16, zero outside the window.
-template <int CIN>
-struct Halo {
-  static constexpr int kCols = kGrid + 2;
-  static constexpr int kUnits = 4 * kCols * (CIN / 8);  // 16-byte chunks
-  static constexpr int kBytes = kUnits * 16;
-};
-
-// Stages a tile's halo with every load of a thread in flight before its
-// first store (one exposed latency per tile instead of one per chunk).
-template <int CIN>
-__device__ __forceinline__ void stage_halo(const __nv_bfloat16* x, uint32_t net, int y0, int cw, int ch,
-                                           uint8_t* halo, int tid) {
-  constexpr int kUnits = Halo<CIN>::kUnits;
-  constexpr int kPer = (kUnits + 127) / 128;
-  uint4 v[kPer];
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int u = tid + k * 128;
-    v[k] = make_uint4(0u, 0u, 0u, 0u);
-    if (u < kUnits) {
-      const int j = u % (CIN / 8), rest = u / (CIN / 8);
-      const int c = rest % Halo<CIN>::kCols, r = rest / Halo<CIN>::kCols;
-      const int sy = y0 - 1 + r, sx = c - 1;
-      if (sx >= 0 && sy >= 0 && sx < cw && sy < ch) {
-        v[k] = __ldg(reinterpret_cast<const uint4*>(x + act_cell(net, sy, sx) * CIN) + j);
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int u = tid + k * 128;
-    if (u < kUnits) reinterpret_cast<uint4*>(halo)[u] = v[k];
-  }
-}
-
-// Halo chunk j of the input cell read by output cell m (0..127) through tap t.
-template <int CIN>
-__device__ __forceinline__ uint4 halo_chunk(const uint8_t* halo, int m, int t, int j) {
-  const int r = m / kGrid + t / 3, c = m % kGrid + t % 3;
-  return reinterpret_cast<const uint4*>(halo)[(r * Halo<CIN>::kCols + c) * (CIN / 8) + j];
-}
-
 // The forward conv's operands.  A: the tile's four input rows (y0 - 1 ..
 // y0 + 2, 64 cells each) staged as CIN / 8 planes of 16-byte chunks (8
 // channels of one cell).  Each plane is [128-byte lead][256 cells][128-byte
@@ -720,135 +676,280 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_tc_kernel(const __grid_c
 
 // ------------------- weight gradient on tensor cores ----------------------
 
+// dw[co][tap][ci] += sum over cells of x[cell + tap][ci] * dy[cell][co];
+// db[co] += sum over cells of dy[cell][co].
+//
+// The contraction runs over cells, and a stage holds its cells exactly as the
+// MN-major operands want them, so there is no im2col copy.  A tile is two
+// output rows y0, y0 + 1 of one net.  Its four input rows y0 - 1 .. y0 + 2 land
+// by one TMA copy as [row r][chunk of 8 channels][cell] planes of 16-byte
+// units, its two gradient rows as [row yy][chunk][cell].  With the rows of A
+// being (r, ci) (8 channels per plane, planes one after another) and the rows
+// of B being (yy, co), one M = 128, N = 64 product per K = 16 cells gives
+//   D[(r, ci)][(yy, co)] = sum over cells of x[r][cell + dx][ci] * dy[yy][cell][co],
+// the taps dy = r - yy - 1 of one dx for two rows at once; the three dx are
+// three accumulators whose A (dx = -1) or B (dx = +1) starts one cell earlier.
+// The cell before a plane is the previous plane's last column (zero: a window
+// is at most 63, or in the narrow form 31, columns wide) or, before the first
+// plane, the zeroed lead.  The blocks with r - yy outside 0 .. 2 are never
+// read; the second row of a window of odd height is left out (N = 32), since
+// its lower neighbour may lie below the rows the layout defines.
+//
+// Bound by the loads (20 to 24 KB of planes per tile).  The kernel it replaced
+// built the 288 x 128 im2col operand in shared memory with ordinary loads and
+// stores, one tile at a time: about 12,000 cycles a tile against about 600 for
+// the products; 32 -> 32 channels, 256 nets of about 42 x 42 cells: 240 us a
+// layer before, 42 us now.
 struct WgradArgs {
-  const __nv_bfloat16* x;   // layer input [n][64][64][cin]
-  const __nv_bfloat16* dy;  // gradient at the layer's pre-activation [n][64][64][32]
   const uint32_t* dims;
   uint32_t count;
-  float* dw;                // [32][9 * cin] (added to)
-  float* db;                // [32] (added to)
+  float* dw;  // [32][9 * cin] (added to)
+  float* db;  // [32] (added to)
   uint32_t* error;
 };
 
 template <int CIN>
 struct WgradSmem {
-  static constexpr int K = 9 * CIN;                    // rows of D
-  static constexpr int kTiles = (K + 127) / 128;       // M tiles of 128 rows
-  static constexpr int kSbo = 2048;                    // 16 K-groups x 128 bytes
-  static constexpr int kBytesTile = 16 * kSbo;         // 128 rows x 128 cells
-  static constexpr int kBytesA = kTiles * kBytesTile;
-  static constexpr int kBytesB = 4 * kSbo;             // 32 rows x 128 cells
-  static constexpr int kBytes = kBytesA + kBytesB + Halo<CIN>::kBytes + 16;
+  static constexpr int K = 9 * CIN;
+  static constexpr int kLead = 128;                            // zeros before each operand
+  static constexpr int kBytesX = 4 * (CIN / 8) * kGrid * 16;   // four input rows
+  static constexpr int kBytesDy = 2 * (kCh / 8) * kGrid * 16;  // two gradient rows
+  static constexpr int kOffDy = kLead + kBytesX + kLead;
+  static constexpr int kStage = kOffDy + kBytesDy;
+  static constexpr int kStages = 8;  // one CTA per SM: 0.13 to 0.2 MB of loads in flight
+  static constexpr int kTx = kBytesX + kBytesDy;
+  static constexpr int kOffBar = kStages * kStage;  // full, empty, done
+  static constexpr int kBytes = kOffBar + 8 * (2 * kStages + 1);
+  static_assert(kStage % 128 == 0, "TMA destinations are 128-byte aligned");
+  // With 16 input channels the product's rows 64 .. 127 read 8 KB past the
+  // input planes: inside the stage, and into rows that nothing reads.
+  static_assert(kLead + 16 * kGrid * 16 <= kStage, "A's 16 planes lie inside the stage");
+  static_assert(3 * 32 * 128 * 4 <= kStages * kStage, "the epilogue's exchange reuses the stages");
 };
+constexpr uint32_t kWgradCols = 64;     // accumulator columns of one dx: (yy, co)
+constexpr uint32_t kWgradTmem = 256;    // 3 * 64, as a power of two
 
-// dw[co][tap * CIN + ci] += sum over cells of x[cell + tap][ci] * dy[cell][co];
-// db[co] += sum over cells of dy[cell][co].  Operands MN-major: element
-// (row r, cell k) at (r % 8) * 2 + (k % 8) * 16 + (r / 8) * SBO + (k / 8) * 128.
+// Rows `row` on (four of the input, two of the gradient), the first 64 or 32
+// columns: box {8, columns, chunks, rows} at {0, 0, 0, padded row}.
+__device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap* map, int row, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %2, "
+      "%3}], [%4];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(row), "r"(bar)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_zero32(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
+      "r"(0)
+      : "memory");
+}
+
+// Tile `item` (net = item / 32, y0 = 2 * (item % 32)); one exists when y0 < ch.
+struct WgradTile {
+  uint32_t net;
+  int y0, cw, ch;
+  int pitch;  // cells per plane: 32 when the window is at most 31 columns wide, else 64
+};
+__device__ __forceinline__ bool wgrad_tile(const uint32_t* dims, uint32_t item, WgradTile& t) {
+  t.net = item / (kGrid / 2);
+  t.y0 = static_cast<int>(item % (kGrid / 2)) * 2;
+  const uint32_t d = __ldg(dims + t.net);
+  t.cw = static_cast<int>(dims_w(d));
+  t.ch = static_cast<int>(dims_h(d));
+  t.pitch = t.cw < kGrid / 2 ? kGrid / 2 : kGrid;
+  return t.y0 < t.ch;
+}
+__device__ __forceinline__ uint32_t next_wgrad_item(const uint32_t* dims, uint32_t item, uint32_t items,
+                                                    WgradTile& t) {
+  for (; item < items; item += gridDim.x) {
+    if (wgrad_tile(dims, item, t)) return item;
+  }
+  return items;
+}
+
+// Roles as in the convolution: warp 4 lane 0 loads, warp 5 lane 0 issues the
+// MMAs, warps 0-3 sum the bias gradient from the staged rows (warp = chunk)
+// and drain the accumulators once at the end.
 template <int CIN>
-__global__ void __launch_bounds__(128) conv_wgrad_tc_kernel(WgradArgs a) {
+__global__ void __launch_bounds__(kConvThreads)
+    conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap xnarrow,
+                         const __grid_constant__ CUtensorMap dymap, const __grid_constant__ CUtensorMap dynarrow,
+                         WgradArgs a) {
   using S = WgradSmem<CIN>;
+  constexpr int kSt = S::kStages;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* sa = smem;
-  uint8_t* sb = smem + S::kBytesA;
-  uint8_t* halo = smem + S::kBytesA + S::kBytesB;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + S::kBytesA + S::kBytesB + Halo<CIN>::kBytes);
+  const uint32_t bar0 = smem_addr(smem + S::kOffBar);
+  const auto full = [&](int st) { return bar0 + 8u * static_cast<uint32_t>(st); };
+  const auto empty = [&](int st) { return bar0 + 8u * static_cast<uint32_t>(kSt + st); };
+  const uint32_t done = bar0 + 8u * static_cast<uint32_t>(2 * kSt);
   __shared__ uint32_t tmem_slot;
-  __shared__ float bias_part[32];
+  __shared__ int abort_flag;
+  __shared__ uint32_t loaded, waited;  // stages loaded / whose loads the MMA role waited for
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // rows K .. kTiles * 128 of the last tile stay zero
-  for (int u = tid; u < S::kBytesA / 16; u += 128) reinterpret_cast<uint4*>(sa)[u] = make_uint4(0, 0, 0, 0);
-  if (tid < 32) bias_part[tid] = 0.f;
-  if (warp == 0) tmem_alloc(&tmem_slot, 128);
-  if (tid == 0) bar_init(smem_addr(bar), 1);
+
+  // the leads before both operands of every stage stay zero (TMA writes planes only)
+  for (int u = tid; u < kSt * 2 * (S::kLead / 16); u += kConvThreads) {
+    const int st = u / (2 * (S::kLead / 16)), i = u % (2 * (S::kLead / 16));
+    const int at = i < S::kLead / 16 ? i * 16 : S::kOffDy - S::kLead + (i - S::kLead / 16) * 16;
+    *reinterpret_cast<uint4*>(smem + st * S::kStage + at) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (warp == 5) tmem_alloc(&tmem_slot, kWgradTmem);
+  if (tid == 0) {
+    for (int st = 0; st < kSt; ++st) {
+      bar_init(full(st), 1);
+      bar_init(empty(st), 1 + kEpiWarps);
+    }
+    bar_init(done, 1);
+    abort_flag = 0;
+    loaded = waited = 0;
+  }
+  fence_async_smem();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  const uint32_t idesc = idesc_bf16(128, 32, 1, 1);
-  uint32_t phase = 0;
-  bool failed = false, any = false;
-  float bsum = 0.f;  // this thread's share of db (co = tid % 32)
-
-  const uint32_t items = a.count * (kGrid / 2);
-  for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) {
-    const uint32_t net = item / (kGrid / 2);
-    const int y0 = static_cast<int>(item % (kGrid / 2)) * 2;
-    const uint32_t d = a.dims[net];
-    const int cw = static_cast<int>(dims_w(d)), ch = static_cast<int>(dims_h(d));
-    if (y0 >= ch) continue;
-    // B: dy chunks (8 channels) per cell; zero outside the window
-    for (int u = tid; u < 128 * 4; u += 128) {
-      const int k = u % 128, j = u / 128;
-      const int py = y0 + k / kGrid, px = k % kGrid;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (px < cw && py < ch) v = __ldg(reinterpret_cast<const uint4*>(a.dy + act_cell(net, py, px) * kCh) + j);
-      *reinterpret_cast<uint4*>(sb + (k % 8) * 16 + j * S::kSbo + (k / 8) * 128) = v;
-    }
-    // A: im2col rows (tap, ci) per cell, from the staged halo (cells outside
-    // the window carry finite halo values against a zero dy)
-    stage_halo<CIN>(a.x, net, y0, cw, ch, halo, tid);
-    __syncthreads();
-    for (int u = tid; u < 128 * 9 * (CIN / 8); u += 128) {
-      const int k = u % 128, r = u / 128;
-      const int j = r % (CIN / 8), t = r / (CIN / 8);
-      const uint4 v = halo_chunk<CIN>(halo, k, t, j);
-      const int row = t * CIN + j * 8;
-      *reinterpret_cast<uint4*>(sa + (row / 128) * S::kBytesTile + (k % 8) * 16 + ((row % 128) / 8) * S::kSbo +
-                                (k / 8) * 128) = v;
-    }
-    fence_async_smem();
-    __syncthreads();
-    // bias gradient from the staged dy (thread: channel tid % 32, cells tid / 32 + 4 i)
-    {
-      const int c = tid % 32;
-      for (int k = tid / 32; k < 128; k += 4) {
-        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(
-            sb + (k % 8) * 16 + (c / 8) * S::kSbo + (k / 8) * 128) + (c % 8);
-        bsum += __bfloat162float(*e);
-      }
-    }
-    if (tid == 0) {
-      fence_after_sync();
-      const uint32_t b0 = smem_addr(sb);
-#pragma unroll 1
-      for (int mt = 0; mt < S::kTiles; ++mt) {
-        const uint32_t a0 = smem_addr(sa) + mt * S::kBytesTile;
-#pragma unroll 1
-        for (int kk = 0; kk < 8; ++kk) {
-          mma_bf16(tmem + mt * 32, umma_desc(a0 + kk * 256, 128, S::kSbo),
-                   umma_desc(b0 + kk * 256, 128, S::kSbo), idesc, (any || kk > 0) ? 1u : 0u);
-        }
-      }
-      mma_commit(smem_addr(bar));
-    }
-    any = true;
-    const bool ok = bar_wait(smem_addr(bar), phase);
-    phase ^= 1u;
-    if (__syncthreads_or(!ok)) {
-      failed = true;
-      break;
-    }
-  }
-  if (failed) {
-    if (tid == 0) atomicOr(a.error, APGAR_B200_CNN_TIMEOUT);
-    bar_wait(smem_addr(bar), phase);
-  } else if (any) {
-    fence_after_sync();
-    for (int mt = 0; mt < S::kTiles; ++mt) {
-      float v[32];
-      tmem_load32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + mt * 32, v);
-      const int row = mt * 128 + warp * 32 + lane;
-      if (row < S::K) {
+  const uint32_t mine = tmem + (static_cast<uint32_t>(warp * 32) << 16);  // warps 0-3: their lanes
+  if (warp < kEpiWarps) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) atomicAdd(a.dw + c * S::K + row, v[c]);
-      }
-    }
-    atomicAdd(&bias_part[tid % 32], bsum);
+    for (uint32_t c = 0; c < 3 * kWgradCols; c += 32) tmem_zero32(mine + c);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   }
   fence_before_sync();
   __syncthreads();
-  if (!failed && any && tid < 32) atomicAdd(a.db + tid, bias_part[tid]);
-  if (warp == 0) tmem_free(tmem, 128);
+  fence_after_sync();
+
+  const uint32_t items = a.count * (kGrid / 2);
+  const volatile int* abort_v = &abort_flag;
+  // a bounded wait; on expiry every role stops at its next check
+  const auto wait = [&](uint32_t bar, uint32_t parity) {
+    if (bar_wait(bar, parity)) return true;
+    atomicExch(&abort_flag, 1);
+    return false;
+  };
+  WgradTile tile;
+  float bsum[8];  // warp j: this lane's cells of channels 8 j .. 8 j + 7
+#pragma unroll
+  for (int i = 0; i < 8; ++i) bsum[i] = 0.f;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      uint32_t k = 0;
+      for (uint32_t item = next_wgrad_item(a.dims, blockIdx.x, items, tile); item < items;
+           item = next_wgrad_item(a.dims, item + gridDim.x, items, tile), ++k) {
+        const int st = static_cast<int>(k % kSt);
+        if (*abort_v || !wait(empty(st), ((k / kSt) & 1u) ^ 1u)) break;
+        const int row = static_cast<int>(tile.net * kPadRows) + tile.y0;  // padded index of row y0 - 1
+        const uint32_t dst = smem_addr(smem + st * S::kStage);
+        const bool wide = tile.pitch == kGrid;
+        bar_expect_tx(full(st), wide ? S::kTx : S::kTx / 2);
+        tma_load_rows(dst + S::kLead, wide ? &xmap : &xnarrow, row, full(st));
+        tma_load_rows(dst + S::kOffDy, wide ? &dymap : &dynarrow, row + 1, full(st));
+      }
+      loaded = k;
+    }
+  } else if (warp == 5) {
+    if (lane == 0) {
+      uint32_t k = 0, consumed = 0;
+      for (uint32_t item = next_wgrad_item(a.dims, blockIdx.x, items, tile); item < items;
+           item = next_wgrad_item(a.dims, item + gridDim.x, items, tile), ++k) {
+        const int st = static_cast<int>(k % kSt);
+        if (*abort_v || !wait(full(st), (k / kSt) & 1u)) break;
+        ++consumed;
+        fence_after_sync();
+        const uint32_t a0 = smem_addr(smem + st * S::kStage) + S::kLead;
+        const uint32_t b0 = smem_addr(smem + st * S::kStage) + S::kOffDy;
+        const uint32_t plane = static_cast<uint32_t>(tile.pitch) * 16u;
+        const uint32_t idesc = idesc_bf16(128, tile.y0 + 1 < tile.ch ? 64 : 32, 1, 1);
+        const int steps = tile.cw / 16 + 1;  // cells 0 .. cw, and for dx = +1 one later
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+          const uint32_t ad = a0 - (dx == 0 ? 16u : 0u), bd = b0 - (dx == 2 ? 16u : 0u);
+          for (int kk = 0; kk < steps; ++kk) {
+            mma_bf16(tmem + dx * kWgradCols, umma_desc(ad + kk * 256, 128, plane),
+                     umma_desc(bd + kk * 256, 128, plane), idesc, 1u);
+          }
+        }
+        mma_commit(empty(st));
+      }
+      waited = consumed;
+      // every MMA is done before the accumulators are read or freed
+      mma_commit(done);
+      wait(done, 0u);
+    }
+  } else {
+    uint32_t k = 0;
+    for (uint32_t item = next_wgrad_item(a.dims, blockIdx.x, items, tile); item < items;
+         item = next_wgrad_item(a.dims, item + gridDim.x, items, tile), ++k) {
+      const int st = static_cast<int>(k % kSt);
+      const bool ok = !*abort_v && wait(full(st), (k / kSt) & 1u);
+      if (__any_sync(0xFFFFFFFFu, !ok)) break;
+      const uint4* dy = reinterpret_cast<const uint4*>(smem + st * S::kStage + S::kOffDy);
+#pragma unroll
+      for (int yy = 0; yy < 2; ++yy) {
+        for (int c = lane; c < tile.pitch; c += 32) {
+          float v[8];
+          unpack8(dy[(yy * (kCh / 8) + warp) * tile.pitch + c], v);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) bsum[i] += v[i];
+        }
+      }
+      __syncwarp();
+      if (lane == 0) bar_arrive(empty(st));
+    }
+  }
+  __syncthreads();
+  if (warp == 4 && lane == 0) {
+    // loads nobody waited for (only after an expired wait): let them land
+    // before the CTA's shared memory goes away
+    for (uint32_t k = waited; k < loaded; ++k) {
+      bar_wait(full(static_cast<int>(k % kSt)), (k / kSt) & 1u);
+    }
+  }
+  const bool failed = abort_flag != 0;
+  if (failed) {
+    if (tid == 0) atomicOr(a.error, APGAR_B200_CNN_TIMEOUT);
+  } else if (loaded != 0) {  // uniform
+    // tap (t, dx) = D[(r = t, ci)][(0, co)] + D[(r = t + 1, ci)][(1, co)]
+    fence_after_sync();
+    float* part = reinterpret_cast<float*>(smem);  // [dx][co][row of D]: the second rows' terms
+    const int row = warp * 32 + lane;
+    float v[32];
+    if (warp < kEpiWarps) {
+#pragma unroll 1
+      for (int dx = 0; dx < 3; ++dx) {
+        tmem_load32(mine + dx * kWgradCols + 32, v);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) part[(dx * 32 + c) * 128 + row] = v[c];
+      }
+    }
+    __syncthreads();
+    if (warp < kEpiWarps) {
+      const int t = row / CIN, ci = row % CIN;
+#pragma unroll 1
+      for (int dx = 0; dx < 3; ++dx) {
+        tmem_load32(mine + dx * kWgradCols, v);
+        if (t < 3) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            atomicAdd(a.dw + c * S::K + (t * 3 + dx) * CIN + ci, v[c] + part[(dx * 32 + c) * 128 + row + CIN]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        for (int o = 16; o > 0; o >>= 1) bsum[i] += __shfl_xor_sync(0xFFFFFFFFu, bsum[i], o);
+        if (lane == i) atomicAdd(a.db + warp * 8 + i, bsum[i]);
+      }
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  if (warp == 5) tmem_free(tmem, kWgradTmem);
 }
 
 // ------------------------------ head + loss -------------------------------
@@ -1208,16 +1309,41 @@ cudaError_t launch_conv(const ConvArgs& a, int sm_count, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
+// An activation or gradient tensor [count][66][64][C] bf16 as {8 channels,
+// 64 columns, C / 8 chunks, rows}: a box {8, columns, C / 8, rows} lands as
+// [row][chunk][cell] planes.
+cudaError_t plane_map(const void* x, uint32_t count, int channels, int columns, int rows, CUtensorMap* map) {
+  const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+  if (encode == nullptr) return cudaErrorNotSupported;
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0) return cudaErrorInvalidValue;
+  const cuuint32_t elem[4] = {1, 1, 1, 1};
+  const cuuint64_t cell = static_cast<cuuint64_t>(channels) * 2;
+  const cuuint64_t dims[4] = {8, kGrid, static_cast<cuuint64_t>(channels / 8),
+                              static_cast<cuuint64_t>(count) * kPadRows};
+  const cuuint64_t strides[3] = {cell, 16, kGrid * cell};
+  const cuuint32_t box[4] = {8, static_cast<cuuint32_t>(columns), static_cast<cuuint32_t>(channels / 8),
+                             static_cast<cuuint32_t>(rows)};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), dims, strides, box,
+                            elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 template <int CIN>
-cudaError_t launch_wgrad(const WgradArgs& a, int sm_count, cudaStream_t stream) {
+cudaError_t launch_wgrad(const WgradArgs& a, const void* x, const void* dy, int sm_count, cudaStream_t stream) {
   const int bytes = WgradSmem<CIN>::kBytes;
-  cudaError_t e = cudaFuncSetAttribute(conv_wgrad_tc_kernel<CIN>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return e;
   const uint32_t items = a.count * (kGrid / 2);
-  const uint32_t grid = min(items, static_cast<uint32_t>(max(sm_count, 1) * 2));
-  if (grid == 0) return cudaSuccess;
-  conv_wgrad_tc_kernel<CIN><<<grid, 128, bytes, stream>>>(a);
+  if (items == 0) return cudaSuccess;
+  CUtensorMap xmap, xnarrow, dymap, dynarrow;
+  cudaError_t e = plane_map(x, a.count, CIN, kGrid, 4, &xmap);
+  if (e == cudaSuccess) e = plane_map(x, a.count, CIN, kGrid / 2, 4, &xnarrow);
+  if (e == cudaSuccess) e = plane_map(dy, a.count, kCh, kGrid, 2, &dymap);
+  if (e == cudaSuccess) e = plane_map(dy, a.count, kCh, kGrid / 2, 2, &dynarrow);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(conv_wgrad_tc_kernel<CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return e;
+  const uint32_t grid = min(items, static_cast<uint32_t>(max(sm_count, 1)));
+  conv_wgrad_tc_kernel<CIN><<<grid, kConvThreads, bytes, stream>>>(xmap, xnarrow, dymap, dynarrow, a);
   return cudaGetLastError();
 }
 
@@ -1302,14 +1428,13 @@ cudaError_t launch_backward(const float* params, const void* operands, const voi
   int cur = 0;
   for (int l = 4; l >= 0; --l) {
     WgradArgs wa{};
-    wa.x = static_cast<const __nv_bfloat16*>(l == 0 ? rasters : acts[l - 1]);
-    wa.dy = static_cast<const __nv_bfloat16*>(g[cur]);
     wa.dims = dims;
     wa.count = count;
     wa.dw = grads + P.w[l];
     wa.db = grads + P.b[l];
     wa.error = error;
-    e = l == 0 ? launch_wgrad<kCin0>(wa, sm_count, stream) : launch_wgrad<kCh>(wa, sm_count, stream);
+    e = l == 0 ? launch_wgrad<kCin0>(wa, rasters, g[cur], sm_count, stream)
+               : launch_wgrad<kCh>(wa, acts[l - 1], g[cur], sm_count, stream);
     if (e != cudaSuccess) return e;
     if (l == 0) break;
     ConvArgs a{};
