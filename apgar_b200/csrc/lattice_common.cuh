@@ -67,6 +67,7 @@ struct SweepLaunch {
   uint64_t path_arena_capacity;
   unsigned long long* arena_cursor;
   const volatile uint32_t* cancel;  // host-mapped flag or nullptr
+  int row_warps;                    // warps side by side in a row (set by the launcher)
 };
 
 // One width class of the frontier form (lattice_frontier.cu).  The kernel

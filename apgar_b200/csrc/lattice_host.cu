@@ -20,9 +20,10 @@
 
 namespace apgar_b200 {
 
-int lattice_cells_per_lane(int layers);
-size_t lattice_sweep_smem_bytes(int layers, int warps_per_net, int max_rows);
-cudaError_t launch_lattice_sweep(int layers, int warps_per_net, const SweepLaunch& launch,
+bool lattice_sweep_shape(int layers, int index, int* cells, int* warps);
+uint32_t lattice_sweep_widest(int layers);
+size_t lattice_sweep_smem_bytes(int layers, int cells, int warps, int max_rows);
+cudaError_t launch_lattice_sweep(int layers, int cells, int warps, SweepLaunch launch,
                                  int max_rows, cudaStream_t stream);
 cudaError_t launch_accumulate_cells(const apgar_b200_lattice_result* results, uint32_t count,
                                     const uint32_t* paths, uint32_t* usage, uint64_t cell_count,
@@ -67,12 +68,9 @@ cudaError_t launch_corridors(const float* logits, const uint32_t* dims,
 
 namespace {
 
-// Width classes: warps per net.  A sweep net takes the fewest warps whose
-// lanes cover its frame row (each lane holds lattice_cells_per_lane(L) cells
-// of every layer, so G warps cover 32 * C * G cells): the widest class is
-// issue-bound, and warps past the row's end would run every instruction on
-// padding.  The frontier's classes are 1, 2, 4, 8 and 16 warps.
-constexpr int kGroupSizes[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16};
+// Width classes.  A sweep net's class is a shape of lattice_sweep_shape (cells
+// per lane and warps side by side on each layer); the frontier's classes are
+// 1, 2, 4, 8 and 16 warps a net.
 constexpr int kClassCount = 16;
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;
 constexpr size_t kStatesAt = 32;  // of PlanObject::counters (256 bytes on: the states are 128 bytes each)
@@ -80,7 +78,8 @@ constexpr size_t kStatesAt = 32;  // of PlanObject::counters (256 bytes on: the 
 struct LatticeObject;
 
 struct ClassRange {
-  int warps_per_net = 0;
+  int warps_per_net = 0;  // SWEEP: of each layer
+  int cells = 0;          // SWEEP: per lane
   uint32_t begin = 0;  // into plans
   uint32_t count = 0;
   int max_rows = 0;
@@ -242,16 +241,17 @@ int check_device(int expected) {
   return APGAR_B200_OK;
 }
 
-// Smallest width class whose row coverage holds `width` cells; -1 if none.
+// Smallest sweep class whose row coverage holds `width` cells; -1 if none.
 int class_for_width(uint32_t width, int layers) {
-  const uint32_t per_warp = 32u * static_cast<uint32_t>(lattice_cells_per_lane(layers));
-  for (int i = 0; i < kClassCount; ++i) {
-    if (per_warp * static_cast<uint32_t>(kGroupSizes[i]) >= width) return i;
+  if (width > lattice_sweep_widest(layers)) return -1;
+  int cells = 0, warps = 0;
+  for (int i = 0; i < kClassCount && lattice_sweep_shape(layers, i, &cells, &warps); ++i) {
+    if (32u * static_cast<uint32_t>(cells) * static_cast<uint32_t>(warps) >= width) return i;
   }
   return -1;
 }
 
-// Frontier width class (index into kGroupSizes) from the window's cell count.
+// Frontier width class (warps per net as a power of two) from the window's cell count.
 // A frontier round is a chain of dependent memory waves, so its latency falls
 // when more warps share a round's cells; the thresholds (measured on the
 // medium batch: 4-layer windows of 10^4 to 10^7 cells) give every window
@@ -605,7 +605,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
       return ca > cb;
     });
     ClassRange range;
-    range.warps_per_net = kGroupSizes[ci];
+    lattice_sweep_shape(v.layers, ci, &range.cells, &range.warps_per_net);
     range.begin = static_cast<uint32_t>(plans.size());
     range.count = static_cast<uint32_t>(m.size());
     for (uint32_t i : m) {
@@ -622,7 +622,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
       range.max_rows = std::max(range.max_rows, static_cast<int>(np.rows));
       plans.push_back(np);
     }
-    if (lattice_sweep_smem_bytes(v.layers, range.warps_per_net, range.max_rows) > kMaxSmemPerBlock) {
+    if (lattice_sweep_smem_bytes(v.layers, range.cells, range.warps_per_net, range.max_rows) > kMaxSmemPerBlock) {
       return set_error(APGAR_B200_UNSUPPORTED, "window too tall for the shared-memory row map");
     }
     plan->classes.push_back(range);
@@ -835,7 +835,7 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
       APGAR_B200_CUDA("cudaStreamWaitEvent", cudaStreamWaitEvent(s, plan->fork, 0));
     }
     APGAR_B200_CUDA("lattice sweep launch",
-                    launch_lattice_sweep(v.layers, c.warps_per_net, launch, c.max_rows, s));
+                    launch_lattice_sweep(v.layers, c.cells, c.warps_per_net, launch, c.max_rows, s));
     if (fan_out) {
       APGAR_B200_CUDA("cudaEventRecord(join)", cudaEventRecord(plan->joins[k], s));
       APGAR_B200_CUDA("cudaStreamWaitEvent", cudaStreamWaitEvent(stream, plan->joins[k], 0));
@@ -1422,6 +1422,18 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
     h.width_class[i] = static_cast<int8_t>(ci);
   }
 
+  // The launches follow one another on the caller's stream, so the nets of
+  // rows that one warp covers share one: each takes the shape of the widest.
+  // (A launch of its own for each shape measured 1.16 ms against 0.73 for the
+  // 96 nets of a planar board.)
+  constexpr int kOneWarp = 2;
+  int shared_class = -1;
+  for (uint32_t i = 0; i < count; ++i) {
+    if (h.width_class[i] <= kOneWarp) shared_class = std::max(shared_class, static_cast<int>(h.width_class[i]));
+  }
+  for (uint32_t i = 0; i < count; ++i) {
+    if (h.width_class[i] >= 0 && h.width_class[i] < shared_class) h.width_class[i] = static_cast<int8_t>(shared_class);
+  }
   // Plan records, class by class, larger windows first (ties by net index).
   ClassRange ranges[kClassCount];
   int range_count = 0;
@@ -1440,7 +1452,7 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
     });
     ClassRange& range = ranges[range_count++];
     range = ClassRange{};
-    range.warps_per_net = kGroupSizes[ci];
+    lattice_sweep_shape(v.layers, ci, &range.cells, &range.warps_per_net);
     range.begin = planned;
     range.count = members;
     for (uint32_t k = 0; k < members; ++k) {
@@ -1458,7 +1470,7 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
       arena_cells += 8ull * (n.win_w + n.win_h) + 64ull * v.layers;
       range.max_rows = std::max(range.max_rows, static_cast<int>(np.rows));
     }
-    if (lattice_sweep_smem_bytes(v.layers, range.warps_per_net, range.max_rows) >
+    if (lattice_sweep_smem_bytes(v.layers, range.cells, range.warps_per_net, range.max_rows) >
         kMaxSmemPerBlock) {
       return set_error(APGAR_B200_UNSUPPORTED, "window too tall for the shared-memory row map");
     }
@@ -1527,7 +1539,7 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
     launch.plans = d_plans + ranges[k].begin;
     launch.plan_count = ranges[k].count;
     APGAR_B200_CUDA("lattice sweep launch",
-                    launch_lattice_sweep(v.layers, ranges[k].warps_per_net, launch,
+                    launch_lattice_sweep(v.layers, ranges[k].cells, ranges[k].warps_per_net, launch,
                                          ranges[k].max_rows, stream));
   }
   APGAR_B200_CUDA("lattice pack launch",

@@ -7,28 +7,36 @@
 // column-major bit planes uploaded with the lattice serve that case); the
 // move model is symmetric under the swap.
 //
-// Work split: a net is owned by a group of G warps; each lane owns C
-// consecutive cells of the frame row on every layer (L*C labels in
-// registers), so a group covers rows of up to 32*C*G cells.  Small nets use
-// one warp (no block barrier at all) and several nets share a CTA; wide nets
-// use G warps that meet at named barriers once per row-local pass.
+// Work split: a net is a CTA, a warp holds one layer of 32 * C consecutive
+// cells of the frame row (C labels per lane in registers), and G warps side by
+// side cover the row on each of the L layers.  The sweep of one net is a chain
+// of dependent row steps and a batch ends with its longest chains, so what
+// counts is the latency of a step: up to 512 cells the warps' instructions one
+// after the other, beyond that the integer throughput of the net's one SM.  Two
+// things keep instructions out of a step: a row that the relaxation leaves
+// alone ends there, and a warp whose labels nothing changed skips its scan and
+// its via cascade.  With all layers of a chunk in one warp a warp had 4 x C
+// cells to go through and no way to skip any: 1,024 nets of 4 x 1024^2, median
+// row 162 cells, took 11.1 ms, 8.6 now; 96 planar nets, where the gain is
+// fewer cells a lane and the rows that end early, 0.89 ms and 0.56.
 //
 // A row step:
 //   1. relaxes the row from the previous row in sweep order (straight plus
-//      both diagonals; the previous row stays in registers between steps);
+//      both diagonals; the previous row stays in registers between steps) and
+//      applies the via cascade across layers;
 //   2. runs, for every layer, a two-sided row scan: the east and west
 //      one-sided scans of the same input combined by min (equal to an east
 //      scan followed by a west scan on every connected segment).  Each is a
-//      lane-serial add-min chain, a 5-step warp shuffle scan of
-//      (value, crossing cost) lane summaries and a fold over the group's
-//      preceding warps;
-//   3. applies the via cascade across layers inside each lane (registers
-//      only) and repeats 2-3 until no via lowers a label;
+//      lane-serial add-min chain, a 5-step warp shuffle scan of lane summaries
+//      and a fold over the row's preceding warps;
+//   3. applies the via cascade again and repeats 2-3 until no via lowers a
+//      label.  The layers meet in shared memory: every warp publishes its
+//      labels, and each lane folds the column of its cells from the lowest
+//      layer up and from the highest down to its own;
 //   4. writes back only the layers whose labels changed.
-// Blocked cells hold INF and every update is clamped back to INF there, so
-// orthogonal moves need no legality test; diagonal moves test their two side
-// cells.  The next row's labels and mask bits are prefetched while the
-// current row is processed whenever the schedule guarantees it will run.
+// Blocked cells hold INF and a move into one costs INF, so orthogonal moves
+// need no legality test; diagonal moves test their two side cells.  The next
+// row's labels and mask bits are loaded while the current row is processed.
 //
 // Schedule (restated on the CPU by the oracle, lo_sweep_schedule): a row is
 // skipped when neither it nor its predecessor row changed since the previous
@@ -62,20 +70,19 @@ struct Frame {
   int x0, y0;
 };
 
-// Per-lane view of the guard-padded sweep planes for one net: the two words
-// holding the lane's span (frame positions xs-1 .. xs+C) of frame row r on
-// layer l sit at base + l*layer_stride + r*row_stride.
+// Per-lane view of one layer's guard-padded sweep planes for one net: the two
+// words holding the lane's span (frame positions xs-1 .. xs+C) of frame row r
+// sit at base + r*row_stride.
 struct BitSpan {
   const uint32_t* blocked;
-  const uint32_t* via;  // nullptr without a via mask
-  size_t layer_stride;
-  int row_stride;
+  const uint32_t* via;  // nullptr without a via mask; layer pair (layer, layer + 1)
+  uint32_t row_stride;
   int shift;
   uint32_t valid;  // span positions inside the frame (bit j <-> position xs-1+j)
 };
 
 template <int C>
-__device__ __forceinline__ BitSpan make_span(const LatticeDeviceView& lat, const Frame& f, int xs) {
+__device__ __forceinline__ BitSpan make_span(const LatticeDeviceView& lat, const Frame& f, int xs, int layer) {
   static_assert(C + 2 <= 32, "a lane's span must fit one word");
   BitSpan s;
   const int origin = f.transposed ? f.y0 : f.x0;
@@ -83,12 +90,12 @@ __device__ __forceinline__ BitSpan make_span(const LatticeDeviceView& lat, const
   const int first_row = f.transposed ? f.x0 : f.y0;
   const int rows_in_plane = f.transposed ? lat.width : lat.height;
   s.row_stride = (f.transposed ? lat.words_t : lat.words) + 2;
-  s.layer_stride = static_cast<size_t>(rows_in_plane) * s.row_stride;
   // a lane wholly outside the frame clamps its position; its valid mask is 0
   const int pos = min(origin + xs - 1, limit);
   const int wi = pos >> 5;  // -1 for pos == -1: the leading guard word
   s.shift = pos & 31;
-  const size_t base = static_cast<size_t>(first_row) * s.row_stride + 1 + wi;
+  const size_t base =
+      (static_cast<size_t>(layer) * rows_in_plane + static_cast<size_t>(first_row)) * s.row_stride + 1 + wi;
   s.blocked = (f.transposed ? lat.sweep_cols : lat.sweep_rows) + base;
   const uint32_t* via_plane = f.transposed ? lat.sweep_via_cols : lat.sweep_via_rows;
   s.via = via_plane == nullptr ? nullptr : via_plane + base;
@@ -104,17 +111,34 @@ __device__ __forceinline__ BitSpan make_span(const LatticeDeviceView& lat, const
   return s;
 }
 
-// Free bits of the lane's span (bit j+1 is the lane's cell j).
-__device__ __forceinline__ uint32_t span_free(const BitSpan& s, int l, int r) {
-  const uint32_t* w = s.blocked + l * s.layer_stride + static_cast<size_t>(r) * s.row_stride;
-  return ~__funnelshift_r(__ldg(w), __ldg(w + 1), s.shift) & s.valid;
+// The two words of a plane that hold the lane's span of frame row r.  They are kept as loaded until the row is processed, so that nothing
+// waits for a prefetch when it is issued.
+__device__ __forceinline__ uint2 span_words(const BitSpan& s, const uint32_t* plane, int r) {
+  const uint32_t* w = plane + static_cast<uint32_t>(r) * s.row_stride;
+  return make_uint2(__ldg(w), __ldg(w + 1));
 }
 
-// Via bits of layer pair (l, l+1) for the span; all ones without a via mask.
-__device__ __forceinline__ uint32_t span_via(const BitSpan& s, int l, int r) {
-  if (s.via == nullptr) return 0xFFFFFFFFu;
-  const uint32_t* w = s.via + l * s.layer_stride + static_cast<size_t>(r) * s.row_stride;
-  return __funnelshift_r(__ldg(w), __ldg(w + 1), s.shift);
+// Free bits of the lane's span (bit j+1 is the lane's cell j).
+__device__ __forceinline__ uint32_t span_free(const BitSpan& s, uint2 w) {
+  return ~__funnelshift_r(w.x, w.y, s.shift) & s.valid;
+}
+
+// 0 where bit j is set, INF where it is clear.
+__device__ __forceinline__ uint32_t inf_unless(uint32_t bits, int j) {
+  return ((bits >> j) & 1u) ? 0u : kLabelInf;
+}
+
+// Shuffles that stop at a lane of the caller's choice: a lane whose source
+// lies beyond `stop` gets its own value back.
+__device__ __forceinline__ uint32_t shfl_up_to(uint32_t v, int by, int stop) {
+  uint32_t d;
+  asm volatile("shfl.sync.up.b32 %0, %1, %2, %3, 0xFFFFFFFF;" : "=r"(d) : "r"(v), "r"(by), "r"(stop));
+  return d;
+}
+__device__ __forceinline__ uint32_t shfl_down_to(uint32_t v, int by, int stop) {
+  uint32_t d;
+  asm volatile("shfl.sync.down.b32 %0, %1, %2, %3, 0xFFFFFFFF;" : "=r"(d) : "r"(v), "r"(by), "r"(stop));
+  return d;
 }
 
 template <int C>
@@ -196,51 +220,60 @@ __device__ __forceinline__ bool via_bit_at(const LatticeDeviceView& lat,
 __constant__ int kDxc[8] = {1, 1, 0, -1, -1, -1, 0, 1};
 __constant__ int kDyc[8] = {0, 1, 1, 1, 0, -1, -1, -1};
 
-// Nets (warp groups) per CTA: small groups share a CTA to keep blocks at 128+
-// threads.
-__host__ __device__ constexpr int groups_per_block(int G) { return G >= 4 ? 1 : 4 / G; }
-
-// Per-group shared memory carve-up (shared by the kernel and the host).
-struct GroupSmem {
-  size_t modified, edges, sums, flags, total;
+// Shared memory of a CTA (shared by the kernel and the host).
+struct SweepSmem {
+  size_t modified, labels, bits, edges, sums, flags, total;
 };
 
-__host__ __device__ inline GroupSmem group_smem(int L, int G, int max_rows) {
-  GroupSmem s{};
+__host__ __device__ inline SweepSmem sweep_smem(int L, int C, int G, int max_rows) {
+  SweepSmem s{};
   size_t off = 0;
   s.modified = off;
   off += (static_cast<size_t>(max_rows) * sizeof(int16_t) + 15) & ~size_t(15);
-  s.edges = off;  // [2 buffers][G][L][first, last] of the previous row
-  off += 2 * static_cast<size_t>(G) * L * 2 * sizeof(uint32_t);
-  s.sums = off;  // [G][L][aE, bE, aW, bW]
-  off += static_cast<size_t>(G) * L * 4 * sizeof(uint32_t);
-  s.flags = off;  // [2 parities][G]: bit 0 via improved, bit 1 changed, bit 8+l layer l changed
-  off += 2 * static_cast<size_t>(G) * sizeof(uint32_t);
+  s.labels = off;  // [2][L][G][C / 4][32 lanes] uint4: the exchanged labels
+  if (L > 1) off += 2 * static_cast<size_t>(L) * G * 32 * C * sizeof(uint32_t);
+  s.bits = off;  // [L][G][32 lanes]: free cells, and via bits to the layer above << 16
+  if (L > 1) off += static_cast<size_t>(L) * G * 32 * sizeof(uint32_t);
+  s.edges = off;  // [2 buffers][L][G][first, last] of the previous row
+  off += 2 * static_cast<size_t>(L) * G * 2 * sizeof(uint32_t);
+  off = (off + 15) & ~size_t(15);
+  s.sums = off;  // [L][G]: east far-cell value, crossing cost, west far-cell value
+  off += static_cast<size_t>(L) * G * sizeof(uint4);
+  s.flags = off;  // [2 parities][L * G]: bit l: layer l changed
+  off += 2 * static_cast<size_t>(L) * G * sizeof(uint32_t);
   s.total = (off + 15) & ~size_t(15);
   return s;
 }
 
-template <int G>
-__device__ __forceinline__ void group_sync(int barrier_id) {
-  if constexpr (G == 1) {
+// All warps of the net (a barrier of the whole CTA; kOne: its only warp).
+template <bool kOne>
+__device__ __forceinline__ void net_sync() {
+  if constexpr (kOne) {
     __syncwarp();
   } else {
-    __threadfence_block();
-    asm volatile("bar.sync %0, %1;" ::"r"(barrier_id), "r"(G * 32) : "memory");
+    __syncthreads();
   }
 }
 
-template <int L, int C, int G>
-__global__ void __launch_bounds__(groups_per_block(G) * G * 32)
+// Nets an SM should hold: a large batch of narrow nets is bound by the nets in
+// flight (4 layers, 1,000 nets of median row 107: 5.3 ms with the registers
+// the compiler takes by itself, 4.7 with this bound).
+__host__ __device__ constexpr int resident_nets(int L, int C, int kMost) {
+  return kMost > 1 ? 1 : C == 4 ? 20 / L : C == 8 ? 16 / L : 1;
+}
+
+// G = p.row_warps <= kMost warps side by side.
+template <int L, int C, int kMost>
+__global__ void __launch_bounds__(32 * L * kMost, resident_nets(L, C, kMost))
     lattice_sweep_kernel(SweepLaunch p, int max_rows) {
-  constexpr int kGroups = groups_per_block(G);
+  constexpr bool kMulti = kMost > 1;
+  constexpr bool kOne = L == 1 && !kMulti;  // the CTA is one warp
+  const uint32_t plan_index = blockIdx.x;
+  const int G = kMulti ? p.row_warps : 1;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int gi = warp / G;      // group (net) within the CTA
-  const int g = warp - gi * G;  // warp within the group
-  const uint32_t plan_index = blockIdx.x * kGroups + gi;
-  if (plan_index >= p.plan_count) return;  // whole group leaves together
-  const int barrier_id = gi + 1;
+  const int my_layer = L > 1 ? warp / G : 0;
+  const int g = warp - my_layer * G;  // warp within the row
   const NetPlan plan = p.plans[plan_index];
   const apgar_b200_lattice_net net = p.nets[plan.net];
   const LatticeDeviceView& lat = p.lat;
@@ -253,17 +286,25 @@ __global__ void __launch_bounds__(groups_per_block(G) * G * 32)
   f.x0 = static_cast<int>(net.win_x0);
   f.y0 = static_cast<int>(net.win_y0);
   uint32_t* slab = p.dist_pool + plan.dist_offset;
-  const size_t layer_stride = static_cast<size_t>(f.R) * f.pitch;
-  const BitSpan span = make_span<C>(lat, f, xs);
+  // a window's labels are fewer than 2^31: 32-bit offsets into its slab
+  const uint32_t layer_stride = static_cast<uint32_t>(f.R) * static_cast<uint32_t>(f.pitch);
+  uint32_t* const my_slab = slab + static_cast<uint32_t>(my_layer) * layer_stride;
+  const auto row_at = [&](int r) { return my_slab + static_cast<uint32_t>(r) * static_cast<uint32_t>(f.pitch); };
+  const BitSpan span = make_span<C>(lat, f, xs, my_layer);
+  const bool via_words = L > 1 && span.via != nullptr && my_layer + 1 < L;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const GroupSmem gs = group_smem(L, G, max_rows);
-  unsigned char* my_smem = smem_raw + gs.total * gi;
-  int16_t* modified = reinterpret_cast<int16_t*>(my_smem + gs.modified);
-  uint32_t* const sh_edges = reinterpret_cast<uint32_t*>(my_smem + gs.edges);
-  constexpr int kEdgeBuf = G * L * 2;  // entries of one edge buffer
-  uint32_t* sh_sum = reinterpret_cast<uint32_t*>(my_smem + gs.sums);
-  uint32_t* sh_flags = reinterpret_cast<uint32_t*>(my_smem + gs.flags);
+  const SweepSmem gs = sweep_smem(L, C, G, max_rows);
+  int16_t* modified = reinterpret_cast<int16_t*>(smem_raw + gs.modified);
+  uint4* const sh_labels = reinterpret_cast<uint4*>(smem_raw + gs.labels);
+  uint32_t* const sh_bits = reinterpret_cast<uint32_t*>(smem_raw + gs.bits);
+  uint32_t* const sh_edges = reinterpret_cast<uint32_t*>(smem_raw + gs.edges);
+  uint4* const sh_sum = reinterpret_cast<uint4*>(smem_raw + gs.sums) + my_layer * G;
+  uint32_t* const sh_flags = reinterpret_cast<uint32_t*>(smem_raw + gs.flags);
+  const int warps = L * G;
+  const int edge_buf = warps * 2;                  // entries of one edge buffer
+  const int layer_quads = G * (C / 4) * 32;        // uint4 of one layer of exchanged labels
+  const int my_quads = g * (C / 4) * 32 + lane;    // this lane's first quad within a layer
 
   const uint32_t orth = p.lat.orth, diag = p.lat.diag, via = p.lat.via;
   const int lsx = static_cast<int>(net.start_x) - f.x0, lsy = static_cast<int>(net.start_y) - f.y0;
@@ -271,53 +312,54 @@ __global__ void __launch_bounds__(groups_per_block(G) * G * 32)
   const int s_layer = static_cast<int>(net.start_layer), g_layer = static_cast<int>(net.goal_layer);
   const int sr = f.transposed ? lsx : lsy, sp = f.transposed ? lsy : lsx;
 
-  for (int y = g * 32 + lane; y < f.R; y += G * 32) modified[y] = kNever;
+  for (int y = threadIdx.x; y < f.R; y += blockDim.x) modified[y] = kNever;
   const bool endpoints_free =
       cell_free(lat, net, s_layer, lsx, lsy) && cell_free(lat, net, g_layer, lgx, lgy);
-  // counters live in registers (every warp of a group follows the same
-  // control flow; warp 0's copy is reported)
+  // counters live in registers (every warp of a net follows the same control
+  // flow; warp 0's copy is reported)
   uint32_t stat_rows = 0, stat_stores = 0, stat_loads = 0;
   bool fault = false;
-  group_sync<G>(barrier_id);
+  net_sync<kOne>();
 
   uint32_t completion = APGAR_B200_COMPLETION_DISCONNECTED;
   uint32_t sweeps_done = 0;
   if (endpoints_free) {
     {  // initial row: INF except the start cell
+      uint32_t v0[C];
 #pragma unroll
-      for (int l = 0; l < L; ++l) {
-        uint32_t v0[C];
-#pragma unroll
-        for (int j = 0; j < C; ++j) v0[j] = (l == s_layer && xs + j == sp) ? 0u : kLabelInf;
-        store_cells<C>(slab + l * layer_stride + static_cast<size_t>(sr) * f.pitch, f.pitch, xs, v0);
-      }
+      for (int j = 0; j < C; ++j) v0[j] = (my_layer == s_layer && xs + j == sp) ? 0u : kLabelInf;
+      store_cells<C>(row_at(sr), f.pitch, xs, v0);
       modified[sr] = 0;  // same value from every thread
       stat_stores += L;
     }
-    group_sync<G>(barrier_id);
+    net_sync<kOne>();
 
     bool converged = false, cancelled = false;
     int parity = 0;
+    int xb = 0;  // exchange buffer
     // The row step reads its predecessor row's warp-edge labels from buffer
-    // eb and publishes its own into the other buffer before its last group
-    // vote, which therefore also ends the step (no barrier of its own).
+    // eb and publishes its own into the other buffer before its last vote,
+    // which therefore also ends the step (no barrier of its own).
     int eb = 0;
-    uint32_t prv[L][C], nxt[L][C];
-    uint32_t pf[L], nf[L], nvb[L];
+    uint32_t prv[C], nxt[C];
+    uint32_t pf = 0;    // free bits of the previous row
+    uint2 nf{}, nvb{};  // the next row's plane words, as loaded
+    // The carries of the row scan: what a crossing of C cells costs, and of
+    // the chunks to the warp's last and first lane.
+    const uint32_t stepC = orth * C;
+    const uint32_t to_last = static_cast<uint32_t>(31 - lane) * stepC;
+    const uint32_t to_first = static_cast<uint32_t>(lane) * stepC;
     for (uint32_t k = 1; k <= p.max_sweeps; ++k) {
       // The host-mapped flag is read by one thread and broadcast, so every
-      // thread of the group takes the same branch.
-      uint32_t cancel_now = 0;
-      if (g == 0 && lane == 0) cancel_now = (p.cancel != nullptr && *p.cancel != 0u) ? 1u : 0u;
-      if constexpr (G == 1) {
+      // thread of the net takes the same branch.
+      int cancel_now = 0;
+      if (threadIdx.x == 0) cancel_now = (p.cancel != nullptr && *p.cancel != 0u) ? 1 : 0;
+      if constexpr (kOne) {
         cancel_now = __shfl_sync(0xFFFFFFFFu, cancel_now, 0);
       } else {
-        if (g == 0 && lane == 0) sh_flags[parity * G] = cancel_now;
-        group_sync<G>(barrier_id);
-        cancel_now = sh_flags[parity * G];
-        group_sync<G>(barrier_id);
+        cancel_now = __syncthreads_or(cancel_now);
       }
-      if (cancel_now != 0u) {
+      if (cancel_now != 0) {
         cancelled = true;
         break;
       }
@@ -328,12 +370,13 @@ __global__ void __launch_bounds__(groups_per_block(G) * G * 32)
       bool any_change = false;
       bool have_prev = false;
       bool have_next = false;  // nxt/nf/nvb hold this step's row
-      bool next_loaded = false;
+      int16_t mp = kNever, my = kNever, mn = modified[fwd ? 0 : f.R - 1];  // of rows r - dr, r, r + dr
       for (int step = 0; step < f.R; ++step) {
         const int r = fwd ? step : f.R - 1 - step;
-        const int pr = r - dr;
-        const int16_t mp = (pr >= 0 && pr < f.R) ? modified[pr] : kNever;
-        const int16_t my = modified[r];
+        const int pr = r - dr, nr = r + dr;
+        mp = my;
+        my = mn;
+        mn = (step + 1 < f.R) ? modified[nr] : kNever;
         const bool skip = (ki <= 2) ? (mp == kNever && my == kNever)
                                     : (mp <= ki - 2 && my <= ki - 2);
         if (skip) {
@@ -343,336 +386,360 @@ __global__ void __launch_bounds__(groups_per_block(G) * G * 32)
         }
         // ---- previous row (registers, or reloaded after a skipped row) ----
         if (!have_prev) {
+          if (mp != kNever) {
+            load_cells<C>(row_at(pr), f.pitch, xs, prv);
+            pf = span_free(span, span_words(span, span.blocked, pr));
+            stat_loads += L;
+          } else {
 #pragma unroll
-          for (int l = 0; l < L; ++l) {
-            if (mp != kNever) {
-              load_cells<C>(slab + l * layer_stride + static_cast<size_t>(pr) * f.pitch, f.pitch,
-                            xs, prv[l]);
-              pf[l] = span_free(span, l, pr);
-            } else {
-#pragma unroll
-              for (int j = 0; j < C; ++j) prv[l][j] = kLabelInf;
-              pf[l] = 0;
-            }
+            for (int j = 0; j < C; ++j) prv[j] = kLabelInf;
+            pf = 0;
           }
-          if (mp != kNever) stat_loads += L;
-          if constexpr (G > 1) {
-            if (lane == 0 || lane == 31) {
-#pragma unroll
-              for (int l = 0; l < L; ++l) {
-                sh_edges[eb * kEdgeBuf + (g * L + l) * 2 + (lane == 0 ? 0 : 1)] =
-                    lane == 0 ? prv[l][0] : prv[l][C - 1];
-              }
-            }
-            group_sync<G>(barrier_id);
+          if constexpr (kMulti) {
+            if (lane == 0) sh_edges[eb * edge_buf + warp * 2] = prv[0];
+            if (lane == 31) sh_edges[eb * edge_buf + warp * 2 + 1] = prv[C - 1];
+            net_sync<kOne>();
           }
         }
         // ---- current row ----
-        uint32_t v[L][C];
-        uint32_t cf[L], vb[L];
+        uint32_t v[C];
+        uint2 cw, vw;
         if (have_next) {
 #pragma unroll
-          for (int l = 0; l < L; ++l) {
-#pragma unroll
-            for (int j = 0; j < C; ++j) v[l][j] = next_loaded ? nxt[l][j] : kLabelInf;
-            cf[l] = nf[l];
-            vb[l] = nvb[l];
-          }
-          if (next_loaded) stat_loads += L;
+          for (int j = 0; j < C; ++j) v[j] = my != kNever ? nxt[j] : kLabelInf;
+          cw = nf;
+          vw = nvb;
         } else {
-#pragma unroll
-          for (int l = 0; l < L; ++l) {
-            if (my != kNever) {
-              load_cells<C>(slab + l * layer_stride + static_cast<size_t>(r) * f.pitch, f.pitch, xs,
-                            v[l]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < C; ++j) v[l][j] = kLabelInf;
-            }
-            cf[l] = span_free(span, l, r);
-            vb[l] = (l + 1 < L) ? span_via(span, l, r) : 0u;
-          }
-          if (my != kNever) stat_loads += L;
-        }
-        // ---- prefetch the next row when the schedule guarantees it runs ----
-        {
-          const int nr = r + dr;
-          have_next = false;
-          next_loaded = false;
-          if (nr >= 0 && nr < f.R) {
-            const int16_t mn = modified[nr];
-            const bool sure = (ki <= 2) ? (my != kNever || mn != kNever)
-                                        : (my >= ki - 1 || mn >= ki - 1);
-            if (sure) {
-              have_next = true;
-              next_loaded = mn != kNever;
-#pragma unroll
-              for (int l = 0; l < L; ++l) {
-                if (next_loaded) {
-                  load_cells<C>(slab + l * layer_stride + static_cast<size_t>(nr) * f.pitch,
-                                f.pitch, xs, nxt[l]);
-                }
-                nf[l] = span_free(span, l, nr);
-                nvb[l] = (l + 1 < L) ? span_via(span, l, nr) : 0u;
-              }
-            }
-          }
-        }
-        uint32_t orig[L][C];
-        uint32_t blk[L][C];  // 0 where free, INF where blocked
-#pragma unroll
-        for (int l = 0; l < L; ++l) {
-#pragma unroll
-          for (int j = 0; j < C; ++j) {
-            orig[l][j] = v[l][j];
-            blk[l][j] = ((cf[l] >> (j + 1)) & 1u) ? 0u : kLabelInf;
-          }
-        }
-        // ---- 1. relax from the previous row ----
-#pragma unroll
-        for (int l = 0; l < L; ++l) {
-          // diagonal side cells: (p in the previous row, p-1 / p+1 in this row)
-          const uint32_t side_l = (pf[l] >> 1) & cf[l];
-          const uint32_t side_r = (pf[l] >> 1) & (cf[l] >> 2);
-          uint32_t left = __shfl_up_sync(0xFFFFFFFFu, prv[l][C - 1], 1);
-          uint32_t right = __shfl_down_sync(0xFFFFFFFFu, prv[l][0], 1);
-          if constexpr (G > 1) {
-            const uint32_t* const sh_edge = sh_edges + eb * kEdgeBuf;
-            if (lane == 0) left = (g > 0) ? sh_edge[((g - 1) * L + l) * 2 + 1] : kLabelInf;
-            if (lane == 31) right = (g + 1 < G) ? sh_edge[((g + 1) * L + l) * 2 + 0] : kLabelInf;
+          if (my != kNever) {
+            load_cells<C>(row_at(r), f.pitch, xs, v);
           } else {
-            if (lane == 0) left = kLabelInf;
-            if (lane == 31) right = kLabelInf;
+#pragma unroll
+            for (int j = 0; j < C; ++j) v[j] = kLabelInf;
+          }
+          cw = span_words(span, span.blocked, r);
+          vw = via_words ? span_words(span, span.via, r) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+        }
+        if (my != kNever) stat_loads += L;
+        // ---- prefetch the next row: it runs if this one changes, which the
+        // step learns only after the loads would be due (waiting for that
+        // left one step in four with its loads exposed)
+        have_next = step + 1 < f.R;
+        if (have_next) {
+          if (mn != kNever) load_cells<C>(row_at(nr), f.pitch, xs, nxt);
+          nf = span_words(span, span.blocked, nr);
+          nvb = via_words ? span_words(span, span.via, nr) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+        }
+        const uint32_t cf = span_free(span, cw);
+        uint32_t diff = 0;     // labels that changed since the row was loaded
+        uint32_t into[C];      // cost of a straight move into the cell: INF where blocked
+        // ---- 1. relax from the previous row ----
+        {
+          // A diagonal step from (p -+ 1) of the previous row needs two free
+          // side cells: the one below its source (this row), and the one
+          // above its target (previous row).
+          uint32_t src[C], slant[C];
+#pragma unroll
+          for (int j = 0; j < C; ++j) {
+            const bool open = (cf >> (j + 1)) & 1u;
+            into[j] = open ? orth : kLabelInf;
+            slant[j] = open ? diag : kLabelInf;
+            src[j] = open ? prv[j] : kLabelInf;
+          }
+          uint32_t left = __shfl_up_sync(0xFFFFFFFFu, src[C - 1], 1);
+          uint32_t right = __shfl_down_sync(0xFFFFFFFFu, src[0], 1);
+          if (lane == 0) {
+            left = kLabelInf;
+            if (kMulti && g > 0 && (cf & 1u)) left = sh_edges[eb * edge_buf + (warp - 1) * 2 + 1];
+          }
+          if (lane == 31) {
+            right = kLabelInf;
+            if (kMulti && g + 1 < G && ((cf >> (C + 1)) & 1u)) right = sh_edges[eb * edge_buf + (warp + 1) * 2];
+          }
+          uint32_t across[C];
+#pragma unroll
+          for (int j = 0; j < C; ++j) {
+            across[j] = min(j == 0 ? left : src[j - 1], j == C - 1 ? right : src[j + 1]);
+          }
+          if (diag >= orth) {
+            // The previous row is at its fixed point: a free cell there is at
+            // most one straight move above its neighbours, and one that holds
+            // INF (blocked, or as unreached as they are) leaves at least INF.
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+              across[j] = static_cast<uint32_t>(__viaddmax_s32(
+                  static_cast<int>(prv[j]), -static_cast<int>(orth), static_cast<int>(across[j])));
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < C; ++j) across[j] = max(across[j], inf_unless(pf, j + 1));
           }
 #pragma unroll
           for (int j = 0; j < C; ++j) {
-            const uint32_t pl = (j == 0) ? left : prv[l][j - 1];
-            const uint32_t prr = (j == C - 1) ? right : prv[l][j + 1];
-            const uint32_t cl = ((side_l >> j) & 1u) ? diag : kLabelInf;
-            const uint32_t cr = ((side_r >> j) & 1u) ? diag : kLabelInf;
-            uint32_t t = __viaddmin_u32(prv[l][j], orth, v[l][j]);
-            t = __viaddmin_u32(pl, cl, t);
-            t = __viaddmin_u32(prr, cr, t);
-            v[l][j] = max(t, blk[l][j]);
+            const uint32_t t = __viaddmin_u32(across[j], slant[j], __viaddmin_u32(prv[j], into[j], v[j]));
+            diff |= t ^ v[j];
+            v[j] = t;
           }
         }
         // Lanes whose whole chunk is free pass a carry straight through; the
         // nearest non-free lane at or below (east scan) / at or above (west
         // scan) bounds the segment a lane's scan value can come from.
-        const uint32_t stepC = orth * C;
+        constexpr uint32_t kChunk = (1u << C) - 1u;
+        const uint32_t free_lanes = __ballot_sync(0xFFFFFFFFu, ((cf >> 1) & kChunk) == kChunk);
         const uint32_t below_me = (lane == 31) ? 0xFFFFFFFFu : ((2u << lane) - 1u);
-        const uint32_t above_me = ~((1u << lane) - 1u);
-        int segE[L], segW[L];
-        bool through_below[L], through_above[L];
-        uint32_t warp_free[L];
-#pragma unroll
-        for (int l = 0; l < L; ++l) {
-          const uint32_t m = (1u << C) - 1u;
-          const uint32_t free_lanes = __ballot_sync(0xFFFFFFFFu, ((cf[l] >> 1) & m) == m);
-          const uint32_t blocked_lanes = ~free_lanes;
-          const uint32_t lo = blocked_lanes & below_me;
-          const uint32_t hi = blocked_lanes & above_me;
-          segE[l] = lo ? 31 - __clz(lo) : 0;
-          segW[l] = hi ? __ffs(hi) - 1 : 31;
-          through_below[l] = (blocked_lanes & ((1u << lane) - 1u)) == 0u;   // lanes < me all free
-          through_above[l] = (blocked_lanes & ~below_me) == 0u;             // lanes > me all free
-          warp_free[l] = free_lanes;
+        const uint32_t lo = ~free_lanes & below_me, hi = ~free_lanes & ~((1u << lane) - 1u);
+        const int segE = lo ? 31 - __clz(lo) : 0;
+        const int segW = hi ? __ffs(hi) - 1 : 31;
+        const bool through_below = (~free_lanes & ((1u << lane) - 1u)) == 0u;  // lanes < me all free
+        const bool through_above = (~free_lanes & ~below_me) == 0u;            // lanes > me all free
+        // Legal via hops of the lane's cells between layers q and q + 1,
+        // known after the row's first exchange.
+        uint32_t hop[L > 1 ? L - 1 : 1];
+        if constexpr (L > 1) {
+          const uint32_t vb = __funnelshift_r(vw.x, vw.y, span.shift);
+          sh_bits[warp * 32 + lane] = ((cf >> 1) & kChunk) | ((vb >> 1) << 16);
         }
-        // via hop costs of the row (INF where the via bit forbids the hop)
-        uint32_t hopc[L > 1 ? L - 1 : 1][C];
+        // Via cascade: upwards then downwards through consecutive legal vias,
+        // to this warp's layer; returns the bits that changed.
+        // Only what layers `lo` .. `hi` changed can lower a label.
+        const auto via_cascade = [&](const uint4* x, int lo, int hi) -> uint32_t {
+          uint32_t changed = 0;
 #pragma unroll
-        for (int l = 0; l + 1 < L; ++l) {
+          for (int q = 0; q < C / 4; ++q) {
+            uint32_t up[4], down[4];
 #pragma unroll
-          for (int j = 0; j < C; ++j) hopc[l][j] = ((vb[l] >> (j + 1)) & 1u) ? via : kLabelInf;
-        }
-        // via cascade inside the lane: upwards then downwards through
-        // consecutive legal vias (blocked cells clamp the cascade); returns
-        // whether any label changed
-        auto via_cascade = [&]() -> uint32_t {
-          uint32_t diff = 0;
-          if constexpr (L > 1) {
+            for (int i = 0; i < 4; ++i) up[i] = down[i] = kLabelInf;
 #pragma unroll
-            for (int j = 0; j < C; ++j) {
-              uint32_t d = v[0][j];
+            for (int l = 0; l + 1 < L; ++l) {
+              if (l >= lo && l < my_layer) {  // warp-uniform
+                const uint4 t = x[l * layer_quads + q * 32];
+                const uint32_t c[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
-              for (int l = 1; l < L; ++l) {
-                const uint32_t t = max(__viaddmin_u32(d, hopc[l - 1][j], v[l][j]), blk[l][j]);
-                diff |= t ^ v[l][j];
-                v[l][j] = t;
-                d = t;
-              }
-#pragma unroll
-              for (int l = L - 2; l >= 0; --l) {
-                const uint32_t t = max(__viaddmin_u32(d, hopc[l][j], v[l][j]), blk[l][j]);
-                diff |= t ^ v[l][j];
-                v[l][j] = t;
-                d = t;
+                for (int i = 0; i < 4; ++i) {
+                  up[i] = __viaddmin_u32(min(up[i], c[i]), (hop[l] >> (4 * q + i)) & 1u ? via : kLabelInf, kLabelInf);
+                }
               }
             }
+#pragma unroll
+            for (int l = L - 1; l > 0; --l) {
+              if (l <= hi && l > my_layer) {
+                const uint4 t = x[l * layer_quads + q * 32];
+                const uint32_t c[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  down[i] =
+                      __viaddmin_u32(min(down[i], c[i]), (hop[l - 1] >> (4 * q + i)) & 1u ? via : kLabelInf, kLabelInf);
+                }
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t t = __vimin3_u32(up[i], down[i], v[4 * q + i]);
+              changed |= t ^ v[4 * q + i];
+              v[4 * q + i] = t;
+            }
           }
-          return diff;
+          return changed;
         };
-        // a path that switches layer as it arrives needs no second pass
-        via_cascade();
-        // ---- 2./3. row-local fixed point ----
-        // Each pass lowers at least one label, so the loop is finite; the cap
-        // only guards against a broken invariant (reported, never silent).
-        uint32_t row_flags = 0;  // group-wide: bit 1 changed, bit 8+l layer l changed
-        for (int pass = 0;; ++pass) {
-          if (pass == kMaxRowPasses) {
-            fault = true;
-            break;
-          }
-          uint32_t inclE[L], inclW[L];
+        // Publishes this warp's labels (L > 1) and meets the net's other
+        // warps: whether any of them reports `changed`; the labels to read.
+        const uint4* x = nullptr;
+        const auto exchange = [&](bool changed) -> bool {
+          if constexpr (kOne) {
+            return __any_sync(0xFFFFFFFFu, changed);
+          } else {
+            if constexpr (L > 1) {
+              uint4* const out = sh_labels + xb * (L * layer_quads) + my_quads;
 #pragma unroll
-          for (int l = 0; l < L; ++l) {
-            // lane-local one-sided scans: value at the far cell with no carry
-            uint32_t ce = v[l][0];
-#pragma unroll
-            for (int j = 1; j < C; ++j) ce = max(__viaddmin_u32(ce, orth, v[l][j]), blk[l][j]);
-            uint32_t cw = v[l][C - 1];
-#pragma unroll
-            for (int j = C - 2; j >= 0; --j) cw = max(__viaddmin_u32(cw, orth, v[l][j]), blk[l][j]);
-            // segmented min scans over lanes of lane-offset values: a chunk's
-            // far-cell value reaches lane i through free chunks at C*orth each
-            inclE[l] = ce + static_cast<uint32_t>(31 - lane) * stepC;
-            inclW[l] = cw + static_cast<uint32_t>(lane) * stepC;
-          }
-#pragma unroll
-          for (int sft = 1; sft < 32; sft <<= 1) {
-#pragma unroll
-            for (int l = 0; l < L; ++l) {
-              const uint32_t oE = __shfl_up_sync(0xFFFFFFFFu, inclE[l], sft);
-              const uint32_t oW = __shfl_down_sync(0xFFFFFFFFu, inclW[l], sft);
-              if (lane - sft >= segE[l]) inclE[l] = min(inclE[l], oE);
-              if (lane + sft <= segW[l]) inclW[l] = min(inclW[l], oW);
-            }
-          }
-#pragma unroll
-          for (int l = 0; l < L; ++l) {
-            inclE[l] = min(inclE[l] - static_cast<uint32_t>(31 - lane) * stepC, kLabelInf);
-            inclW[l] = min(inclW[l] - static_cast<uint32_t>(lane) * stepC, kLabelInf);
-          }
-          uint32_t warp_cE[L], warp_cW[L];
-#pragma unroll
-          for (int l = 0; l < L; ++l) warp_cE[l] = warp_cW[l] = kLabelInf;
-          if constexpr (G > 1) {
-            // warp summaries: far-cell value without outside carry, and the
-            // cost to cross the whole warp (INF unless every chunk is free)
-            if (lane == 31) {
-#pragma unroll
-              for (int l = 0; l < L; ++l) sh_sum[(g * L + l) * 4 + 0] = inclE[l];
-            }
-            if (lane == 0) {
-#pragma unroll
-              for (int l = 0; l < L; ++l) {
-                sh_sum[(g * L + l) * 4 + 1] = warp_free[l] == 0xFFFFFFFFu ? 32u * stepC : kLabelInf;
-                sh_sum[(g * L + l) * 4 + 2] = inclW[l];
+              for (int q = 0; q < C / 4; ++q) {
+                out[my_layer * layer_quads + q * 32] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
               }
+              x = out;
+              xb ^= 1;
             }
-            group_sync<G>(barrier_id);
+            return __syncthreads_or(changed) != 0;
+          }
+        };
+        // The votes of a row: did a label change since the row was loaded (bit
+        // l for layer l, for the write-back) and since the last exchange (bit
+        // 8), and this row's edges for the next step.  Buffer eb ^ 1 is read by no warp until the next step, and
+        // every read of it by the previous step came before this step's first
+        // barrier.
+        const auto publish_flags = [&](bool recent) {
+          if constexpr (kMulti) {
+            if (lane == 0) sh_edges[(eb ^ 1) * edge_buf + warp * 2] = v[0];
+            if (lane == 31) sh_edges[(eb ^ 1) * edge_buf + warp * 2 + 1] = v[C - 1];
+          }
+          if constexpr (!kOne) {
+            const uint32_t flags = __reduce_or_sync(
+                0xFFFFFFFFu, (diff != 0u ? 1u << my_layer : 0u) | (recent ? 1u << 8 : 0u));
+            if (lane == 0) sh_flags[parity * warps + warp] = flags;
+          }
+        };
+        // The layers of this warp's cells that changed before the last
+        // exchange (bit l); no via can lower a label unless another's did.
+        const auto changed_layers = [&]() -> uint32_t {
+          return __ballot_sync(0xFFFFFFFFu, lane < L && (sh_flags[parity * warps + lane * G + g] & (1u << 8)));
+        };
+        uint32_t row_layers = 0;  // layers that changed
+        // A row that the relaxation does not lower is at its fixed point
+        // already (the start's row is not until it has run): nearly half of
+        // the steps end here.
+        bool dirty = diff != 0u || my == 0;  // this warp's labels are not as a scan left them
+        publish_flags(dirty);
+        if (exchange(dirty)) {
+          dirty = __any_sync(0xFFFFFFFFu, dirty);
+          if constexpr (L > 1) {
+            uint32_t b[L];
 #pragma unroll
-            for (int l = 0; l < L; ++l) {
+            for (int l = 0; l < L; ++l) b[l] = sh_bits[(l * G + g) * 32 + lane];
+#pragma unroll
+            for (int l = 0; l + 1 < L; ++l) hop[l] = b[l] & b[l + 1] & (b[l] >> 16);
+            // a path that switches layer as it arrives needs no second pass
+            const uint32_t from = changed_layers();
+            if (from & ~(1u << my_layer)) {
+              const uint32_t lowered = via_cascade(x, __ffs(from) - 1, 31 - __clz(from));
+              diff |= lowered;
+              dirty = __any_sync(0xFFFFFFFFu, dirty || lowered != 0u);
+            }
+          }
+          // ---- 2./3. row-local fixed point ----
+          // Each pass lowers at least one label, so the loop is finite; the
+          // cap only guards against a broken invariant (reported, never
+          // silent).
+          for (int pass = 0;; ++pass) {
+            if (pass == kMaxRowPasses) {
+              fault = true;
+              break;
+            }
+            // What reaches the chunk from outside, and the far cells' values.
+            // A chunk that is as a scan left it has nothing to scan: its
+            // labels are the far-cell values, and only a carry from another
+            // warp can lower them.
+            uint32_t inclE = v[C - 1], inclW = v[0];
+            uint32_t carryE = kLabelInf, carryW = kLabelInf;
+            if (dirty) {
+              // lane-local one-sided scans: value at the far cell with no carry
+              inclE = v[0];
+              inclW = v[C - 1];
+#pragma unroll
+              for (int j = 1; j < C; ++j) {
+                inclE = __viaddmin_u32(inclE, into[j], v[j]);
+                inclW = __viaddmin_u32(inclW, into[C - 1 - j], v[C - 1 - j]);
+              }
+              // segmented min scans over lanes of lane-offset values: a chunk's
+              // far-cell value reaches lane i through free chunks at C*orth each
+              inclE += to_last;
+              inclW += to_first;
+#pragma unroll
+              for (int sft = 1; sft < 32; sft <<= 1) {
+                inclE = min(inclE, shfl_up_to(inclE, sft, segE));
+                inclW = min(inclW, shfl_down_to(inclW, sft, segW));
+              }
+              inclE = min(inclE - to_last, kLabelInf);
+              inclW = min(inclW - to_first, kLabelInf);
+              // carry into the lane: the neighbour lane's far-cell value, or the
+              // warp carry when every chunk between is free
+              carryE = __shfl_up_sync(0xFFFFFFFFu, inclE, 1);
+              carryW = __shfl_down_sync(0xFFFFFFFFu, inclW, 1);
+              if (lane == 0) carryE = kLabelInf;
+              if (lane == 31) carryW = kLabelInf;
+            }
+            bool chain = dirty;
+            if constexpr (kMulti) {
+              // warp summaries: far-cell value without outside carry, and the
+              // cost to cross the whole warp (INF unless every chunk is free)
+              if (lane == 31) sh_sum[g].x = inclE;
+              if (lane == 0) {
+                sh_sum[g].y = free_lanes == 0xFFFFFFFFu ? 32u * stepC : kLabelInf;
+                sh_sum[g].z = inclW;
+              }
+              __syncthreads();
+              uint32_t warp_cE = kLabelInf, warp_cW = kLabelInf;
               for (int q = 0; q < g; ++q) {
-                warp_cE[l] = __viaddmin_u32(warp_cE[l], sh_sum[(q * L + l) * 4 + 1],
-                                            sh_sum[(q * L + l) * 4 + 0]);
+                const uint4 t = sh_sum[q];
+                warp_cE = __viaddmin_u32(warp_cE, t.y, t.x);
               }
               for (int q = G - 1; q > g; --q) {
-                warp_cW[l] = __viaddmin_u32(warp_cW[l], sh_sum[(q * L + l) * 4 + 1],
-                                            sh_sum[(q * L + l) * 4 + 2]);
+                const uint4 t = sh_sum[q];
+                warp_cW = __viaddmin_u32(warp_cW, t.y, t.z);
+              }
+              if (through_below) carryE = __viaddmin_u32(warp_cE, to_first, carryE);
+              if (through_above) carryW = __viaddmin_u32(warp_cW, to_last, carryW);
+              // a carry that lowers any cell lowers the first one it enters
+              const bool enters = (lane == 0 && __viaddmin_u32(carryE, into[0], v[0]) != v[0]) ||
+                                  (lane == 31 && __viaddmin_u32(carryW, into[C - 1], v[C - 1]) != v[C - 1]);
+              chain = __any_sync(0xFFFFFFFFu, enters) || dirty;
+            }
+            uint32_t scanned = 0;
+            if (chain) {
+              uint32_t e[C];
+#pragma unroll
+              for (int j = 0; j < C; ++j) {
+                carryE = __viaddmin_u32(carryE, into[j], v[j]);
+                e[j] = carryE;
+              }
+#pragma unroll
+              for (int j = C - 1; j >= 0; --j) {
+                carryW = __viaddmin_u32(carryW, into[j], v[j]);
+                const uint32_t t = min(e[j], carryW);
+                scanned |= t ^ v[j];
+                v[j] = t;
               }
             }
-          }
-#pragma unroll
-          for (int l = 0; l < L; ++l) {
-            // carry into the lane: the neighbour lane's far-cell value, or the
-            // warp carry when every chunk between is free
-            uint32_t carryE = __shfl_up_sync(0xFFFFFFFFu, inclE[l], 1);
-            uint32_t carryW = __shfl_down_sync(0xFFFFFFFFu, inclW[l], 1);
-            if (lane == 0) carryE = kLabelInf;
-            if (lane == 31) carryW = kLabelInf;
-            if (through_below[l]) carryE = __viaddmin_u32(warp_cE[l], static_cast<uint32_t>(lane) * stepC, carryE);
-            if (through_above[l]) carryW = __viaddmin_u32(warp_cW[l], static_cast<uint32_t>(31 - lane) * stepC, carryW);
-            uint32_t e[C];
-#pragma unroll
-            for (int j = 0; j < C; ++j) {
-              carryE = max(__viaddmin_u32(carryE, orth, v[l][j]), blk[l][j]);
-              e[j] = carryE;
+            diff |= scanned;
+            if constexpr (!kOne) {
+              parity ^= 1;
+              publish_flags(scanned != 0u);
+              // vote: labels that no scan lowered are at the cascade's fixed
+              // point already
+              if (!exchange(scanned != 0u)) break;
             }
-#pragma unroll
-            for (int j = C - 1; j >= 0; --j) {
-              carryW = max(__viaddmin_u32(carryW, orth, v[l][j]), blk[l][j]);
-              v[l][j] = min(e[j], carryW);
+            if constexpr (L > 1) {
+              const uint32_t from = changed_layers();
+              const uint32_t lowered =
+                  (from & ~(1u << my_layer)) ? via_cascade(x, __ffs(from) - 1, 31 - __clz(from)) : 0u;
+              diff |= lowered;
+              dirty = __any_sync(0xFFFFFFFFu, lowered != 0u);
+              parity ^= 1;
+              publish_flags(false);
+              if (__syncthreads_or(lowered != 0u) == 0) break;
+            } else {
+              break;
             }
           }
-          const uint32_t via_diff = via_cascade();
-          // group vote: did a via lower a label (another pass needed), and
-          // which layers changed since the row was loaded
-          uint32_t lane_flags = via_diff != 0u ? 1u : 0u;
-#pragma unroll
-          for (int l = 0; l < L; ++l) {
-            uint32_t diff = 0;
-#pragma unroll
-            for (int j = 0; j < C; ++j) diff |= v[l][j] ^ orig[l][j];
-            if (diff != 0u) lane_flags |= 2u | (1u << (8 + l));
+          if constexpr (kOne) {
+            row_layers = __any_sync(0xFFFFFFFFu, diff != 0u) ? 1u : 0u;
+          } else {
+            row_layers = __reduce_or_sync(0xFFFFFFFFu, lane < warps ? sh_flags[parity * warps + lane] & 0xFFu : 0u);
           }
-          uint32_t warp_flags = __reduce_or_sync(0xFFFFFFFFu, lane_flags);
-          if constexpr (G > 1) {
-            // this pass's row edges for the next step (final if the vote ends
-            // the row): buffer eb ^ 1 is read by no warp until the next step,
-            // and every read of it by the previous step came before this
-            // step's first barrier
-            if (lane == 0 || lane == 31) {
-#pragma unroll
-              for (int l = 0; l < L; ++l) {
-                sh_edges[(eb ^ 1) * kEdgeBuf + (g * L + l) * 2 + (lane == 0 ? 0 : 1)] =
-                    lane == 0 ? v[l][0] : v[l][C - 1];
-              }
-            }
-            if (lane == 0) sh_flags[parity * G + g] = warp_flags;
-            group_sync<G>(barrier_id);
-            warp_flags = 0;
-            for (int q = 0; q < G; ++q) warp_flags |= sh_flags[parity * G + q];
-            parity ^= 1;
-          }
-          row_flags = warp_flags;
-          if ((warp_flags & 1u) == 0u || L == 1) break;
         }
+        parity ^= 1;
         // ---- 4. write-back ----
-        if (row_flags & 2u) {
+        if (row_layers != 0u) {
           const bool materialise = (my == kNever);
-#pragma unroll
-          for (int l = 0; l < L; ++l) {
-            if (materialise || (row_flags & (1u << (8 + l)))) {
-              store_cells<C>(slab + l * layer_stride + static_cast<size_t>(r) * f.pitch, f.pitch,
-                             xs, v[l]);
-              ++stat_stores;
-            }
-          }
-          modified[r] = static_cast<int16_t>(k);  // same value from every thread
+          if (materialise || ((row_layers >> my_layer) & 1u)) store_cells<C>(row_at(r), f.pitch, xs, v);
+          stat_stores += materialise ? L : __popc(row_layers);
+          modified[r] = my = static_cast<int16_t>(k);  // same value from every thread
           any_change = true;
         }
         ++stat_rows;
 #pragma unroll
-        for (int l = 0; l < L; ++l) {
-#pragma unroll
-          for (int j = 0; j < C; ++j) prv[l][j] = v[l][j];
-          pf[l] = cf[l];
-        }
+        for (int j = 0; j < C; ++j) prv[j] = v[j];
+        pf = cf;
         have_prev = true;
         eb ^= 1;
-        // The step's last vote barrier published the edges; every thread
+        // The step's last vote published the edges; every thread
         // wrote modified[r] itself (the same value) and reads only its own
         // lane's cells of the slab.  A faulted row left the pass loop before
         // its vote, so it ends with a barrier of its own.
-        if (fault) group_sync<G>(barrier_id);
+        if (fault) net_sync<kOne>();
       }
       if (!any_change && k >= 2) {
         converged = true;
         break;
       }
     }
-    group_sync<G>(barrier_id);
+    net_sync<kOne>();
     if (fault) {
       completion = APGAR_B200_COMPLETION_REJECTED;
     } else if (cancelled) {
@@ -685,7 +752,7 @@ __global__ void __launch_bounds__(groups_per_block(G) * G * 32)
   }
 
   // ----------------------------- result + walk -----------------------------
-  if (g != 0) return;
+  if (warp != 0) return;
   apgar_b200_lattice_result res{};
   res.cost = APGAR_B200_UNREACHABLE;
   res.completion = completion;
@@ -695,8 +762,9 @@ __global__ void __launch_bounds__(groups_per_block(G) * G * 32)
   res.row_loads = stat_loads;
   auto label_at = [&](int l, int x, int y) -> uint32_t {
     const int r = f.transposed ? x : y, q = f.transposed ? y : x;
-    if (modified[r] == kNever) return kLabelInf;
-    return slab[static_cast<size_t>(l) * layer_stride + static_cast<size_t>(r) * f.pitch + q];
+    const uint32_t label = slab[static_cast<uint32_t>(l) * layer_stride +
+                                static_cast<uint32_t>(r) * static_cast<uint32_t>(f.pitch) + static_cast<uint32_t>(q)];
+    return modified[r] == kNever ? kLabelInf : label;  // a row never stored holds no labels
   };
   if (completion == APGAR_B200_COMPLETION_REACHED) {
     const uint32_t goal = label_at(g_layer, lgx, lgy);
@@ -728,29 +796,31 @@ __global__ void __launch_bounds__(groups_per_block(G) * G * 32)
             ok = true;
             break;
           }
-          bool cand = false;
+          // One round of independent loads per cell (0.45 us a cell with the
+          // bit planes read first and the labels after).  The labels tell
+          // what is free: at the fixed point every free cell next to a
+          // reached one is reached, so an unreached side cell is blocked.
           int pl = cl, px = cx, py = cy;
-          uint32_t pd = kLabelInf;
+          bool via_legal = true;
           if (lane < 8) {
             px = cx - kDxc[lane];
             py = cy - kDyc[lane];
-            bool legal = cell_free(lat, net, cl, px, py);
-            if (legal && (lane & 1)) {
-              legal = cell_free(lat, net, cl, cx, py) && cell_free(lat, net, cl, px, cy);
-            }
-            if (legal) {
-              pd = label_at(cl, px, py);
-              cand = pd < kLabelInf && pd + ((lane & 1) ? diag : orth) == here;
-            }
           } else if (lane == 8 || lane == 9) {
             pl = (lane == 8) ? cl - 1 : cl + 1;
-            const int lower = (lane == 8) ? cl - 1 : cl;
-            if (pl >= 0 && pl < Ln && cell_free(lat, net, pl, cx, cy) &&
-                via_bit_at(lat, net, lower, cx, cy)) {
-              pd = label_at(pl, cx, cy);
-              cand = pd < kLabelInf && pd + via == here;
-            }
+            if (pl >= 0 && pl < Ln) via_legal = via_bit_at(lat, net, min(pl, cl), cx, cy);
           }
+          uint32_t pd = kLabelInf;
+          if (lane < 10 && pl >= 0 && pl < Ln && px >= 0 && px < static_cast<int>(net.win_w) && py >= 0 &&
+              py < static_cast<int>(net.win_h)) {
+            pd = label_at(pl, px, py);
+          }
+          // the side cells of diagonal h are the neighbours at h - 1 and h + 1
+          const uint32_t side_a = __shfl_sync(0xFFFFFFFFu, pd, (lane + 7) & 7);
+          const uint32_t side_b = __shfl_sync(0xFFFFFFFFu, pd, (lane + 1) & 7);
+          const bool diagonal = lane < 8 && (lane & 1);
+          const uint32_t move = lane >= 8 ? via : diagonal ? diag : orth;
+          const bool legal = via_legal && (!diagonal || (side_a < kLabelInf && side_b < kLabelInf));
+          const bool cand = legal && pd < kLabelInf && pd + move == here;
           const unsigned ballot = __ballot_sync(0xFFFFFFFFu, cand);
           if (ballot == 0u) break;
           const int hsel = __ffs(ballot) - 1;
@@ -825,71 +895,90 @@ __global__ void pack_copy_kernel(apgar_b200_lattice_result* results, uint32_t co
   }
 }
 
-template <int L, int C, int G>
+template <int L, int C, int kMost>
 cudaError_t launch_one(const SweepLaunch& launch, int max_rows, cudaStream_t stream) {
-  constexpr int kGroups = groups_per_block(G);
-  const size_t smem = group_smem(L, G, max_rows).total * kGroups;
-  cudaError_t e = cudaFuncSetAttribute(lattice_sweep_kernel<L, C, G>,
+  const size_t smem = sweep_smem(L, C, launch.row_warps, max_rows).total;
+  cudaError_t e = cudaFuncSetAttribute(lattice_sweep_kernel<L, C, kMost>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  const unsigned grid = (launch.plan_count + kGroups - 1) / kGroups;
-  lattice_sweep_kernel<L, C, G><<<grid, kGroups * G * 32, smem, stream>>>(launch, max_rows);
+  lattice_sweep_kernel<L, C, kMost>
+      <<<launch.plan_count, L * launch.row_warps * 32, smem, stream>>>(launch, max_rows);
   return cudaGetLastError();
 }
 
-template <int L, int C>
-cudaError_t launch_layers(int G, const SweepLaunch& launch, int max_rows, cudaStream_t stream) {
-  // every group size 1..16: the host gives a net the fewest warps that
-  // cover its frame row
-  switch (G) {
-    case 1: return launch_one<L, C, 1>(launch, max_rows, stream);
-    case 2: return launch_one<L, C, 2>(launch, max_rows, stream);
-    case 3: return launch_one<L, C, 3>(launch, max_rows, stream);
-    case 4: return launch_one<L, C, 4>(launch, max_rows, stream);
-    case 5: return launch_one<L, C, 5>(launch, max_rows, stream);
-    case 6: return launch_one<L, C, 6>(launch, max_rows, stream);
-    case 7: return launch_one<L, C, 7>(launch, max_rows, stream);
-    case 8: return launch_one<L, C, 8>(launch, max_rows, stream);
-    case 9: return launch_one<L, C, 9>(launch, max_rows, stream);
-    case 10: return launch_one<L, C, 10>(launch, max_rows, stream);
-    case 11: return launch_one<L, C, 11>(launch, max_rows, stream);
-    case 12: return launch_one<L, C, 12>(launch, max_rows, stream);
-    case 13: return launch_one<L, C, 13>(launch, max_rows, stream);
-    case 14: return launch_one<L, C, 14>(launch, max_rows, stream);
-    case 15: return launch_one<L, C, 15>(launch, max_rows, stream);
-    case 16: return launch_one<L, C, 16>(launch, max_rows, stream);
+template <int L>
+cudaError_t launch_layers(int cells, const SweepLaunch& launch, int max_rows, cudaStream_t stream) {
+  constexpr int kWidest = 16 / L;  // warps of a row: 16 a net
+  const int warps = launch.row_warps;
+  if (warps < 1 || warps > kWidest) return cudaErrorInvalidValue;
+  switch (cells) {
+    case 4: return warps == 1 ? launch_one<L, 4, 1>(launch, max_rows, stream) : cudaErrorInvalidValue;
+    case 8:
+      return warps == 1 ? launch_one<L, 8, 1>(launch, max_rows, stream)
+                        : launch_one<L, 8, kWidest>(launch, max_rows, stream);
+    case 16:
+      return warps == 1 ? launch_one<L, 16, 1>(launch, max_rows, stream)
+                        : launch_one<L, 16, kWidest>(launch, max_rows, stream);
     default: return cudaErrorInvalidValue;
   }
 }
 
 }  // namespace
 
-// Cells per lane per layer for a layer count (L*C labels per lane).
-int lattice_cells_per_lane(int layers) {
-  switch (layers) {
-    case 1: return 16;
-    case 2: return 8;
-    case 3:
-    case 4: return 4;
-    default: return 2;
+// The widest row of a layer count.
+uint32_t lattice_sweep_widest(int layers) {
+  return 8192u / (layers <= 1 ? 1u : layers == 2 ? 2u : layers <= 4 ? 4u : 8u);
+}
+
+// Row width classes of a layer count, narrowest first: cells per lane and
+// warps side by side; false past the last class.  One warp a row up to 512
+// cells: a second one brings a barrier and a fold into every scan (4 layers of
+// 424 cells: 2.2 us a step with 4 x 1 warps of 16 cells a lane, 3.0 with
+// 4 x 4 of 4; 1 layer of 310: 0.88 us with one warp, 1.58 with three).  Past
+// 512, eight cells a lane while 16 warps a net suffice (4 layers of 601 cells:
+// 3.4 us a step with 4 x 3 warps of 8, 4.1 with 4 x 2 of 16: both are bound by
+// one SM's integer throughput), then sixteen.
+bool lattice_sweep_shape(int layers, int index, int* cells, int* warps) {
+  if (layers < 1 || index < 0) return false;
+  *warps = 1;
+  *cells = index < 2 ? 4 << index : 16;
+  if (index < 3) return true;
+  index -= 3;
+  const int most = min(8, 16 / layers);  // warps of a row of eight cells a lane
+  *cells = 8;
+  for (int w = 3; w <= most; ++w) {
+    if (index-- == 0) {
+      *warps = w;
+      return true;
+    }
   }
+  *cells = 16;
+  const int widest = static_cast<int>(lattice_sweep_widest(layers));
+  for (int w = most < 3 ? 2 : most / 2 + 1; 512 * (w - 1) < widest && w * layers <= 16; w += w < 6 ? 1 : 2) {
+    if (index-- == 0) {
+      *warps = w;
+      return true;
+    }
+  }
+  return false;
 }
 
-size_t lattice_sweep_smem_bytes(int layers, int warps_per_net, int max_rows) {
-  return group_smem(layers, warps_per_net, max_rows).total * groups_per_block(warps_per_net);
+size_t lattice_sweep_smem_bytes(int layers, int cells, int warps, int max_rows) {
+  return sweep_smem(layers, cells, warps, max_rows).total;
 }
 
-cudaError_t launch_lattice_sweep(int layers, int warps_per_net, const SweepLaunch& launch,
-                                 int max_rows, cudaStream_t stream) {
+cudaError_t launch_lattice_sweep(int layers, int cells, int warps, SweepLaunch launch, int max_rows,
+                                 cudaStream_t stream) {
   if (launch.plan_count == 0) return cudaSuccess;
+  launch.row_warps = warps;
   switch (layers) {
-    case 1: return launch_layers<1, 16>(warps_per_net, launch, max_rows, stream);
-    case 2: return launch_layers<2, 8>(warps_per_net, launch, max_rows, stream);
-    case 3: return launch_layers<3, 4>(warps_per_net, launch, max_rows, stream);
-    case 4: return launch_layers<4, 4>(warps_per_net, launch, max_rows, stream);
-    case 6: return launch_layers<6, 2>(warps_per_net, launch, max_rows, stream);
-    case 8: return launch_layers<8, 2>(warps_per_net, launch, max_rows, stream);
+    case 1: return launch_layers<1>(cells, launch, max_rows, stream);
+    case 2: return launch_layers<2>(cells, launch, max_rows, stream);
+    case 3: return launch_layers<3>(cells, launch, max_rows, stream);
+    case 4: return launch_layers<4>(cells, launch, max_rows, stream);
+    case 6: return launch_layers<6>(cells, launch, max_rows, stream);
+    case 8: return launch_layers<8>(cells, launch, max_rows, stream);
     default: return cudaErrorInvalidValue;
   }
 }
