@@ -201,7 +201,9 @@ def frontier_bytes(lat, nets, results):
     GPU's own work: the distinct cells the A* restatement of RouteWithCpuAStar
     expands per net (the cell expansions an exact search needs) times the
     bytes of an expansion, plus 4 B per emitted path cell.  Returns (those
-    bytes, the bytes of the GPU's own expansions, re-expansions included)."""
+    bytes, the same bytes for each of the GPU's own row_steps: expansions of the
+    cell form, steps over lines of 32 cells in shared memory of the tile form,
+    so there a measure of its work and not of its traffic)."""
     import oracle
 
     _, _, cells = oracle.astar_batch(lat, nets, counts=True)
