@@ -336,7 +336,7 @@ struct Swept {
 };
 
 // One directional sweep over the lines of a unit, in the order of the line
-// index i (0..31): cell + i * kStride is this lane's cell of line i, bit i of
+// index i (0..31): cell + i * stride is this lane's cell of line i, bit i of
 // `blocked` set when it is not free.  Chunks of eight lines run when `need`
 // has a line in them or the line before them changed; the rim is not a source
 // here.  A diagonal move needs four free cells: its source (a blocked cell
@@ -345,21 +345,22 @@ struct Swept {
 // its label over.  The outermost lanes get their own label back from a
 // shuffle; p + diag is then no better than the straight p + orth, unless a
 // diagonal is cheaper than a straight move (kCheapDiagonal).  Priced, every
-// move into a cell also costs price + i * kPriceStride.  In a corridor
+// move into a cell also costs price[i * price_stride].  In a corridor
 // (kCorr), `blocked` has the cells outside it too and `sides`, for the
 // diagonals' side cells, only the blocked ones; else both are the same.
-template <int kStride, int kPriceStride, bool kCheapDiagonal, bool kPriced, bool kCorr>
-__device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* price, uint32_t blocked, uint32_t sides, uint32_t need, uint32_t orth,
+template <bool kCheapDiagonal, bool kPriced, bool kCorr>
+__device__ __forceinline__ Swept sweep_lines(uint32_t* cell, int stride, const uint32_t* price, int price_stride,
+                                             uint32_t blocked, uint32_t sides, uint32_t need, uint32_t orth,
                                              uint32_t diag, int lane, uint32_t& steps) {
   Swept out{0u, 0u, 0u};
   uint32_t pair = blocked | (sides << 1);
 #pragma unroll 1
   for (int c = 0; c < 32; c += 8) {
     if (((need >> c) & 0xFFu) != 0u) {
-      uint32_t p = c == 0 ? kTileInf : cell[-kStride];
+      uint32_t p = c == 0 ? kTileInf : cell[-stride];
       uint32_t v[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = cell[k * kStride];
+      for (int k = 0; k < 8; ++k) v[k] = cell[k * stride];
       uint32_t diff = 0, first = 0, last = 0;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
@@ -373,12 +374,12 @@ __device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* pri
         uint32_t t;
         if constexpr (kPriced) {
           t = __viaddmin_u32(unless(pair, k, min(before, after)), diag, straight + orth);
-          t = __viaddmin_u32(min(t, kTileInf), price[k * kPriceStride], v[k]);
+          t = __viaddmin_u32(min(t, kTileInf), price[k * price_stride], v[k]);
         } else {
           t = __viaddmin_u32(straight, orth, v[k]);
           t = __viaddmin_u32(unless(pair, k, min(before, after)), diag, t);
         }
-        cell[k * kStride] = t;
+        cell[k * stride] = t;
         diff |= t ^ v[k];
         if (k == 0) first = diff;
         if (k == 7) last = t ^ v[k];
@@ -393,8 +394,8 @@ __device__ __forceinline__ Swept sweep_lines(uint32_t* cell, const uint32_t* pri
       need |= last_changed ? (0x80u << c) << 1 : 0u;
       steps += 8;
     }
-    cell += 8 * kStride;
-    price += 8 * kPriceStride;
+    cell += 8 * stride;
+    price += 8 * price_stride;
     blocked >>= 8;
     sides >>= 8;
     pair >>= 8;
@@ -963,46 +964,49 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
       if (lane == 0) atomicMax(&st->stop, 2u);
       break;
     }
-    __syncwarp();
-    if (down != 0u) {
-      const Swept w = sweep_lines<kPitch, kPricePitch, kCheapDiagonal, kPriced, kCorr>(first_row, prices + lane, ~m.col_free, ~col_open, down, orth, diag, lane, steps);
-      down = 0u;
-      up |= w.back;
-      right |= w.lanes << 1;
-      left |= w.lanes >> 1;
-      rows |= w.lines;
-      cols |= w.lanes;
-    }
-    if (up != 0u) {
-      const Swept w = sweep_lines<-kPitch, -kPricePitch, kCheapDiagonal, kPriced, kCorr>(
-          first_row + 31 * kPitch, prices + 31 * kPricePitch + lane, __brev(~m.col_free), __brev(~col_open), __brev(up), orth, diag, lane, steps);
-      up = 0u;
-      down |= __brev(w.back);
-      right |= w.lanes << 1;
-      left |= w.lanes >> 1;
-      rows |= __brev(w.lines);
-      cols |= w.lanes;
-    }
-    __syncwarp();
-    if (right != 0u) {
-      const Swept w = sweep_lines<1, 1, kCheapDiagonal, kPriced, kCorr>(first_col, prices + lane * kPricePitch, ~m.row_free, ~row_open, right,
-                                                                orth, diag, lane, steps);
-      right = 0u;
-      left |= w.back;
-      down |= w.lanes << 1;
-      up |= w.lanes >> 1;
-      cols |= w.lines;
-      rows |= w.lanes;
-    }
-    if (left != 0u) {
-      const Swept w = sweep_lines<-1, -1, kCheapDiagonal, kPriced, kCorr>(
-          first_col + 31, prices + lane * kPricePitch + 31, __brev(~m.row_free), __brev(~row_open), __brev(left), orth, diag, lane, steps);
-      left = 0u;
-      right |= __brev(w.back);
-      down |= w.lanes << 1;
-      up |= w.lanes >> 1;
-      cols |= __brev(w.lines);
-      rows |= w.lanes;
+    // Down, up, right, left: one copy of the sweep's code for the four, with
+    // the stride in a register, so that it stays in the instruction cache
+    // while an SM's warps are at different places of a unit (four copies:
+    // waits for instructions were the top stall, 3.2 cycles an instruction;
+    // medium batch 11.9 ms, 10.7 with one, priced rounds 50 ms and 44).
+#pragma unroll 1
+    for (int dir = 0; dir < 4; ++dir) {
+      const bool across = dir >= 2, reverse = (dir & 1) != 0;
+      uint32_t need = across ? (reverse ? left : right) : (reverse ? up : down);
+      if (need == 0u) continue;
+      __syncwarp();
+      uint32_t blocked = ~(across ? m.row_free : m.col_free), sides = ~(across ? row_open : col_open);
+      uint32_t* cell = across ? first_col : first_row;
+      const uint32_t* price = across ? prices + lane * kPricePitch : prices + lane;
+      int stride = across ? 1 : kPitch, price_stride = across ? 1 : kPricePitch;
+      if (reverse) {
+        need = __brev(need);
+        blocked = __brev(blocked);
+        sides = __brev(sides);
+        cell += 31 * stride;
+        price += 31 * price_stride;
+        stride = -stride;
+        price_stride = -price_stride;
+      }
+      const Swept w = sweep_lines<kCheapDiagonal, kPriced, kCorr>(cell, stride, price, price_stride, blocked, sides, need,
+                                                                  orth, diag, lane, steps);
+      const uint32_t back = reverse ? __brev(w.back) : w.back, lines = reverse ? __brev(w.lines) : w.lines;
+      const uint32_t after = w.lanes << 1, before = w.lanes >> 1;
+      if (across) {
+        right = reverse ? right | back : 0u;
+        left = reverse ? 0u : left | back;
+        down |= after;
+        up |= before;
+        cols |= lines;
+        rows |= w.lanes;
+      } else {
+        down = reverse ? down | back : 0u;
+        up = reverse ? 0u : up | back;
+        right |= after;
+        left |= before;
+        rows |= lines;
+        cols |= w.lanes;
+      }
     }
   }
   __syncwarp();
