@@ -311,7 +311,7 @@ def round0_sample(args, lat, segs, dev):
         "roofline": {
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_kind": peak_kind, "traffic": None,
-            "kernel": f"lattice_frontier_kernel, round 0 (zero prices) of the first {n} segments",
+            "kernel": f"lattice_tiles_kernel, round 0 (zero prices) of the first {n} segments",
             "bytes_alg_per_launch": fbytes,
             "bytes_alg_source": "oracle A* expanded cells x 92 B + 4 B per path cell",
         },
@@ -881,7 +881,7 @@ def main():
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_kind": peak_kind,
                 "traffic": (traffic or {}).get("frontier_dram_bytes_per_step"),
-                "kernel": "lattice_frontier_kernel (all width classes of one execution)",
+                "kernel": "lattice_tiles_kernel (all width classes of one execution)",
                 "bytes_alg_per_step": fbytes,
                 "bytes_alg_source": "oracle A* expanded cells x 92 B + 4 B per path cell",
                 "gpu_expansion_bytes_per_step": gpu_fbytes,
