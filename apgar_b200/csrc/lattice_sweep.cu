@@ -913,7 +913,11 @@ cudaError_t launch_layers(int cells, const SweepLaunch& launch, int max_rows, cu
   const int warps = launch.row_warps;
   if (warps < 1 || warps > kWidest) return cudaErrorInvalidValue;
   switch (cells) {
-    case 4: return warps == 1 ? launch_one<L, 4, 1>(launch, max_rows, stream) : cudaErrorInvalidValue;
+    case 4:
+      if constexpr (L == 2) {
+        if (warps > 1) return launch_one<L, 4, kWidest>(launch, max_rows, stream);
+      }
+      return warps == 1 ? launch_one<L, 4, 1>(launch, max_rows, stream) : cudaErrorInvalidValue;
     case 8:
       return warps == 1 ? launch_one<L, 8, 1>(launch, max_rows, stream)
                         : launch_one<L, 8, kWidest>(launch, max_rows, stream);
@@ -938,7 +942,9 @@ uint32_t lattice_sweep_widest(int layers) {
 // 4 x 4 of 4; 1 layer of 310: 0.88 us with one warp, 1.58 with three).  Past
 // 512, eight cells a lane while 16 warps a net suffice (4 layers of 601 cells:
 // 3.4 us a step with 4 x 3 warps of 8, 4.1 with 4 x 2 of 16: both are bound by
-// one SM's integer throughput), then sixteen.
+// one SM's integer throughput), then sixteen; two layers leave room for four
+// cells a lane up to 1,024 (200 nets of 2 x 1024^2, rows up to 718: 4.14 ms with
+// eight cells a lane, 3.82 with four; 1,000 nets, rows up to 651: 5.8 and 4.9).
 bool lattice_sweep_shape(int layers, int index, int* cells, int* warps) {
   if (layers < 1 || index < 0) return false;
   *warps = 1;
@@ -946,8 +952,17 @@ bool lattice_sweep_shape(int layers, int index, int* cells, int* warps) {
   if (index < 3) return true;
   index -= 3;
   const int most = min(8, 16 / layers);  // warps of a row of eight cells a lane
+  if (layers == 2) {
+    *cells = 4;
+    for (int w = 5; w <= 8; ++w) {
+      if (index-- == 0) {
+        *warps = w;
+        return true;
+      }
+    }
+  }
   *cells = 8;
-  for (int w = 3; w <= most; ++w) {
+  for (int w = layers == 2 ? 5 : 3; w <= most; ++w) {
     if (index-- == 0) {
       *warps = w;
       return true;
