@@ -548,9 +548,26 @@ __device__ __noinline__ bool lift_corridor(int tx, int ty, Space ws, TileNetStat
     st->far_count[0] = st->far_count[1] = 0u;
     atomicAdd(&st->active, 1u);  // this warp, until every unit is queued
   }
+  const Win shape{0, 0, tx * 32, ty * 32, 0, 0, 0, tx, ty};
+  const int plane = tx * ty, layers = static_cast<int>(units) / plane;
+  const auto unit_at = [&](uint32_t i) {
+    const int l = static_cast<int>(i) / plane, rest = static_cast<int>(i) - l * plane, y = rest / tx;
+    return pack_unit(l, y, rest - y * tx);
+  };
   for (uint32_t i = lane; i < units; i += 32) {
+    // (kTouched stays as it is, so a neighbour that is already rewritten reads the same)
     const bool touched = (__ldcg(ws.flags + i) & kTouched) != 0u;
-    __stcg(ws.flags + i, touched ? kTouched | kSourceBits | kWhole : 0u);
+    uint32_t sides = 0;
+    if (touched) {  // a side bit means a neighbour with labels
+      const uint32_t exist = neighbours(shape, unpack_unit(shape, unit_at(i)), layers);
+#pragma unroll 1
+      for (int k = 0; k < 10; ++k) {
+        if (((exist >> k) & 1u) != 0u && (__ldcg(ws.flags + static_cast<int>(i) + neighbour_offset(shape, k)) & kTouched) != 0u) {
+          sides |= 1u << k;
+        }
+      }
+    }
+    __stcg(ws.flags + i, touched ? kTouched | kWhole | sides : 0u);
     __stcg(ws.pend + i, touched ? 0u : kNoKey);
   }
   __threadfence();
@@ -563,8 +580,7 @@ __device__ __noinline__ bool lift_corridor(int tx, int ty, Space ws, TileNetStat
     if (lane == 0 && lanes != 0u) atomicAdd(&st->active, __popc(lanes));
     __threadfence();
     __syncwarp();
-    const int plane = tx * ty, l = static_cast<int>(i) / plane, rest = static_cast<int>(i) - l * plane, y = rest / tx;
-    push_units(st, ws, take, pack_unit(l, y, rest - y * tx), lane);
+    push_units(st, ws, take, unit_at(i), lane);
   }
   uint32_t left = 1;
   if (lane == 0) {
@@ -874,7 +890,8 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
     }
   }
   const uint32_t exist = neighbours(win, u, lat.layers);
-  const uint32_t touched = touched_neighbours(ws, part, u.id, exist, lane);
+  // (a side bit also says that the neighbour has labels: its kTouched may land later)
+  const uint32_t touched = touched_neighbours(ws, part, u.id, exist, lane) | (flags & exist);
   load_unit(ws.labels, win, u, touched, own, tile, lane);
   bool high = false;  // a price or label near the 32-bit limit
   if constexpr (kPriced) high = load_prices(p, win, ws, u, m.col_free, prices, lane);
@@ -1157,15 +1174,26 @@ __device__ __forceinline__ void relax_unit(const TileLaunch& p, const Win& win, 
   if constexpr (kPriced) {
     if (__any_sync(kFull, high) && lane == 0) atomicMax(&st->stop, 3u);
   }
-  __threadfence();  // labels before the flags and keys that announce them
+  // What lands before what: the labels before the side bits and kTouched that
+  // announce them, these before the neighbours' keys and before this unit's
+  // own key is free again (in `finish`).  kTouched and the side bits may land
+  // in either order, so a warp that takes a neighbour reads this unit's labels
+  // on its side bit alone.
   __syncwarp();
-  if (!own && lane == 0) atomicOr(ws.flags + u.id, kTouched);
+  __threadfence();
+  __syncwarp();
   const uint32_t limit = peek(&st->limit), thr = peek(&st->thr);
-  bool near = false, far = false;
-  if (out_key <= limit) {  // lanes 0..9 only: the others hold kNoKey
-    const int nb = u.id + part.offset;
-    atomicOr(ws.flags + nb, part.seen);
+  const bool lowers = out_key <= limit;  // lanes 0..9 only: the others hold kNoKey
+  const int nb = u.id + part.offset;
+  if (!own && lane == 0) atomicOr(ws.flags + u.id, kTouched);
+  if (lowers) atomicOr(ws.flags + nb, part.seen);
+  if (!own || __any_sync(kFull, lowers)) {
+    __syncwarp();
     __threadfence();
+    __syncwarp();
+  }
+  bool near = false, far = false;
+  if (lowers) {
     const uint32_t old = atomicMin(ws.pend + nb, out_key);
     if (old == kNoKey) {
       near = out_key < thr;
