@@ -150,7 +150,7 @@ struct TileNetState {
   uint32_t far_par;       // the far list in use
   uint32_t far_count[2];
   uint32_t goal;          // least goal label so far
-  uint32_t stop;          // 1 cancelled, 2 a broken invariant
+  uint32_t stop;          // 1 cancelled, 2 a broken invariant, 3 handed over to the cell form
   uint32_t steps, units, levels;
   uint32_t slot;          // workspace slot (slot mode)
   uint32_t guests;        // warps that help the owner
@@ -192,7 +192,9 @@ struct TileLaunch {
   unsigned int* finished;  // nets that are done
   // prices, kept routes and rip-up pricing, as in FrontierLaunch; own_bits is
   // one bit per label word of the pool.  A net whose prices or labels come
-  // near the 32-bit limit goes to `redo` (the cell form then decides it).
+  // near the 32-bit limit goes to `redo` (the cell form then decides it): the
+  // team class's nets from its start on, the others' after room for all of
+  // those, counted apart in redo_count[0] and [1].
   const uint32_t* cell_cost;
   const uint32_t* cell_cost_own;
   uint32_t* own_bits;

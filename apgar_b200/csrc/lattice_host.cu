@@ -148,12 +148,10 @@ struct PlanObject {
   DeviceBuffer<NetPlan> tile_plans;
   DeviceBuffer<uint32_t> tile_pool;
   uint32_t tile_warps = 0;  // warps of a launch
-  // FRONTIER, tile form with prices: nets whose prices or labels come near the
-  // 32-bit limit, and the slots (in words and lists) of their cell-form search
-  DeviceBuffer<NetPlan> redo;
-  DeviceBuffer<uint32_t> redo_own;
-  uint32_t redo_slots = 0;
-  uint64_t redo_cells = 0;
+  // FRONTIER, tile form with prices: the cell form's classes for nets that the
+  // tile search hands over (see plan_tiles), the CTA-wide class's own first
+  ClassRange redo[2];
+  bool one_shot = false;  // never gets prices
   std::vector<apgar_b200_lattice_net> host_nets;  // FRONTIER: the batch, as planned
   std::vector<uint32_t> admitted;                 // FRONTIER: its admitted nets
   const uint32_t* cell_cost = nullptr;  // caller-owned device prices (frontier only)
@@ -181,8 +179,8 @@ struct PlanObject {
   DeviceBuffer<unsigned long long> words;  // FRONTIER: label | ~round stamp per cell
   DeviceBuffer<uint32_t> lists;            // FRONTIER: three queue lists per net
   // [0] arena cursor, [1] packed total, [2 + class] work-stealing cursors,
-  // [2 + kClassCount] the tile form's finished nets, nets handed over and their
-  // cursor, then its net states
+  // [2 + kClassCount] the tile form's finished nets, nets handed over (a 32-bit
+  // count for each of `redo`) and their cursors (likewise), then its net states
   DeviceBuffer<unsigned long long> counters;
   uint64_t label_cells = 0;
   uint64_t arena_capacity = 0;
@@ -210,7 +208,7 @@ struct PlanObject {
   uint64_t workspace_bytes() const {
     return nets.bytes() + plans.bytes() + dist_pool.bytes() + results.bytes() + arena.bytes() +
            paths.bytes() + counters.bytes() + words.bytes() + lists.bytes() + tile_plans.bytes() +
-           tile_pool.bytes() + redo.bytes() + redo_own.bytes();
+           tile_pool.bytes();
   }
 };
 
@@ -342,8 +340,8 @@ std::vector<std::vector<uint32_t>> frontier_members(const PlanObject* plan, uint
 // Slot workspace within its budget: the class with the largest slot gives up
 // an eighth of its slots until the total fits (every class keeps at least
 // one; fewer slots only means fewer of its nets in flight).
-template <typename SlotBytes>
-void fit_slots(std::vector<ClassRange>& classes, uint64_t budget, SlotBytes slot_bytes) {
+template <typename Classes, typename SlotBytes>
+void fit_slots(Classes& classes, uint64_t budget, SlotBytes slot_bytes) {
   const auto total = [&]() {
     uint64_t t = 0;
     for (const ClassRange& c : classes) t += c.slots * slot_bytes(c);
@@ -362,8 +360,8 @@ void fit_slots(std::vector<ClassRange>& classes, uint64_t budget, SlotBytes slot
 uint64_t per_net_budget() { return budget_from_env("APGAR_B200_FRONTIER_PER_NET_BYTES", kPerNetFrontierBytes); }
 uint64_t slot_budget() { return budget_from_env("APGAR_B200_FRONTIER_SLOT_BYTES", kSlotFrontierBytes); }
 
-int upload_plans(DeviceBuffer<NetPlan>& dst, const std::vector<NetPlan>& plans) {
-  APGAR_B200_CUDA("cudaMalloc(plans)", dst.ensure(std::max<size_t>(plans.size(), 1)));
+int upload_plans(DeviceBuffer<NetPlan>& dst, const std::vector<NetPlan>& plans, size_t extra = 0) {
+  APGAR_B200_CUDA("cudaMalloc(plans)", dst.ensure(std::max<size_t>(plans.size() + extra, 1)));
   if (!plans.empty()) {
     APGAR_B200_CUDA("cudaMemcpy(plans)", cudaMemcpy(dst.get(), plans.data(), plans.size() * sizeof(NetPlan),
                                                     cudaMemcpyHostToDevice));
@@ -476,50 +474,48 @@ int plan_tiles(PlanObject* plan) {
     }
   }
   plan->label_cells = words;
-  APGAR_B200_CUDA("cudaMalloc(tile workspace)", plan->tile_pool.ensure(std::max<uint64_t>(words, 32)));
-  return upload_plans(plan->tile_plans, plans);
-}
-
-// Workspace budget of the nets that a priced tile search hands over.
-constexpr uint64_t kRedoBytes = 256ull << 20;
-
-int use_cells(PlanObject* plan);
-
-// Prices on a tile plan: a place for the nets whose prices or labels come
-// near the 32-bit limit, which the cell form then decides.  (Its rejections
-// depend on the level width, so one width for all nets is needed.)
-int use_prices(PlanObject* plan) {
-  if (!plan->tiles || plan->redo_slots != 0) return APGAR_B200_OK;
-  if (plan->wide_bucket_width != plan->bucket_width) return use_cells(plan);
-  uint64_t cells = 0;
-  for (uint32_t i : plan->admitted) {
-    const apgar_b200_lattice_net& n = plan->host_nets[i];
-    cells = std::max(cells, static_cast<uint64_t>(plan->lattice->view.layers) * n.win_w * n.win_h);
+  // Prices may come and go at any time, under capture too, so everything that
+  // a priced execution needs is here from the start.  A net whose prices or
+  // labels come near the 32-bit limit is handed over to the cell form, which
+  // decides it with its class's level width (its rejections depend on that).
+  // That search runs after the tile search, so its workspace (20 B a window
+  // cell and slot) takes the tile form's place in the pool; a pool with less
+  // than one slot for each class is larger for it.
+  uint32_t extra = 0;  // plan records of handed over nets
+  for (ClassRange& r : plan->redo) r = ClassRange{};
+  if (!plan->one_shot) {
+    extra = static_cast<uint32_t>(plans.size());
+    uint32_t begin = 0;
+    for (int k = 1; k >= 0; --k) {  // the CTA-wide class, the others
+      ClassRange& r = plan->redo[1 - k];
+      for (int m = k == 1 ? 4 : 0; m < (k == 1 ? 5 : 4); ++m) {
+        for (uint32_t i : members[m]) {
+          const apgar_b200_lattice_net& n = plan->host_nets[i];
+          r.slab_cells = std::max(r.slab_cells, static_cast<uint64_t>(v.layers) * n.win_w * n.win_h);
+        }
+        r.count += static_cast<uint32_t>(members[m].size());
+      }
+      r.begin = begin;
+      begin += r.count;
+      r.warps_per_net = k == 1 ? 16 : 8;
+      r.slots = std::min<uint32_t>(r.count, static_cast<uint32_t>(plan->sm_count) * (k == 1 ? 1u : 2u));
+      r.slab_cells = ((r.slab_cells + 127ull) & ~127ull) + 512ull;
+      r.list_cap = static_cast<uint32_t>(r.slab_cells);
+    }
+    fit_slots(plan->redo, words * 4ull, [](const ClassRange& c) { return c.slab_cells * 20ull; });
+    uint64_t at = 0;  // in 32-bit words of the pool: label words, then lists
+    for (ClassRange& r : plan->redo) {
+      r.words_offset = at;
+      at += r.slots * r.slab_cells * 2ull;
+    }
+    for (ClassRange& r : plan->redo) {
+      r.lists_offset = at;
+      at += r.slots * r.slab_cells * 3ull;
+    }
+    words = std::max(words, at);
   }
-  cells = ((cells + 127ull) & ~127ull) + 512ull;
-  const uint64_t slots = std::min<uint64_t>(std::max<uint64_t>(kRedoBytes / (cells * 20ull), 1),
-                                            std::max<size_t>(plan->admitted.size(), 1));
-  plan->redo_cells = cells;
-  APGAR_B200_CUDA("cudaMalloc(handed over nets)", plan->redo.ensure(std::max<size_t>(plan->admitted.size(), 1)));
-  plan->redo_slots = static_cast<uint32_t>(std::min<uint64_t>(slots, static_cast<uint64_t>(plan->sm_count)));
-  APGAR_B200_CUDA("cudaMalloc(label words)", plan->words.ensure(plan->redo_slots * cells));
-  APGAR_B200_CUDA("cudaMalloc(queue lists)", plan->lists.ensure(plan->redo_slots * 3ull * cells));
-  APGAR_B200_CUDA("cudaMalloc(own-route bits)", plan->redo_own.ensure(plan->redo_slots * cells / 32 + 1));
-  return APGAR_B200_OK;
-}
-
-// Moves a tile plan over to the cell form for good (and gives the tile form's
-// workspace back first).
-int use_cells(PlanObject* plan) {
-  if (!plan->tiles) return APGAR_B200_OK;
-  APGAR_B200_CUDA("cudaDeviceSynchronize(tile form)", cudaDeviceSynchronize());
-  plan->tile_pool.reset();
-  plan->tile_plans.reset();
-  plan->redo.reset();
-  plan->redo_own.reset();
-  plan->redo_slots = 0;
-  plan->tiles = false;
-  return plan_cells(plan);
+  APGAR_B200_CUDA("cudaMalloc(tile workspace)", plan->tile_pool.ensure(std::max<uint64_t>(words, 32)));
+  return upload_plans(plan->tile_plans, plans, extra);
 }
 
 // Builds (or rebuilds into existing buffers) a plan for `nets`.
@@ -556,7 +552,6 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
   uint64_t largest = 0;  // FRONTIER: cells of the largest window
   plan->admitted.clear();
   plan->tiles = false;
-  plan->redo_slots = 0;
   plan->classes.clear();
   std::vector<apgar_b200_lattice_result> init(count);
   std::memset(init.data(), 0, init.size() * sizeof(apgar_b200_lattice_result));
@@ -750,21 +745,32 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
     t.prev_paths = plan->prev_paths;
     t.corridor = fbase.corridor;
     t.corridor_status = fbase.corridor_status;
-    t.redo = plan->redo.get();
+    t.redo = plan->tile_plans.get() + t.total;
     t.redo_count = reinterpret_cast<uint32_t*>(plan->counters.get() + 2 + kClassCount + 1);
     APGAR_B200_CUDA("lattice tiles launch", launch_lattice_tiles(t, plan->sm_count, stream));
     if (plan->cell_cost != nullptr) {
       FrontierClasses fc{};
-      FrontierLaunch& fl = fc.c[4];
-      fl = fbase;
-      fl.plans = plan->redo.get();
-      fl.plan_count_dev = t.redo_count;
-      fl.skip = nullptr;
-      fl.slab_cells = plan->redo_cells;
-      fl.list_cap = static_cast<uint32_t>(plan->redo_cells);
-      fl.slots = plan->redo_slots;
-      fl.own_bits = plan->cell_cost_own != nullptr ? plan->redo_own.get() : nullptr;
-      fl.next_plan = reinterpret_cast<unsigned int*>(plan->counters.get() + 2 + kClassCount + 2);
+      auto* const cursors = reinterpret_cast<unsigned int*>(plan->counters.get() + 2 + kClassCount + 2);
+      uint32_t* own_bits = plan->own_bits;
+      for (int k = 0; k < 2; ++k) {
+        const ClassRange& r = plan->redo[k];
+        if (r.count == 0) continue;
+        FrontierLaunch& fl = fc.c[k == 0 ? 4 : 3];
+        fl = fbase;
+        fl.plans = t.redo + r.begin;
+        fl.plan_count_dev = t.redo_count + k;
+        fl.skip = nullptr;
+        fl.words = reinterpret_cast<unsigned long long*>(plan->tile_pool.get() + r.words_offset);
+        fl.lists = plan->tile_pool.get() + r.lists_offset;
+        fl.slab_cells = r.slab_cells;
+        fl.list_cap = r.list_cap;
+        fl.slots = r.slots;
+        if (k == 0) fl.bucket_width = plan->wide_bucket_width;
+        // (a bit per label word of the pool: room for every slot's cells)
+        fl.own_bits = own_bits;
+        if (own_bits != nullptr) own_bits += r.slots * r.slab_cells / 32u;
+        fl.next_plan = cursors + k;
+      }
       APGAR_B200_CUDA("lattice frontier launch", launch_lattice_frontier(fc, plan->sm_count, stream));
     }
     APGAR_B200_CUDA("lattice pack launch",
@@ -1026,10 +1032,6 @@ extern "C" int apgar_b200_lattice_plan_set_cell_costs(void* plan, const uint32_t
   if (cell_costs != nullptr && p->generator != APGAR_B200_LATTICE_FRONTIER) {
     return set_error(APGAR_B200_UNSUPPORTED, "per-cell prices need the frontier generator");
   }
-  if (cell_costs != nullptr) {
-    if (int rc = check_device(p->device); rc != APGAR_B200_OK) return rc;
-    if (int rc = use_prices(p); rc != APGAR_B200_OK) return rc;
-  }
   p->cell_cost = cell_costs;
   clear_error();
   return APGAR_B200_OK;
@@ -1195,6 +1197,7 @@ int route_impl(void* lattice, const apgar_b200_lattice_net* nets, uint32_t count
     std::scoped_lock lock(lat->route_mutex);
     if (lat->route_plan == nullptr) lat->route_plan = std::make_unique<PlanObject>();
     PlanObject* plan = lat->route_plan.get();
+    plan->one_shot = true;
     if (int rc = build_plan(lat, nets, count, o.max_iterations, plan, o.generator, o.bucket_width,
                             o.chain, o.class_bounds, o.wide_bucket_width, o.wide_chain);
         rc != APGAR_B200_OK) {
@@ -1642,7 +1645,6 @@ struct NegotiationObject {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   uint32_t graph_rounds = 0;
-  bool form_tiles = false;  // the plan's form when own_bits was sized
   // split-round steps: the next (round, phase) a step may run
   uint32_t step_round = 0, step_phase = 0;
 
@@ -1664,25 +1666,6 @@ struct NegotiationObject {
     }
   }
 };
-
-// One own-route bit per label word of the plan's form (which set_corridors
-// may have changed since; a captured run is then captured again).
-int ensure_own_bits(NegotiationObject* n) {
-  const PlanObject* p = n->plan;
-  const size_t words = (p->tiles ? p->tile_pool.count() : p->words.count()) / 32 + 1;
-  if (words > n->own_bits.count()) {
-    APGAR_B200_CUDA("cudaDeviceSynchronize(own-route bits)", cudaDeviceSynchronize());
-    APGAR_B200_CUDA("cudaMalloc(own-route bits)", n->own_bits.ensure(words));
-  }
-  if (n->form_tiles != p->tiles && n->exec != nullptr) {
-    cudaGraphExecDestroy(n->exec);
-    cudaGraphDestroy(n->graph);
-    n->exec = nullptr;
-    n->graph = nullptr;
-  }
-  n->form_tiles = p->tiles;
-  return APGAR_B200_OK;
-}
 
 bool checked_factor(const apgar_b200_price_policy& p, uint64_t epoch, uint64_t* out) {
   const unsigned __int128 f =
@@ -1796,7 +1779,6 @@ extern "C" int apgar_b200_negotiation_create(void* plan, const apgar_b200_price_
     return set_error(APGAR_B200_UNSUPPORTED, "lattice has more cells than a price pass indexes");
   }
   try {
-    if (int rc = use_prices(p); rc != APGAR_B200_OK) return rc;
     auto n = std::make_unique<NegotiationObject>();
     n->plan = p;
     n->policy = *policy;
@@ -1804,7 +1786,8 @@ extern "C" int apgar_b200_negotiation_create(void* plan, const apgar_b200_price_
     APGAR_B200_CUDA("cudaMalloc(usage)", n->usage.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(cell costs)", n->cell_cost.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(own-route cell costs)", n->cell_cost_own.ensure(cells));
-    if (int rc = ensure_own_bits(n.get()); rc != APGAR_B200_OK) return rc;
+    const size_t label_words = p->tiles ? p->tile_pool.count() : p->words.count();
+    APGAR_B200_CUDA("cudaMalloc(own-route bits)", n->own_bits.ensure(label_words / 32 + 1));
     APGAR_B200_CUDA("cudaMalloc(history)", n->history.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(previous results)", n->prev_results.ensure(std::max<uint32_t>(p->count, 1)));
     APGAR_B200_CUDA("cudaMalloc(previous paths)", n->prev_paths.ensure(std::max<uint64_t>(p->arena_capacity, 1)));
@@ -1836,7 +1819,6 @@ extern "C" int apgar_b200_negotiation_run_ex(void* negotiation, uint32_t rounds,
     APGAR_B200_CUDA("cudaMalloc(round stats)", n->stats.ensure(2ull * rounds));
     n->rounds_capacity = rounds;
   }
-  if (int rc = ensure_own_bits(n); rc != APGAR_B200_OK) return rc;
   // work runs on the negotiation's own stream, ordered after the caller's
   APGAR_B200_CUDA("cudaEventRecord(entry)", cudaEventRecord(n->entry, caller));
   APGAR_B200_CUDA("cudaStreamWaitEvent", cudaStreamWaitEvent(n->work, n->entry, 0));
@@ -1920,7 +1902,6 @@ extern "C" int apgar_b200_negotiation_step(void* negotiation, uint32_t round, ui
     APGAR_B200_CUDA("cudaMalloc(round stats)", n->stats.ensure(2ull * kMaxStepRounds));
     n->rounds_capacity = kMaxStepRounds;
   }
-  if (int rc = ensure_own_bits(n); rc != APGAR_B200_OK) return rc;
   const auto caller = static_cast<cudaStream_t>(stream);
   APGAR_B200_CUDA("cudaEventRecord(entry)", cudaEventRecord(n->entry, caller));
   APGAR_B200_CUDA("cudaStreamWaitEvent", cudaStreamWaitEvent(n->work, n->entry, 0));

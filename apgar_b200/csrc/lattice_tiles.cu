@@ -1474,7 +1474,7 @@ __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n,
 
 // The net's result, and its path by the canonical walk.
 template <bool kPriced>
-__device__ __forceinline__ void finish_net(const TileLaunch& p, const TileNet& n, const TileNetState* st, bool free_ends,
+__device__ __forceinline__ void finish_net(const TileLaunch& p, const TileNet& n, const TileNetState* st, bool free_ends, bool team,
                                            uint32_t net, uint32_t* tile, uint64_t* quads, uint32_t* prices, int lane) {
   const LatticeDeviceView& lat = p.lat;
   __threadfence();
@@ -1483,7 +1483,9 @@ __device__ __forceinline__ void finish_net(const TileLaunch& p, const TileNet& n
     if (lane == 0) {
       NetPlan plan{};
       plan.net = net;
-      p.redo[atomicAdd(p.redo_count, 1u)] = plan;
+      // (the team class's nets come first among the plans, so here too)
+      const uint32_t first = team || p.c[0].team == 0u ? 0u : p.c[0].end;
+      p.redo[first + atomicAdd(p.redo_count + (team ? 0 : 1), 1u)] = plan;
     }
     return;
   }
@@ -1654,7 +1656,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
     } else if (done || idle > kIdleLimit) {
       if (!done && lane == 0) atomicMax(&st->stop, 2u);
       __syncwarp();
-      if (!kept) finish_net<kPriced>(p, n, st, free_ends, p.plans[index].net, tile, quads, prices, lane);
+      if (!kept) finish_net<kPriced>(p, n, st, free_ends, p.c[k].team != 0u, p.plans[index].net, tile, quads, prices, lane);
       __syncwarp();
       if (lane == 0) atomicAdd(p.finished, 1u);
       busy = false;

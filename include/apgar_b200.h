@@ -519,10 +519,13 @@ APGAR_B200_API int apgar_b200_lattice_plan_info(void* plan, apgar_b200_plan_info
  *  FRONTIER: bucketed, label-correcting A* (key = label + octile-plus-via
  *            bound) in key levels of `bucket_width`, persistent and
  *            work-stealing, largest windows first.  It stops once every cell
- *            with key <= the goal label is final.  Two forms: over 32 x 32
- *            tiles (plans without a bound on the rounds and without chains
- *            or windows above 2^25 cells), and over single cells (the rest,
- *            and priced nets near the 32-bit limit).  Result
+ *            with key <= the goal label is final.  Two forms, chosen for the
+ *            whole batch when it is planned: over 32 x 32 tiles (no bound on
+ *            the rounds, no chains, and no window above 2^25 cells or whose
+ *            cells times the largest move cost reach 0x7FFE0000), and over
+ *            single cells (every other batch).  Priced nets of a tile batch
+ *            that come near the 32-bit limit are handed over to the search
+ *            over cells.  Result
  *            counters, tiles / cells: sweeps = units relaxed / rounds,
  *            row_steps = line steps of 32 cells / cell expansions,
  *            row_stores = key levels opened, row_loads = 0.  They depend on
@@ -559,7 +562,10 @@ typedef struct apgar_b200_lattice_options {
  * `cell_costs` is a device array [layers][height][width] of uint32, read by
  * every later execute until replaced; NULL removes it.  A move into cell c
  * then costs its move cost plus cell_costs[c].  A net whose path costs reach
- * 2^31 - 1 comes back REJECTED instead of with a wrong cost. */
+ * 2^31 - 1 comes back REJECTED instead of with a wrong cost.  The call only
+ * keeps the pointer: it allocates nothing, does not wait for the device, may
+ * be made while a stream is captured, and leaves executions captured before
+ * it as they are. */
 APGAR_B200_API int apgar_b200_lattice_plan_set_cell_costs(void* plan, const uint32_t* cell_costs);
 
 /* Corridor mode of a FRONTIER plan (no reference counterpart: the learned
