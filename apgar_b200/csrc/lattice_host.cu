@@ -466,6 +466,8 @@ int plan_tiles(PlanObject* plan) {
   plan->tiles_per_net = net_words * 4ull <= per_net_budget();
   uint64_t words = net_words;
   if (!plan->tiles_per_net) {
+    // a slot more than the class has nets would only take memory
+    for (ClassRange& range : plan->tile_classes) range.slots = std::min(range.slots, range.count);
     fit_slots(plan->tile_classes, slot_budget(), [](const ClassRange& c) { return c.slab_cells * 4ull; });
     words = 0;
     for (ClassRange& range : plan->tile_classes) {

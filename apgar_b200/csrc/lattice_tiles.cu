@@ -1552,7 +1552,9 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
   extern __shared__ __align__(16) uint32_t tile_smem[];
   __shared__ Lookout look;
   const int lane = threadIdx.x & 31;
-  const uint32_t warp = blockIdx.x * (kTileThreads / 32) + (threadIdx.x >> 5);
+  // numbered across the CTAs: where the workspace is in slots, the warps that
+  // own nets are spread over the SMs
+  const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   uint32_t* const tile = tile_smem + (threadIdx.x >> 5) * (kWarpWords + (kPriced ? kPriceWords : 0));
   uint64_t* const quads = reinterpret_cast<uint64_t*>(tile + kTileWords);
   uint32_t* const prices = tile + kWarpWords;
