@@ -189,7 +189,7 @@ struct TileLaunch {
   uint64_t path_arena_capacity;
   unsigned long long* arena_cursor;
   const volatile uint32_t* cancel;
-  unsigned int* finished;  // nets that are done
+  unsigned int* finished;  // [0] nets that are done, [1] a net was given up with a warp still in it
   // prices, kept routes and rip-up pricing, as in FrontierLaunch; own_bits is
   // one bit per label word of the pool.  A net whose prices or labels come
   // near the 32-bit limit goes to `redo` (the cell form then decides it): the

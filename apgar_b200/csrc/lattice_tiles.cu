@@ -80,14 +80,18 @@ constexpr uint32_t kWhole = 1u << 18;       // every cell of the unit may lower 
 // The cancel flag is read across the bus: by one lane, when a net starts and
 // after every so many turns of one warp.
 constexpr uint32_t kCancelPollTurns = 256;
-// Guards against a broken invariant only (every pass over a unit lowers a
-// label, so they are finite): reported, never silent.
-constexpr int kMaxUnitPasses = 1 << 16;
+// Guards against a broken invariant only: reported, never silent.  Each pass
+// makes the labels exact whose least path within the unit has one move more,
+// and such a path has at most 1,023 moves, so 1,024 passes do.  A pass is at
+// most 128 steps of 34 cycles, 204 with 24 warps on the SM: at the limit a
+// unit takes 54 million cycles, which a waiting owner outlasts (kIdleLimit).
+constexpr int kMaxUnitPasses = 1 << 11;
 // An idle warp naps between looks at its net's queue: its looks take issue
 // slots from the warps at work.
 constexpr uint32_t kNapNs = 300;
-// Naps without any unit finished in the net before an idle warp gives up, and
-// without work before a helper does.
+// Naps without any unit finished in the net before its owner gives it up, and
+// without work before a helper does.  Between two naps come three dependent
+// reads of the L2, 750 cycles or more: 200 million cycles in all.
 constexpr uint32_t kIdleLimit = 1u << 18;
 // Guests of a net at a time, a guest's looks at an empty queue before it
 // leaves, and SM clocks between a CTA's searches for a net to visit.
@@ -490,8 +494,7 @@ __device__ __forceinline__ uint32_t pop_unit(TileNetState* st, const Space& ws, 
   __syncwarp();
   if (lane == 0) {
     if (unit == kEmptySlot) {
-      atomicMax(&st->stop, 2u);
-      atomicSub(&st->active, 1u);
+      atomicMax(&st->stop, 2u);  // (still active: nobody reuses the net's workspace)
     } else {
       *slot = kEmptySlot;
     }
@@ -1472,6 +1475,17 @@ __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n,
   return free_ends;
 }
 
+// A net that may not be searched: its slot may still be written to.
+__device__ __forceinline__ void reject_net(TileNetState* st, int lane) {
+  if (lane == 0) {
+    st->goal = kTileInf;
+    st->stop = 2u;
+    __threadfence();
+    *reinterpret_cast<volatile uint32_t*>(&st->phase) = 2u;
+  }
+  __syncwarp();
+}
+
 // The net's result, and its path by the canonical walk.
 template <bool kPriced>
 __device__ __forceinline__ void finish_net(const TileLaunch& p, const TileNet& n, const TileNetState* st, bool free_ends, bool team,
@@ -1567,7 +1581,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
   __syncthreads();
   int k = 0;
   uint32_t index = 0, low = 0, skip = 0;
-  bool busy = false, owner = false, member = false, free_ends = false, kept = false;
+  bool busy = false, owner = false, member = false, free_ends = false, kept = false, given_up = false;
   TileNetState* st = nullptr;
   TileNet n;
   LanePart part{};
@@ -1619,7 +1633,12 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
         if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&st->phase) = 2u;
         __syncwarp();
       } else if (owner) {
-        free_ends = start_net(p, n, st, p.c[k].level_width, place, p.plans[index].net, lane);
+        if (p.per_net == 0u && __shfl_sync(kFull, peek(p.finished + 1), 0) != 0u) {
+          reject_net(st, lane);
+          free_ends = true;
+        } else {
+          free_ends = start_net(p, n, st, p.c[k].level_width, place, p.plans[index].net, lane);
+        }
       }
       if (k < 5 && p.c[k].team != 0u) __syncthreads();  // the team waits for the net's set-up
       if (k == 5) {
@@ -1627,6 +1646,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
         __syncwarp();
       }
       busy = true;
+      given_up = false;
       idle = misses = 0;
       seen = kNoKey;
     }
@@ -1655,8 +1675,21 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
         busy = false;
         continue;
       }
+    } else if (!done && idle > kIdleLimit && !given_up) {
+      // Nothing finishes.  The net is rejected, once its units have drained
+      // (each ends at once now): another warp may still be in one.
+      if (lane == 0) atomicMax(&st->stop, 2u);
+      __syncwarp();
+      given_up = true;
+      idle = 0u;
     } else if (done || idle > kIdleLimit) {
-      if (!done && lane == 0) atomicMax(&st->stop, 2u);
+      if (!done && lane == 0) {
+        // Given up for good: a warp that never left a unit may still write to
+        // the net's workspace, so no later net takes a slot.
+        *reinterpret_cast<volatile uint32_t*>(p.finished + 1) = 1u;
+        *reinterpret_cast<volatile uint32_t*>(&st->phase) = 2u;
+        __threadfence();
+      }
       __syncwarp();
       if (!kept) finish_net<kPriced>(p, n, st, free_ends, p.c[k].team != 0u, p.plans[index].net, tile, quads, prices, lane);
       __syncwarp();
