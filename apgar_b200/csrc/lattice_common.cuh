@@ -70,6 +70,15 @@ struct SweepLaunch {
   int row_warps;                    // warps side by side in a row (set by the launcher)
 };
 
+// A row width class of the sweep: the widest row, cells a lane, warps side by
+// side in a row, the kernel's bound on these, nets an SM holds, and whether a
+// lane holds its cells of every layer (lattice_sweep_rows.cu) or a warp one
+// layer's (lattice_sweep.cu).
+struct SweepShape {
+  int width, cells, warps, most, nets;
+  bool lanes;
+};
+
 // One width class of the frontier form (lattice_frontier.cu).  The kernel
 // is persistent: each resident warp group owns one workspace slot and reuses
 // it for every net it takes.  Slot s holds `slab_cells` label words

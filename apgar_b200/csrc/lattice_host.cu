@@ -20,11 +20,10 @@
 
 namespace apgar_b200 {
 
-bool lattice_sweep_shape(int layers, int index, int* cells, int* warps);
-uint32_t lattice_sweep_widest(int layers);
-size_t lattice_sweep_smem_bytes(int layers, int cells, int warps, int max_rows);
-cudaError_t launch_lattice_sweep(int layers, int cells, int warps, SweepLaunch launch,
-                                 int max_rows, cudaStream_t stream);
+SweepShape lattice_sweep_shape(int layers, int index, bool crowded);
+size_t lattice_sweep_smem_bytes(int layers, const SweepShape& shape, int max_rows);
+cudaError_t launch_lattice_sweep(int layers, const SweepShape& shape, SweepLaunch launch, int max_rows,
+                                 cudaStream_t stream);
 cudaError_t launch_accumulate_cells(const apgar_b200_lattice_result* results, uint32_t count,
                                     const uint32_t* paths, uint32_t* usage, uint64_t cell_count,
                                     int sm_count, cudaStream_t stream);
@@ -68,18 +67,17 @@ cudaError_t launch_corridors(const float* logits, const uint32_t* dims,
 
 namespace {
 
-// Width classes.  A sweep net's class is a shape of lattice_sweep_shape (cells
-// per lane and warps side by side on each layer); the frontier's classes are
-// 1, 2, 4, 8 and 16 warps a net.
-constexpr int kClassCount = 16;
+// Width classes.  A sweep net's class is a row width of lattice_sweep_shape (at
+// most 19 of them); the frontier's classes are 1, 2, 4, 8 and 16 warps a net.
+constexpr int kClassCount = 20;
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;
 constexpr size_t kStatesAt = 32;  // of PlanObject::counters (256 bytes on: the states are 128 bytes each)
 
 struct LatticeObject;
 
 struct ClassRange {
-  int warps_per_net = 0;  // SWEEP: of each layer
-  int cells = 0;          // SWEEP: per lane
+  int warps_per_net = 0;  // FRONTIER
+  SweepShape shape{};     // SWEEP
   uint32_t begin = 0;  // into plans
   uint32_t count = 0;
   int max_rows = 0;
@@ -239,15 +237,22 @@ int check_device(int expected) {
   return APGAR_B200_OK;
 }
 
-// Smallest sweep class whose row coverage holds `width` cells; -1 if none.
-int class_for_width(uint32_t width, int layers) {
-  if (width > lattice_sweep_widest(layers)) return -1;
-  int cells = 0, warps = 0;
-  for (int i = 0; i < kClassCount && lattice_sweep_shape(layers, i, &cells, &warps); ++i) {
-    if (32u * static_cast<uint32_t>(cells) * static_cast<uint32_t>(warps) >= width) return i;
+// The sweep's row width classes of a layer count.
+struct SweepClasses {
+  int count = 0;
+  uint32_t width[kClassCount];
+  explicit SweepClasses(int layers) {
+    for (SweepShape s = lattice_sweep_shape(layers, 0, false); count < kClassCount && s.width != 0;
+         s = lattice_sweep_shape(layers, count, false)) {
+      width[count++] = static_cast<uint32_t>(s.width);
+    }
   }
-  return -1;
-}
+  // The narrowest class that holds a row; -1 if none.
+  int of(uint32_t row) const {
+    const int c = static_cast<int>(std::lower_bound(width, width + count, row) - width);
+    return c < count ? c : -1;
+  }
+};
 
 // Frontier width class (warps per net as a power of two) from the window's cell count.
 // A frontier round is a chain of dependent memory waves, so its latency falls
@@ -550,6 +555,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
   const uint64_t max_move = std::max(v.orth, std::max(v.diag, v.via));
 
   std::vector<std::vector<uint32_t>> members(kClassCount);  // SWEEP
+  const SweepClasses sweep_classes(v.layers);
   uint64_t arena_cells = 0;
   uint64_t largest = 0;  // FRONTIER: cells of the largest window
   plan->admitted.clear();
@@ -583,7 +589,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
     }
     const uint32_t frame_width = std::max(n.win_w, n.win_h);
     const uint32_t frame_rows = std::min(n.win_w, n.win_h);
-    const int ci = class_for_width(frame_width, v.layers);
+    const int ci = sweep_classes.of(frame_width);
     if (ci < 0 || frame_rows > 32000u) continue;
     members[ci].push_back(i);
   }
@@ -602,7 +608,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
       return ca > cb;
     });
     ClassRange range;
-    lattice_sweep_shape(v.layers, ci, &range.cells, &range.warps_per_net);
+    range.shape = lattice_sweep_shape(v.layers, ci, m.size() > static_cast<size_t>(plan->sm_count));
     range.begin = static_cast<uint32_t>(plans.size());
     range.count = static_cast<uint32_t>(m.size());
     for (uint32_t i : m) {
@@ -619,7 +625,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
       range.max_rows = std::max(range.max_rows, static_cast<int>(np.rows));
       plans.push_back(np);
     }
-    if (lattice_sweep_smem_bytes(v.layers, range.cells, range.warps_per_net, range.max_rows) > kMaxSmemPerBlock) {
+    if (lattice_sweep_smem_bytes(v.layers, range.shape, range.max_rows) > kMaxSmemPerBlock) {
       return set_error(APGAR_B200_UNSUPPORTED, "window too tall for the shared-memory row map");
     }
     plan->classes.push_back(range);
@@ -656,7 +662,8 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
   int least_priority = 0, greatest_priority = 0;
   APGAR_B200_CUDA("cudaDeviceGetStreamPriorityRange",
                   cudaDeviceGetStreamPriorityRange(&least_priority, &greatest_priority));
-  for (int ci = 0; ci < kClassCount; ++ci) {
+  // (streams of its own for each class that a sweep launches)
+  for (int ci = 0; ci < static_cast<int>(frontier ? 0 : plan->classes.size()); ++ci) {
     if (plan->class_streams[ci] == nullptr) {
       // wider classes (higher positions) get higher priority: their blocks
       // need most of an SM and hold the nets with the most rounds, so they
@@ -843,7 +850,7 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
       APGAR_B200_CUDA("cudaStreamWaitEvent", cudaStreamWaitEvent(s, plan->fork, 0));
     }
     APGAR_B200_CUDA("lattice sweep launch",
-                    launch_lattice_sweep(v.layers, c.cells, c.warps_per_net, launch, c.max_rows, s));
+                    launch_lattice_sweep(v.layers, c.shape, launch, c.max_rows, s));
     if (fan_out) {
       APGAR_B200_CUDA("cudaEventRecord(join)", cudaEventRecord(plan->joins[k], s));
       APGAR_B200_CUDA("cudaStreamWaitEvent", cudaStreamWaitEvent(stream, plan->joins[k], 0));
@@ -1402,6 +1409,7 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
   NoallocStaging& h = g_noalloc_host;
 
   // Admission and width classes: the same rules as a plan.
+  const SweepClasses sweep_classes(v.layers);
   for (uint32_t i = 0; i < count; ++i) {
     const apgar_b200_lattice_net& n = host_nets[i];
     apgar_b200_lattice_result& r = h.init[i];
@@ -1422,19 +1430,22 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
     if (cells * max_move >= kLabelInf) continue;
     const uint32_t frame_width = std::max(n.win_w, n.win_h);
     const uint32_t frame_rows = std::min(n.win_w, n.win_h);
-    const int ci = class_for_width(frame_width, v.layers);
+    const int ci = sweep_classes.of(frame_width);
     if (ci < 0 || frame_rows > 32000u) continue;
     h.width_class[i] = static_cast<int8_t>(ci);
   }
 
+  int sm_count = 0;
+  APGAR_B200_CUDA("cudaDeviceGetAttribute",
+                  cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, lat->device));
   // The launches follow one another on the caller's stream, so the nets of
   // rows that one warp covers share one: each takes the shape of the widest.
   // (A launch of its own for each shape measured 1.16 ms against 0.73 for the
   // 96 nets of a planar board.)
-  constexpr int kOneWarp = 2;
-  int shared_class = -1;
+  int one_warp = 0, shared_class = -1;
+  while (lattice_sweep_shape(v.layers, one_warp + 1, false).warps == 1) ++one_warp;
   for (uint32_t i = 0; i < count; ++i) {
-    if (h.width_class[i] <= kOneWarp) shared_class = std::max(shared_class, static_cast<int>(h.width_class[i]));
+    if (h.width_class[i] <= one_warp) shared_class = std::max(shared_class, static_cast<int>(h.width_class[i]));
   }
   for (uint32_t i = 0; i < count; ++i) {
     if (h.width_class[i] >= 0 && h.width_class[i] < shared_class) h.width_class[i] = static_cast<int8_t>(shared_class);
@@ -1457,7 +1468,7 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
     });
     ClassRange& range = ranges[range_count++];
     range = ClassRange{};
-    lattice_sweep_shape(v.layers, ci, &range.cells, &range.warps_per_net);
+    range.shape = lattice_sweep_shape(v.layers, ci, members > static_cast<uint32_t>(sm_count));
     range.begin = planned;
     range.count = members;
     for (uint32_t k = 0; k < members; ++k) {
@@ -1475,8 +1486,7 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
       arena_cells += 8ull * (n.win_w + n.win_h) + 64ull * v.layers;
       range.max_rows = std::max(range.max_rows, static_cast<int>(np.rows));
     }
-    if (lattice_sweep_smem_bytes(v.layers, range.cells, range.warps_per_net, range.max_rows) >
-        kMaxSmemPerBlock) {
+    if (lattice_sweep_smem_bytes(v.layers, range.shape, range.max_rows) > kMaxSmemPerBlock) {
       return set_error(APGAR_B200_UNSUPPORTED, "window too tall for the shared-memory row map");
     }
   }
@@ -1508,9 +1518,6 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
   auto* d_arena = reinterpret_cast<uint32_t*>(base + arena_at);
   auto* d_paths = reinterpret_cast<uint32_t*>(base + paths_at);
 
-  int sm_count = 0;
-  APGAR_B200_CUDA("cudaDeviceGetAttribute",
-                  cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, lat->device));
   // The pageable source copies return once the bytes are staged, so the host
   // staging arrays may be reused by the next call.
   if (count > 0) {
@@ -1544,8 +1551,7 @@ int route_noalloc(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, u
     launch.plans = d_plans + ranges[k].begin;
     launch.plan_count = ranges[k].count;
     APGAR_B200_CUDA("lattice sweep launch",
-                    launch_lattice_sweep(v.layers, ranges[k].cells, ranges[k].warps_per_net, launch,
-                                         ranges[k].max_rows, stream));
+                    launch_lattice_sweep(v.layers, ranges[k].shape, launch, ranges[k].max_rows, stream));
   }
   APGAR_B200_CUDA("lattice pack launch",
                   launch_lattice_pack(d_results, count, d_counters + 1, d_arena, d_paths, sm_count,

@@ -18,7 +18,9 @@
 // its via cascade.  With all layers of a chunk in one warp a warp had 4 x C
 // cells to go through and no way to skip any: 1,024 nets of 4 x 1024^2, median
 // row 162 cells, took 11.1 ms, 8.6 now; 96 planar nets, where the gain is
-// fewer cells a lane and the rows that end early, 0.89 ms and 0.56.
+// fewer cells a lane and the rows that end early, 0.89 ms and 0.56.  Where that
+// other form is the better one, wide rows of few layers keep it
+// (lattice_sweep_rows.cu).
 //
 // A row step:
 //   1. relaxes the row from the previous row in sweep order (straight plus
@@ -55,20 +57,14 @@
 
 #include <cstdint>
 
-#include "lattice_common.cuh"
+#include "lattice_sweep.cuh"
 
 namespace apgar_b200 {
+
+size_t sweep_rows_smem_bytes(int layers, int warps, int max_rows);
+cudaError_t launch_sweep_rows(int layers, int warps, const SweepLaunch& launch, int max_rows, cudaStream_t stream);
+
 namespace {
-
-constexpr int16_t kNever = -32000;
-constexpr int kMaxRowPasses = 4096;
-
-// Geometry of one net in its frame.
-struct Frame {
-  int transposed;
-  int R, K, pitch;
-  int x0, y0;
-};
 
 // Per-lane view of one layer's guard-padded sweep planes for one net: the two
 // words holding the lane's span (frame positions xs-1 .. xs+C) of frame row r
@@ -111,8 +107,9 @@ __device__ __forceinline__ BitSpan make_span(const LatticeDeviceView& lat, const
   return s;
 }
 
-// The two words of a plane that hold the lane's span of frame row r.  They are kept as loaded until the row is processed, so that nothing
-// waits for a prefetch when it is issued.
+// The two words of a plane that hold the lane's span of frame row r.  They are
+// kept as loaded until the row is processed, so that nothing waits for a
+// prefetch when it is issued.
 __device__ __forceinline__ uint2 span_words(const BitSpan& s, const uint32_t* plane, int r) {
   const uint32_t* w = plane + static_cast<uint32_t>(r) * s.row_stride;
   return make_uint2(__ldg(w), __ldg(w + 1));
@@ -140,85 +137,6 @@ __device__ __forceinline__ uint32_t shfl_down_to(uint32_t v, int by, int stop) {
   asm volatile("shfl.sync.down.b32 %0, %1, %2, %3, 0xFFFFFFFF;" : "=r"(d) : "r"(v), "r"(by), "r"(stop));
   return d;
 }
-
-template <int C>
-__device__ __forceinline__ void load_cells(const uint32_t* src, int pitch, int xs,
-                                           uint32_t (&v)[C]) {
-  static_assert(C % 2 == 0, "C must be even");
-  if constexpr (C % 4 == 0) {
-#pragma unroll
-    for (int q = 0; q < C / 4; ++q) {
-      const int x = xs + 4 * q;
-      if (x < pitch) {
-        const uint4 t = *reinterpret_cast<const uint4*>(src + x);
-        v[4 * q + 0] = t.x;
-        v[4 * q + 1] = t.y;
-        v[4 * q + 2] = t.z;
-        v[4 * q + 3] = t.w;
-      } else {
-        v[4 * q + 0] = v[4 * q + 1] = v[4 * q + 2] = v[4 * q + 3] = kLabelInf;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < C / 2; ++q) {
-      const int x = xs + 2 * q;
-      if (x < pitch) {
-        const uint2 t = *reinterpret_cast<const uint2*>(src + x);
-        v[2 * q + 0] = t.x;
-        v[2 * q + 1] = t.y;
-      } else {
-        v[2 * q + 0] = v[2 * q + 1] = kLabelInf;
-      }
-    }
-  }
-}
-
-template <int C>
-__device__ __forceinline__ void store_cells(uint32_t* dst, int pitch, int xs,
-                                            const uint32_t (&v)[C]) {
-  if constexpr (C % 4 == 0) {
-#pragma unroll
-    for (int q = 0; q < C / 4; ++q) {
-      const int x = xs + 4 * q;
-      if (x < pitch) {
-        *reinterpret_cast<uint4*>(dst + x) =
-            make_uint4(v[4 * q + 0], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < C / 2; ++q) {
-      const int x = xs + 2 * q;
-      if (x < pitch) *reinterpret_cast<uint2*>(dst + x) = make_uint2(v[2 * q + 0], v[2 * q + 1]);
-    }
-  }
-}
-
-__device__ __forceinline__ bool cell_free(const LatticeDeviceView& lat,
-                                          const apgar_b200_lattice_net& n, int l, int x, int y) {
-  if (l < 0 || l >= lat.layers || x < 0 || y < 0 || x >= static_cast<int>(n.win_w) ||
-      y >= static_cast<int>(n.win_h)) {
-    return false;
-  }
-  const int gx = static_cast<int>(n.win_x0) + x, gy = static_cast<int>(n.win_y0) + y;
-  const uint32_t word =
-      __ldg(lat.blocked + (static_cast<size_t>(l) * lat.height + gy) * lat.words + (gx >> 5));
-  return ((word >> (gx & 31)) & 1u) == 0;
-}
-
-__device__ __forceinline__ bool via_bit_at(const LatticeDeviceView& lat,
-                                           const apgar_b200_lattice_net& n, int lower, int x,
-                                           int y) {
-  if (lat.via_ok == nullptr) return true;
-  const int gx = static_cast<int>(n.win_x0) + x, gy = static_cast<int>(n.win_y0) + y;
-  const uint32_t word =
-      __ldg(lat.via_ok + (static_cast<size_t>(lower) * lat.height + gy) * lat.words + (gx >> 5));
-  return ((word >> (gx & 31)) & 1u) != 0;
-}
-
-__constant__ int kDxc[8] = {1, 1, 0, -1, -1, -1, 0, 1};
-__constant__ int kDyc[8] = {0, 1, 1, 1, 0, -1, -1, -1};
 
 // Shared memory of a CTA (shared by the kernel and the host).
 struct SweepSmem {
@@ -255,16 +173,9 @@ __device__ __forceinline__ void net_sync() {
   }
 }
 
-// Nets an SM should hold: a large batch of narrow nets is bound by the nets in
-// flight (4 layers, 1,000 nets of median row 107: 5.3 ms with the registers
-// the compiler takes by itself, 4.7 with this bound).
-__host__ __device__ constexpr int resident_nets(int L, int C, int kMost) {
-  return kMost > 1 ? 1 : C == 4 ? 20 / L : C == 8 ? 16 / L : 1;
-}
-
-// G = p.row_warps <= kMost warps side by side.
-template <int L, int C, int kMost>
-__global__ void __launch_bounds__(32 * L * kMost, resident_nets(L, C, kMost))
+// G = p.row_warps <= kMost warps side by side; an SM holds kNets nets or more.
+template <int L, int C, int kMost, int kNets>
+__global__ void __launch_bounds__(32 * L * kMost, kNets)
     lattice_sweep_kernel(SweepLaunch p, int max_rows) {
   constexpr bool kMulti = kMost > 1;
   constexpr bool kOne = L == 1 && !kMulti;  // the CTA is one warp
@@ -561,9 +472,9 @@ __global__ void __launch_bounds__(32 * L * kMost, resident_nets(L, C, kMost))
         };
         // The votes of a row: did a label change since the row was loaded (bit
         // l for layer l, for the write-back) and since the last exchange (bit
-        // 8), and this row's edges for the next step.  Buffer eb ^ 1 is read by no warp until the next step, and
-        // every read of it by the previous step came before this step's first
-        // barrier.
+        // 8), and this row's edges for the next step.  Buffer eb ^ 1 is read by
+        // no warp until the next step, and every read of it by the previous
+        // step came before this step's first barrier.
         const auto publish_flags = [&](bool recent) {
           if constexpr (kMulti) {
             if (lane == 0) sh_edges[(eb ^ 1) * edge_buf + warp * 2] = v[0];
@@ -753,93 +664,8 @@ __global__ void __launch_bounds__(32 * L * kMost, resident_nets(L, C, kMost))
 
   // ----------------------------- result + walk -----------------------------
   if (warp != 0) return;
-  apgar_b200_lattice_result res{};
-  res.cost = APGAR_B200_UNREACHABLE;
-  res.completion = completion;
-  res.sweeps = sweeps_done;
-  res.row_steps = stat_rows;
-  res.row_stores = stat_stores;
-  res.row_loads = stat_loads;
-  auto label_at = [&](int l, int x, int y) -> uint32_t {
-    const int r = f.transposed ? x : y, q = f.transposed ? y : x;
-    const uint32_t label = slab[static_cast<uint32_t>(l) * layer_stride +
-                                static_cast<uint32_t>(r) * static_cast<uint32_t>(f.pitch) + static_cast<uint32_t>(q)];
-    return modified[r] == kNever ? kLabelInf : label;  // a row never stored holds no labels
-  };
-  if (completion == APGAR_B200_COMPLETION_REACHED) {
-    const uint32_t goal = label_at(g_layer, lgx, lgy);
-    if (goal >= kLabelInf) {
-      res.completion = APGAR_B200_COMPLETION_DISCONNECTED;
-    } else {
-      res.cost = goal;
-      const uint32_t min_move = min(orth, min(diag, via));
-      const unsigned long long bound = goal / min_move + 1ull;
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(p.arena_cursor, bound);
-      base = __shfl_sync(0xFFFFFFFFu, base, 0);
-      if (base + bound > p.path_arena_capacity) {
-        res.completion = APGAR_B200_COMPLETION_REJECTED;
-        res.cost = APGAR_B200_UNREACHABLE;
-      } else {
-        const int Ln = lat.layers;
-        int cl = g_layer, cx = lgx, cy = lgy;
-        uint32_t here = goal;
-        uint32_t n = 0;
-        bool ok = false;
-        while (n < bound) {
-          if (lane == 0) {
-            p.path_arena[base + n] = static_cast<uint32_t>(
-                (static_cast<size_t>(cl) * lat.height + (f.y0 + cy)) * lat.width + (f.x0 + cx));
-          }
-          ++n;
-          if (cl == s_layer && cx == lsx && cy == lsy) {
-            ok = true;
-            break;
-          }
-          // One round of independent loads per cell (0.45 us a cell with the
-          // bit planes read first and the labels after).  The labels tell
-          // what is free: at the fixed point every free cell next to a
-          // reached one is reached, so an unreached side cell is blocked.
-          int pl = cl, px = cx, py = cy;
-          bool via_legal = true;
-          if (lane < 8) {
-            px = cx - kDxc[lane];
-            py = cy - kDyc[lane];
-          } else if (lane == 8 || lane == 9) {
-            pl = (lane == 8) ? cl - 1 : cl + 1;
-            if (pl >= 0 && pl < Ln) via_legal = via_bit_at(lat, net, min(pl, cl), cx, cy);
-          }
-          uint32_t pd = kLabelInf;
-          if (lane < 10 && pl >= 0 && pl < Ln && px >= 0 && px < static_cast<int>(net.win_w) && py >= 0 &&
-              py < static_cast<int>(net.win_h)) {
-            pd = label_at(pl, px, py);
-          }
-          // the side cells of diagonal h are the neighbours at h - 1 and h + 1
-          const uint32_t side_a = __shfl_sync(0xFFFFFFFFu, pd, (lane + 7) & 7);
-          const uint32_t side_b = __shfl_sync(0xFFFFFFFFu, pd, (lane + 1) & 7);
-          const bool diagonal = lane < 8 && (lane & 1);
-          const uint32_t move = lane >= 8 ? via : diagonal ? diag : orth;
-          const bool legal = via_legal && (!diagonal || (side_a < kLabelInf && side_b < kLabelInf));
-          const bool cand = legal && pd < kLabelInf && pd + move == here;
-          const unsigned ballot = __ballot_sync(0xFFFFFFFFu, cand);
-          if (ballot == 0u) break;
-          const int hsel = __ffs(ballot) - 1;
-          cl = __shfl_sync(0xFFFFFFFFu, pl, hsel);
-          cx = __shfl_sync(0xFFFFFFFFu, px, hsel);
-          cy = __shfl_sync(0xFFFFFFFFu, py, hsel);
-          here = __shfl_sync(0xFFFFFFFFu, pd, hsel);
-        }
-        if (ok) {
-          res.path_len = n;
-          res.arena_offset = base;
-        } else {
-          res.completion = APGAR_B200_COMPLETION_REJECTED;
-          res.cost = APGAR_B200_UNREACHABLE;
-        }
-      }
-    }
-  }
-  if (lane == 0) p.results[plan.net] = res;
+  write_sweep_result(p, plan, f, net, slab, layer_stride, modified, completion, sweeps_done, stat_rows, stat_stores,
+                     stat_loads, lane);
 }
 
 // Deterministic packing of the reverse paths in caller net order: one block
@@ -895,105 +721,118 @@ __global__ void pack_copy_kernel(apgar_b200_lattice_result* results, uint32_t co
   }
 }
 
-template <int L, int C, int kMost>
+template <int L, int C, int kMost, int kNets>
 cudaError_t launch_one(const SweepLaunch& launch, int max_rows, cudaStream_t stream) {
   const size_t smem = sweep_smem(L, C, launch.row_warps, max_rows).total;
-  cudaError_t e = cudaFuncSetAttribute(lattice_sweep_kernel<L, C, kMost>,
+  cudaError_t e = cudaFuncSetAttribute(lattice_sweep_kernel<L, C, kMost, kNets>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  lattice_sweep_kernel<L, C, kMost>
+  lattice_sweep_kernel<L, C, kMost, kNets>
       <<<launch.plan_count, L * launch.row_warps * 32, smem, stream>>>(launch, max_rows);
   return cudaGetLastError();
 }
 
-template <int L>
-cudaError_t launch_layers(int cells, const SweepLaunch& launch, int max_rows, cudaStream_t stream) {
-  constexpr int kWidest = 16 / L;  // warps of a row: 16 a net
-  const int warps = launch.row_warps;
-  if (warps < 1 || warps > kWidest) return cudaErrorInvalidValue;
-  switch (cells) {
-    case 4:
-      if constexpr (L == 2) {
-        if (warps > 1) return launch_one<L, 4, kWidest>(launch, max_rows, stream);
+// Row width classes of a layer count, narrowest first (width 0 past the last).
+// `crowded`: the class has more nets than the device has SMs.
+//
+// One warp a row up to 512 cells: a second one brings a barrier and a fold into
+// every scan (4 layers of 424 cells: 2.2 us a step with 4 x 1 warps of 16 cells
+// a lane, 3.0 with 4 x 4 of 4; 1 layer of 310: 0.88 us with one warp, 1.58 with
+// three).  Twelve cells a lane save registers where sixteen leave room for few
+// nets on an SM (1,500 nets of 380 cells: 3 layers 10.7 -> 8.9 ms, 6 layers 30.6
+// -> 15.9).
+//
+// Past that, a class alone on its SMs takes the shape whose step is shortest,
+// and a crowded one the shape of which two nets fit on an SM (a register limit
+// of 8 or 12 warps a net): 4 layers of 645 cells, 8 nets 4.8 ms with 3 warps a
+// row and 6.0 with 2 x 12 cells, 592 nets 20.5 and 16.7.
+//
+// Rows of one layer past 1,024 cells, of two past 512, and the widest of three
+// and four take the other form, a lane with its cells of every layer
+// (lattice_sweep_rows.cu): it has half the barriers a step, and at two layers a
+// third of the warps, so an SM holds more nets (2 layers of 645 cells: 592 nets
+// 7.5 ms, 15.1 with a warp a layer, 8 nets 3.5 and 3.6; 1 layer of 1,500: 592
+// nets 10.8 and 15.4 ms, 8 nets 4.9 and 5.8).
+constexpr SweepShape row_lanes(int cells, int warps) { return {32 * cells * warps, cells, warps, warps, 1, true}; }
+
+constexpr SweepShape sweep_shape_at(int layers, int index, bool crowded) {
+  const SweepShape none{};
+  // width, cells a lane, warps a row, the kernel's bound on these, nets an SM holds
+  switch (layers) {
+    case 1: {
+      const SweepShape t[] = {{128, 4, 1, 1, 20}, {256, 8, 1, 1, 16}, {512, 16, 1, 1, 1}, {768, 8, 3, 16, 1}, {1024, 8, 4, 16, 1}};
+      return index < 5 ? t[index] : index < 19 ? row_lanes(16, index - 2) : none;
+    }
+    case 2: {
+      const SweepShape t[] = {{128, 4, 1, 1, 10}, {256, 8, 1, 1, 8}, {512, 16, 1, 1, 1}};
+      return index < 3 ? t[index] : index < 17 ? row_lanes(8, index) : none;
+    }
+    case 3: {
+      const SweepShape t[] = {{128, 4, 1, 1, 6}, {256, 8, 1, 1, 5}, {384, 12, 1, 1, 1}, {512, 16, 1, 1, crowded ? 4 : 1},
+                              crowded ? SweepShape{768, 12, 2, 2, 2} : SweepShape{768, 8, 3, 3, 1},
+                              crowded ? SweepShape{1024, 16, 2, 2, 2} : SweepShape{1024, 8, 4, 4, 1},
+                              {1280, 8, 5, 5, 1}, {1536, 12, 4, 4, 1}, {2048, 16, 4, 4, 1}};
+      return index < 9 ? t[index] : none;
+    }
+    case 4: {
+      const SweepShape t[] = {{128, 4, 1, 1, 5}, {256, 8, 1, 1, 4}, {384, 12, 1, 1, 1}, {512, 16, 1, 1, 1},
+                              crowded ? SweepShape{768, 12, 2, 2, 2} : SweepShape{768, 8, 3, 3, 1},
+                              crowded ? SweepShape{1024, 16, 2, 2, 2} : SweepShape{1024, 16, 2, 2, 1},
+                              {1152, 12, 3, 3, 1}, {1536, 16, 3, 3, 1}};
+      return index < 8 ? t[index] : index < 12 ? row_lanes(4, index + 5) : none;
+    }
+    case 6: {
+      const SweepShape t[] = {{128, 4, 1, 1, 3}, {256, 8, 1, 1, 2}, {384, 12, 1, 1, crowded ? 2 : 1}, {512, 16, 1, 1, 1},
+                              {768, 12, 2, 2, 1}, {1024, 16, 2, 2, 1}};
+      return index < 6 ? t[index] : none;
+    }
+    case 8: {
+      const SweepShape t[] = {{128, 4, 1, 1, 2}, {256, 8, 1, 1, 2}, {512, 16, 1, 1, 1}, {768, 12, 2, 2, 1}, {1024, 16, 2, 2, 1}};
+      return index < 5 ? t[index] : none;
+    }
+    default: return none;
+  }
+}
+
+template <int L, int kIndex = 0, bool kCrowded = false>
+cudaError_t launch_shape(const SweepShape& shape, const SweepLaunch& launch, int max_rows, cudaStream_t stream) {
+  constexpr SweepShape t = sweep_shape_at(L, kIndex, kCrowded);
+  if constexpr (t.width == 0) {
+    return cudaErrorInvalidValue;
+  } else {
+    if constexpr (!t.lanes) {
+      if (shape.cells == t.cells && shape.warps == t.warps && shape.nets == t.nets) {
+        return launch_one<L, t.cells, t.most, t.nets>(launch, max_rows, stream);
       }
-      return warps == 1 ? launch_one<L, 4, 1>(launch, max_rows, stream) : cudaErrorInvalidValue;
-    case 8:
-      return warps == 1 ? launch_one<L, 8, 1>(launch, max_rows, stream)
-                        : launch_one<L, 8, kWidest>(launch, max_rows, stream);
-    case 16:
-      return warps == 1 ? launch_one<L, 16, 1>(launch, max_rows, stream)
-                        : launch_one<L, 16, kWidest>(launch, max_rows, stream);
-    default: return cudaErrorInvalidValue;
+    }
+    return launch_shape<L, kCrowded ? kIndex + 1 : kIndex, !kCrowded>(shape, launch, max_rows, stream);
   }
 }
 
 }  // namespace
 
-// The widest row of a layer count.
-uint32_t lattice_sweep_widest(int layers) {
-  return 8192u / (layers <= 1 ? 1u : layers == 2 ? 2u : layers <= 4 ? 4u : 8u);
+SweepShape lattice_sweep_shape(int layers, int index, bool crowded) {
+  return index < 0 ? SweepShape{} : sweep_shape_at(layers, index, crowded);
 }
 
-// Row width classes of a layer count, narrowest first: cells per lane and
-// warps side by side; false past the last class.  One warp a row up to 512
-// cells: a second one brings a barrier and a fold into every scan (4 layers of
-// 424 cells: 2.2 us a step with 4 x 1 warps of 16 cells a lane, 3.0 with
-// 4 x 4 of 4; 1 layer of 310: 0.88 us with one warp, 1.58 with three).  Past
-// 512, eight cells a lane while 16 warps a net suffice (4 layers of 601 cells:
-// 3.4 us a step with 4 x 3 warps of 8, 4.1 with 4 x 2 of 16: both are bound by
-// one SM's integer throughput), then sixteen; two layers leave room for four
-// cells a lane up to 1,024 (200 nets of 2 x 1024^2, rows up to 718: 4.14 ms with
-// eight cells a lane, 3.82 with four; 1,000 nets, rows up to 651: 5.8 and 4.9).
-bool lattice_sweep_shape(int layers, int index, int* cells, int* warps) {
-  if (layers < 1 || index < 0) return false;
-  *warps = 1;
-  *cells = index < 2 ? 4 << index : 16;
-  if (index < 3) return true;
-  index -= 3;
-  const int most = min(8, 16 / layers);  // warps of a row of eight cells a lane
-  if (layers == 2) {
-    *cells = 4;
-    for (int w = 5; w <= 8; ++w) {
-      if (index-- == 0) {
-        *warps = w;
-        return true;
-      }
-    }
-  }
-  *cells = 8;
-  for (int w = layers == 2 ? 5 : 3; w <= most; ++w) {
-    if (index-- == 0) {
-      *warps = w;
-      return true;
-    }
-  }
-  *cells = 16;
-  const int widest = static_cast<int>(lattice_sweep_widest(layers));
-  for (int w = most < 3 ? 2 : most / 2 + 1; 512 * (w - 1) < widest && w * layers <= 16; w += w < 6 ? 1 : 2) {
-    if (index-- == 0) {
-      *warps = w;
-      return true;
-    }
-  }
-  return false;
+size_t lattice_sweep_smem_bytes(int layers, const SweepShape& shape, int max_rows) {
+  return shape.lanes ? sweep_rows_smem_bytes(layers, shape.warps, max_rows)
+                     : sweep_smem(layers, shape.cells, shape.warps, max_rows).total;
 }
 
-size_t lattice_sweep_smem_bytes(int layers, int cells, int warps, int max_rows) {
-  return sweep_smem(layers, cells, warps, max_rows).total;
-}
-
-cudaError_t launch_lattice_sweep(int layers, int cells, int warps, SweepLaunch launch, int max_rows,
+cudaError_t launch_lattice_sweep(int layers, const SweepShape& shape, SweepLaunch launch, int max_rows,
                                  cudaStream_t stream) {
   if (launch.plan_count == 0) return cudaSuccess;
-  launch.row_warps = warps;
+  launch.row_warps = shape.warps;
+  if (shape.lanes) return launch_sweep_rows(layers, shape.warps, launch, max_rows, stream);
   switch (layers) {
-    case 1: return launch_layers<1>(cells, launch, max_rows, stream);
-    case 2: return launch_layers<2>(cells, launch, max_rows, stream);
-    case 3: return launch_layers<3>(cells, launch, max_rows, stream);
-    case 4: return launch_layers<4>(cells, launch, max_rows, stream);
-    case 6: return launch_layers<6>(cells, launch, max_rows, stream);
-    case 8: return launch_layers<8>(cells, launch, max_rows, stream);
+    case 1: return launch_shape<1>(shape, launch, max_rows, stream);
+    case 2: return launch_shape<2>(shape, launch, max_rows, stream);
+    case 3: return launch_shape<3>(shape, launch, max_rows, stream);
+    case 4: return launch_shape<4>(shape, launch, max_rows, stream);
+    case 6: return launch_shape<6>(shape, launch, max_rows, stream);
+    case 8: return launch_shape<8>(shape, launch, max_rows, stream);
     default: return cudaErrorInvalidValue;
   }
 }
