@@ -198,6 +198,8 @@ struct TileLaunch {
   uint64_t path_arena_capacity;
   unsigned long long* arena_cursor;
   const volatile uint32_t* cancel;
+  uint32_t* watch;         // [0] the batch is cancelled, [1] when the host's flag was last read (ns)
+  uint64_t units;          // of all nets
   unsigned int* finished;  // [0] nets that are done, [1] a net was given up with a warp still in it
   // prices, kept routes and rip-up pricing, as in FrontierLaunch; own_bits is
   // one bit per label word of the pool.  A net whose prices or labels come

@@ -71,6 +71,7 @@ namespace {
 // most 19 of them); the frontier's classes are 1, 2, 4, 8 and 16 warps a net.
 constexpr int kClassCount = 20;
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;
+static_assert(2 + kClassCount + 4 <= 32, "the counters lie before the states");
 constexpr size_t kStatesAt = 32;  // of PlanObject::counters (256 bytes on: the states are 128 bytes each)
 
 struct LatticeObject;
@@ -145,11 +146,13 @@ struct PlanObject {
   std::vector<ClassRange> tile_classes;
   DeviceBuffer<NetPlan> tile_plans;
   DeviceBuffer<uint32_t> tile_pool;
-  uint32_t tile_warps = 0;  // warps of a launch
+  uint32_t tile_warps = 0;  // warps that fit on the device
+  uint64_t tile_units = 0;  // units of all nets
   // FRONTIER, tile form with prices: the cell form's classes for nets that the
   // tile search hands over (see plan_tiles), the CTA-wide class's own first
   ClassRange redo[2];
   bool one_shot = false;  // never gets prices
+  bool priced_cells = false;  // FRONTIER, tile form: priced executions take the cell form
   std::vector<apgar_b200_lattice_net> host_nets;  // FRONTIER: the batch, as planned
   std::vector<uint32_t> admitted;                 // FRONTIER: its admitted nets
   const uint32_t* cell_cost = nullptr;  // caller-owned device prices (frontier only)
@@ -178,7 +181,8 @@ struct PlanObject {
   DeviceBuffer<uint32_t> lists;            // FRONTIER: three queue lists per net
   // [0] arena cursor, [1] packed total, [2 + class] work-stealing cursors,
   // [2 + kClassCount] the tile form's finished nets, nets handed over (a 32-bit
-  // count for each of `redo`) and their cursors (likewise), then its net states
+  // count for each of `redo`), their cursors (likewise) and its watch on the
+  // cancel flag, then its net states
   DeviceBuffer<unsigned long long> counters;
   uint64_t label_cells = 0;
   uint64_t arena_capacity = 0;
@@ -327,6 +331,26 @@ std::vector<uint32_t> sweep_planes(const uint32_t* in, int planes, int height, i
   return out;
 }
 
+// Batches whose windows hold too few units, or too short searches, for the tile
+// form (a unit costs 10 to 20 us however few of its cells matter): the cell
+// form is the faster one for them.  Measured, cells and tiles in ms: 24 nets of
+// 4 x 4 cells 0.05 and 0.08 on two layers, 0.07 and 0.12 on eight; one net of
+// 64 to 130 cells a side on eight layers 0.13 to 0.18 and 0.15 to 0.25.  More
+// nets, or larger windows, favour the tiles (150 nets of 4 x 4 cells 0.17 and
+// 0.07 to 0.17, one net of 200 x 200 x 8 0.80 and 0.38).
+bool small_batch(int layers, size_t nets, uint64_t largest, uint32_t longest) {
+  return (nets <= 64 && longest <= 16) || (layers >= 8 && nets <= 4 && largest <= (1u << 17));
+}
+
+// The same under prices, where a unit also loads its cells' prices at every
+// visit and a path keeps to few units: with many layers (eight: 600 nets of 70
+// to 130 cells a side 1.7 to 2.4 and 2.1 to 3.1, of 200 4.8 and 5.0; 1,200 nets
+// of half-perimeter 20 2.3 and 3.2, 300 of 45 5.6 and 2.8), and for a handful of
+// nets with short paths (30 of half-perimeter 20, four layers: 0.23 and 0.36).
+bool small_priced_batch(int layers, size_t nets, uint64_t largest) {
+  return (layers >= 8 && largest <= (1u << 18)) || (layers >= 4 && nets <= 32 && largest <= 40960);
+}
+
 // The admitted nets of a frontier batch by width class, largest windows first
 // (longest-processing-time order).
 std::vector<std::vector<uint32_t>> frontier_members(const PlanObject* plan, uint32_t bounds) {
@@ -448,6 +472,7 @@ int plan_tiles(PlanObject* plan) {
   APGAR_B200_CUDA("cudaOccupancyMaxActiveBlocksPerMultiprocessor",
                   lattice_tile_warps(plan->sm_count, &plan->tile_warps));
   uint64_t net_words = 0;
+  plan->tile_units = 0;
   for (int k = 4; k >= 0; --k) {
     if (members[k].empty()) continue;
     ClassRange range;
@@ -461,6 +486,7 @@ int plan_tiles(PlanObject* plan) {
       np.dist_offset = net_words;  // used when every net gets its own workspace
       const uint64_t words = lattice_tile_words(v.layers, n.win_w, n.win_h);
       net_words += words;
+      plan->tile_units += static_cast<uint64_t>(v.layers) * ((n.win_w + 31u) / 32u) * ((n.win_h + 31u) / 32u);
       range.slab_cells = std::max<uint64_t>(range.slab_cells, words);
       plans.push_back(np);
     }
@@ -490,7 +516,7 @@ int plan_tiles(PlanObject* plan) {
   // than one slot for each class is larger for it.
   uint32_t extra = 0;  // plan records of handed over nets
   for (ClassRange& r : plan->redo) r = ClassRange{};
-  if (!plan->one_shot) {
+  if (!plan->one_shot && !plan->priced_cells) {
     extra = static_cast<uint32_t>(plans.size());
     uint32_t begin = 0;
     for (int k = 1; k >= 0; --k) {  // the CTA-wide class, the others
@@ -558,8 +584,9 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
   const SweepClasses sweep_classes(v.layers);
   uint64_t arena_cells = 0;
   uint64_t largest = 0;  // FRONTIER: cells of the largest window
+  uint32_t longest = 0;  // FRONTIER: the longest side of a window
   plan->admitted.clear();
-  plan->tiles = false;
+  plan->tiles = plan->priced_cells = false;
   plan->classes.clear();
   std::vector<apgar_b200_lattice_result> init(count);
   std::memset(init.data(), 0, init.size() * sizeof(apgar_b200_lattice_result));
@@ -585,6 +612,7 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
       plan->admitted.push_back(i);
       arena_cells += 8ull * (n.win_w + n.win_h) + 64ull * v.layers;
       largest = std::max(largest, cells);
+      longest = std::max(longest, std::max(n.win_w, n.win_h));
       continue;
     }
     const uint32_t frame_width = std::max(n.win_w, n.win_h);
@@ -640,9 +668,18 @@ int build_plan(LatticeObject* lat, const apgar_b200_lattice_net* host_nets, uint
     // rounds (its rounds are not the cell form's), no chained expansions, and
     // no window whose queue lists the cell form may cut (a net that outgrows
     // them is rejected) or whose labels could reach the tile form's limit.
+    // Nor does it take batches whose windows are too small for it (see
+    // small_batch).
     plan->tiles = max_sweeps == kUnboundedRounds && plan->chain <= 1u && plan->wide_chain <= 1u &&
-                  largest <= kMaxListEntries && largest * max_move < kTileLabelLimit;
-    if (int rc = plan->tiles ? plan_tiles(plan) : plan_cells(plan); rc != APGAR_B200_OK) return rc;
+                  largest <= kMaxListEntries && largest * max_move < kTileLabelLimit &&
+                  !small_batch(v.layers, plan->admitted.size(), largest, longest);
+    plan->priced_cells = plan->tiles && !plan->one_shot && small_priced_batch(v.layers, plan->admitted.size(), largest);
+    if (!plan->tiles || plan->priced_cells) {
+      if (int rc = plan_cells(plan); rc != APGAR_B200_OK) return rc;
+    }
+    if (plan->tiles) {
+      if (int rc = plan_tiles(plan); rc != APGAR_B200_OK) return rc;
+    }
   } else {
     APGAR_B200_CUDA("cudaMalloc(label slabs)", plan->dist_pool.ensure(std::max<uint64_t>(dist_cells, 4)));
     if (int rc = upload_plans(plan->plans, plans); rc != APGAR_B200_OK) return rc;
@@ -720,7 +757,7 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
     fbase.corridor = plan->corridor;
     fbase.corridor_status = plan->corridor_status.get();
   }
-  if (plan->tiles) {
+  if (plan->tiles && !(plan->priced_cells && plan->cell_cost != nullptr)) {
     TileLaunch t{};
     t.lat = v;
     t.nets = plan->nets.get();
@@ -730,6 +767,8 @@ int execute_plan(PlanObject* plan, cudaStream_t stream) {
     t.path_arena_capacity = plan->arena_capacity;
     t.arena_cursor = plan->counters.get();
     t.cancel = plan->cancel_dev;
+    t.watch = reinterpret_cast<uint32_t*>(plan->counters.get() + 2 + kClassCount + 3);
+    t.units = plan->tile_units;
     t.finished = reinterpret_cast<unsigned int*>(plan->counters.get() + 2 + kClassCount);
     t.plans = plan->tile_plans.get();
     t.states = reinterpret_cast<TileNetState*>(plan->counters.get() + kStatesAt);
@@ -1794,7 +1833,7 @@ extern "C" int apgar_b200_negotiation_create(void* plan, const apgar_b200_price_
     APGAR_B200_CUDA("cudaMalloc(usage)", n->usage.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(cell costs)", n->cell_cost.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(own-route cell costs)", n->cell_cost_own.ensure(cells));
-    const size_t label_words = p->tiles ? p->tile_pool.count() : p->words.count();
+    const size_t label_words = p->tiles && !p->priced_cells ? p->tile_pool.count() : p->words.count();
     APGAR_B200_CUDA("cudaMalloc(own-route bits)", n->own_bits.ensure(label_words / 32 + 1));
     APGAR_B200_CUDA("cudaMalloc(history)", n->history.ensure(cells));
     APGAR_B200_CUDA("cudaMalloc(previous results)", n->prev_results.ensure(std::max<uint32_t>(p->count, 1)));

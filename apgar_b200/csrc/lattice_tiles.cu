@@ -77,9 +77,14 @@ constexpr uint32_t kSourceBits = 0x3FFu;    // unit flags: sides that lowered so
 constexpr uint32_t kInFar = 1u << 16;       // the unit stands in the far list
 constexpr uint32_t kTouched = 1u << 17;     // the unit's labels have been written
 constexpr uint32_t kWhole = 1u << 18;       // every cell of the unit may lower others (the corridor was lifted)
-// The cancel flag is read across the bus: by one lane, when a net starts and
-// after every so many turns of one warp.
+// Cancellation is looked for when a net starts and after every so many turns of
+// its owner.
 constexpr uint32_t kCancelPollTurns = 256;
+// The host's flag is read across the bus, about 1 us a read and one after the
+// other (at every net's start: 600 nets of 12 x 12 cells took 0.6 ms, nearly all
+// of it waiting for these), so one warp of the grid reads it at most this
+// often, and the others its copy on the device.
+constexpr uint32_t kCancelLookNs = 20000;
 // Guards against a broken invariant only: reported, never silent.  Each pass
 // makes the labels exact whose least path within the unit has one move more,
 // and such a path has at most 1,023 moves, so 1,024 passes do.  A pass is at
@@ -1411,6 +1416,18 @@ __device__ __forceinline__ uint32_t find_net(const TileLaunch& p, uint32_t& low,
   return found;
 }
 
+// Whether the batch is cancelled (one lane).
+__device__ __forceinline__ bool batch_cancelled(const TileLaunch& p) {
+  if (p.cancel == nullptr) return false;
+  if (peek(p.watch) != 0u) return true;
+  uint32_t now;
+  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(now));
+  const uint32_t then = peek(p.watch + 1);
+  if (now - then < kCancelLookNs || atomicCAS(p.watch + 1, then, now) != then || *p.cancel == 0u) return false;
+  *reinterpret_cast<volatile uint32_t*>(p.watch) = 1u;
+  return true;
+}
+
 // Clears the net's workspace and queues its start.
 __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n, TileNetState* st, uint32_t level_width,
                                           uint32_t slot, uint32_t net, int lane) {
@@ -1461,7 +1478,7 @@ __device__ __forceinline__ bool start_net(const TileLaunch& p, const TileNet& n,
     st->confined = confined;
     st->exit_key = kNoKey;
     st->corridor = outcome;
-    st->stop = p.cancel != nullptr && *p.cancel != 0u ? 1u : 0u;
+    st->stop = batch_cancelled(p) ? 1u : 0u;
     st->steps = st->units = st->levels = 0u;
     st->slot = slot;
     st->guests = 0u;
@@ -1651,7 +1668,7 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
       seen = kNoKey;
     }
     if (owner && p.cancel != nullptr && (++turns % kCancelPollTurns) == 0u) {
-      if (lane == 0 && *p.cancel != 0u) atomicMax(&st->stop, 1u);
+      if (lane == 0 && batch_cancelled(p)) atomicMax(&st->stop, 1u);
       __syncwarp();
     }
     const uint32_t unit = pop_unit(st, n.ws, lane);
@@ -1693,7 +1710,8 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocks) lattice_tiles_kerne
       __syncwarp();
       if (!kept) finish_net<kPriced>(p, n, st, free_ends, p.c[k].team != 0u, p.plans[index].net, tile, quads, prices, lane);
       __syncwarp();
-      if (lane == 0) atomicAdd(p.finished, 1u);
+      if (lane == 0 && atomicAdd(p.finished, 1u) + 1u >= p.total) *reinterpret_cast<volatile uint32_t*>(&look.over) = 1u;
+      __syncwarp();
       busy = false;
       continue;
     } else {
@@ -1772,7 +1790,9 @@ cudaError_t launch_lattice_tiles(const TileLaunch& launch, int sm_count, cudaStr
   if (launch.total == 0) return cudaSuccess;
   uint32_t warps = 0;
   if (cudaError_t e = lattice_tile_warps(sm_count, &warps); e != cudaSuccess) return e;
-  const unsigned grid = warps / (kTileThreads / 32);
+  // A CTA for every eight units: more would only wait for the end (one net of
+  // 4 x 4 cells: 52 us with all of them).
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(warps, launch.units + 7u) / (kTileThreads / 32));
   const bool priced = launch.cell_cost != nullptr;
   const TileKernel kernel = tile_kernel(launch.lat.diag < launch.lat.orth, priced, launch.corridor != nullptr);
   kernel<<<grid, kTileThreads, tile_smem_bytes(priced), stream>>>(launch);
