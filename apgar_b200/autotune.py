@@ -1,9 +1,14 @@
 """Schedule autotuner for the frontier generator.
 
 The frontier's results do not depend on its schedule: the key-level width
-(bucket width), chained expansions and the width-class limits that give a net
-1, 2, 4, 8 or 16 warps only change how the same exact search is laid out on
-the GPU.  So the tuner times candidate schedules on the caller's own batch
+(bucket width), chained expansions and the width-class limits only change how
+the same exact search is laid out on the GPU.  In the search over tiles the last
+limit says which nets take a whole CTA from the start, and the first three only
+size the slots of a workspace that does not hold every net at once; in the
+search over cells the four give a net 1, 2, 4, 8 or 16 warps.  Chained
+expansions exist over cells only, so the candidate that asks for them times
+that form.  Executions are timed without prices; a schedule without chains
+keeps the plan's form under prices too.  So the tuner times candidate schedules on the caller's own batch
 (or a seeded sample with the batch's window-size mix) and keeps the fastest.
 Every candidate's costs are compared with the first candidate's, and a
 mismatch raises: a schedule that changed a result would be a bug.

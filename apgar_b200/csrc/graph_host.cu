@@ -455,7 +455,7 @@ int run_batch(ViewObject* v, const apgar_b200_batch_request& req,
   }
   APGAR_B200_CUDA("cudaEventRecord", cudaEventRecord(t1, nullptr));
   // The caller's flag is sampled here and forwarded through the view's
-  // mapped flag, which the kernel polls once per round.
+  // mapped flag, which a query reads at its start and every 64 rounds.
   for (;;) {
     const cudaError_t q = cudaEventQuery(t1);
     if (q == cudaSuccess) break;

@@ -442,7 +442,8 @@ __global__ void __launch_bounds__(kThreads) graph_search_kernel(GraphLaunch p) {
 }
 
 // The same search for graphs whose state fits one SM: 32-bit labels, 16-bit
-// neighbours and queues in shared memory (65.5 B per node: about 3,400 nodes).
+// neighbours and queues in shared memory (65.5 B per node: 3,530 nodes without a
+// policy).
 //
 // Every label is the cost of a walk without a repeated state, so at most
 // states * (the batch's largest finite move); the host takes this form only

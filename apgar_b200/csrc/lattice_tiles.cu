@@ -303,7 +303,7 @@ __device__ __forceinline__ void unit_masks(const LatticeDeviceView& lat, const W
 }
 
 // Labels of a unit and its rim into the warp's tile.  touched: bit k set when
-// neighbour k (the order of kNeighbour below) has labels; own: this unit has.
+// neighbour k (the order of `neighbours`) has labels; own: this unit has.
 __device__ __forceinline__ void load_unit(const uint32_t* labels, const Win& win, const Unit& u,
                                           uint32_t touched, bool own, uint32_t* tile, int lane) {
   const uint32_t* mine = labels + static_cast<size_t>(u.id) * 1024u;

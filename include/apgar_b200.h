@@ -523,9 +523,10 @@ APGAR_B200_API int apgar_b200_lattice_plan_info(void* plan, apgar_b200_plan_info
  *            whole batch when it is planned: over 32 x 32 tiles (no bound on
  *            the rounds, no chains, and no window above 2^25 cells or whose
  *            cells times the largest move cost reach 0x7FFE0000), and over
- *            single cells (every other batch).  Priced nets of a tile batch
- *            that come near the 32-bit limit are handed over to the search
- *            over cells.  Result
+ *            single cells (every other batch, and a few small windows).
+ *            Under prices a tile batch of small windows on many layers is
+ *            searched over cells too, as are its nets that come near the
+ *            32-bit limit.  Result
  *            counters, tiles / cells: sweeps = units relaxed / rounds,
  *            row_steps = line steps of 32 cells / cell expansions,
  *            row_stores = key levels opened, row_loads = 0.  They depend on
@@ -577,9 +578,11 @@ APGAR_B200_API int apgar_b200_lattice_plan_set_cell_costs(void* plan, const uint
  * searches its corridor only.  The result is kept when its cost is strictly
  * below the least key (label + move + admissible bound) over every legal
  * move leaving the corridor that the search expanded, which proves it equal
- * to the full-window result, path included.  Otherwise the net is searched
- * again over the whole window, so results never depend on the corridor.
- * NULL detaches the corridors.  Not combined with per-cell prices. */
+ * to the full-window result, path included.  Otherwise the search goes on
+ * over the whole window (over tiles from the corridor's labels, over cells
+ * from the start), so results never depend on the corridor.  With per-cell
+ * prices the keys leave out the exit cell's price, which keeps the proof.
+ * NULL detaches the corridors. */
 enum {
   APGAR_B200_CORRIDOR_NONE = 0,               /* no corridors, or the net's bitmap is empty */
   APGAR_B200_CORRIDOR_CERTIFIED = 1,          /* the corridor result, certified */
