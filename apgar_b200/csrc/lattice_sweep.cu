@@ -664,8 +664,7 @@ __global__ void __launch_bounds__(32 * L * kMost, kNets)
 
   // ----------------------------- result + walk -----------------------------
   if (warp != 0) return;
-  write_sweep_result(p, plan, f, net, slab, layer_stride, modified, completion, sweeps_done, stat_rows, stat_stores,
-                     stat_loads, lane);
+#include "lattice_sweep_walk.cuh"
 }
 
 // Deterministic packing of the reverse paths in caller net order: one block
@@ -739,14 +738,19 @@ cudaError_t launch_one(const SweepLaunch& launch, int max_rows, cudaStream_t str
 // One warp a row up to 512 cells: a second one brings a barrier and a fold into
 // every scan (4 layers of 424 cells: 2.2 us a step with 4 x 1 warps of 16 cells
 // a lane, 3.0 with 4 x 4 of 4; 1 layer of 310: 0.88 us with one warp, 1.58 with
-// three).  Twelve cells a lane save registers where sixteen leave room for few
-// nets on an SM (1,500 nets of 380 cells: 3 layers 10.7 -> 8.9 ms, 6 layers 30.6
-// -> 15.9).
+// three).  Twelve cells a lane save registers where sixteen leave room for too
+// few nets on an SM (1,500 nets of 380 cells: 3 layers 10.7 -> 8.9 ms, 6 layers
+// 30.6 -> 15.9); on four layers a class more, with a launch and a stream of its
+// own, cost a batch of many widths up to 4%.
 //
 // Past that, a class alone on its SMs takes the shape whose step is shortest,
 // and a crowded one the shape of which two nets fit on an SM (a register limit
-// of 8 or 12 warps a net): 4 layers of 645 cells, 8 nets 4.8 ms with 3 warps a
-// row and 6.0 with 2 x 12 cells, 592 nets 20.5 and 16.7.
+// of 8 or 12 warps a net): 4 layers of 645 cells, 8 nets 5.2 ms with 3 warps a
+// row and 6.0 with 2 x 12 cells, 592 nets 22.0 and 16.7.  Up to 1,024 cells on
+// three and four layers the kernel's bound on the warps stays above their
+// number: compiled for 3 warps a row the 8 nets took 4.8 ms, but each held an
+// SM's registers, and a batch of many widths had no room for other nets beside
+// them (1,024 nets of 4 x 1024^2, five seeds of 16: 6.7 to 7.5 -> 7.3 to 7.8 ms).
 //
 // Rows of one layer past 1,024 cells, of two past 512, and the widest of three
 // and four take the other form, a lane with its cells of every layer
@@ -770,17 +774,17 @@ constexpr SweepShape sweep_shape_at(int layers, int index, bool crowded) {
     }
     case 3: {
       const SweepShape t[] = {{128, 4, 1, 1, 6}, {256, 8, 1, 1, 5}, {384, 12, 1, 1, 1}, {512, 16, 1, 1, crowded ? 4 : 1},
-                              crowded ? SweepShape{768, 12, 2, 2, 2} : SweepShape{768, 8, 3, 3, 1},
-                              crowded ? SweepShape{1024, 16, 2, 2, 2} : SweepShape{1024, 8, 4, 4, 1},
+                              crowded ? SweepShape{768, 12, 2, 2, 2} : SweepShape{768, 8, 3, 5, 1},
+                              crowded ? SweepShape{1024, 16, 2, 2, 2} : SweepShape{1024, 8, 4, 5, 1},
                               {1280, 8, 5, 5, 1}, {1536, 12, 4, 4, 1}, {2048, 16, 4, 4, 1}};
       return index < 9 ? t[index] : none;
     }
     case 4: {
-      const SweepShape t[] = {{128, 4, 1, 1, 5}, {256, 8, 1, 1, 4}, {384, 12, 1, 1, 1}, {512, 16, 1, 1, 1},
-                              crowded ? SweepShape{768, 12, 2, 2, 2} : SweepShape{768, 8, 3, 3, 1},
-                              crowded ? SweepShape{1024, 16, 2, 2, 2} : SweepShape{1024, 16, 2, 2, 1},
+      const SweepShape t[] = {{128, 4, 1, 1, 5}, {256, 8, 1, 1, 4}, {512, 16, 1, 1, 1},
+                              crowded ? SweepShape{768, 12, 2, 2, 2} : SweepShape{768, 8, 3, 4, 1},
+                              crowded ? SweepShape{1024, 16, 2, 2, 2} : SweepShape{1024, 8, 4, 4, 1},
                               {1152, 12, 3, 3, 1}, {1536, 16, 3, 3, 1}};
-      return index < 8 ? t[index] : index < 12 ? row_lanes(4, index + 5) : none;
+      return index < 7 ? t[index] : index < 11 ? row_lanes(4, index + 6) : none;
     }
     case 6: {
       const SweepShape t[] = {{128, 4, 1, 1, 3}, {256, 8, 1, 1, 2}, {384, 12, 1, 1, crowded ? 2 : 1}, {512, 16, 1, 1, 1},
